@@ -195,13 +195,7 @@ __global__ void k_combine(const double* __restrict__ part, int nchunks,
   if (i >= n) return;
   const int64_t t = off + i;
   double a[NC];
-#pragma unroll
-  for (int k = 0; k < NC; ++k) a[k] = 0.0;
-  for (int c = 0; c < nchunks; ++c) {
-    const double* p = part + (int64_t)c * NC * ntgt_pad + t;
-#pragma unroll
-    for (int k = 0; k < NC; ++k) a[k] += p[k * ntgt_pad];
-  }
+  sum_chunks<NC>(part + t, nchunks, ntgt_pad, a);
   double pos[3] = {x(i, 0), x(i, 1), NDIM == 3 ? x(i, 2) : 0.0};
   if (MODE == M_REF64) {
     double uu[3], ps = 0;
@@ -231,7 +225,7 @@ template <int MODE, int NDIM, bool WU, bool WP>
 void launch_combine(lpm_context& ctx, const NbodyPlan& p, const double* part,
                     int64_t off, const TgtSeg& seg, const void* tgt,
                     const double* sg, double c0) {
-  const int th = 256;
+  const int th = sum_threads(seg.n);
   const int64_t nb = (seg.n + th - 1) / th;
   k_combine<MODE, NDIM, WU, WP><<<nb, th, 0, ctx.stream>>>(
       part, p.nchunks, p.ntgt_pad, off, seg.n, seg.x, seg.u, seg.psi, tgt, sg, c0, p.form,
@@ -312,6 +306,14 @@ void launch_chord(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
 template <int FORM, bool WU, bool WP>
 void launch_f64(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
                 const int* tself, const void* src, double* part, double eps2) {
+  if (p.fine) {
+    dim3 g(unsigned(p.ntgt_pad / FINE_NT), unsigned(p.nchunks));
+    nbody_f64h<FORM, WU, WP, 1, FINE_NT, FINE_TILE><<<g, FINE_NT, 0, ctx.stream>>>(
+        static_cast<const double4_16a*>(tgt), tself, static_cast<const double4_16a*>(src),
+        p.ntgt_pad, p.nsrc_pad, p.chunk_len, eps2, part, ctx.d_err);
+    ctx.launches++;
+    return;
+  }
   dim3 grid(unsigned(p.ntgt_pad / (F64_NT * F64_R)), unsigned(p.nchunks));
   if (ref64_exact(p.precision))
     nbody_f64<FORM, WU, WP, F64_R, F64_NT, F64_TILE><<<grid, F64_NT, 0, ctx.stream>>>(
@@ -394,8 +396,27 @@ int64_t compact_sources(lpm_context& ctx, const uint8_t* mask, int64_t nslots,
   return total;
 }
 
-NbodyPlan plan_nbody(lpm_context& ctx, int precision, int ndim, int form,
-                     bool wu, bool wp, int64_t ntgt, int64_t nsrc) {
+namespace {
+
+// FP64 kernels of a plan: nbody_split, the one-target-per-thread form of
+// nbody_f64h for grids too small for the tiled one, or the tiled kernels.
+enum Fp64Kind : int { FP64_TILED = 0, FP64_FINE = 1, FP64_SPLIT = 2 };
+
+// Whether the split sums (nbody_split.cuh) replace nbody_f64h: the sphere
+// forms, from 1,024 sources on (their error falls as 1 / sqrt(nsrc); against
+// exact values, icosahedral and cubed meshes of 1,280 to 20,480 sources: split
+// 0.8e-15 to 1.8e-15, nbody_f64h 1.3e-15 to 5.1e-15) and half a million pairs
+// on (below, the fine grid of nbody_f64h takes less than the two extra launches).
+bool split_wanted(int precision, int ndim, int64_t ntgt, int64_t nsrc) {
+  return precision == LPM_FP64 && ndim == 3 && nsrc >= 1024 && double(ntgt) * double(nsrc) >= 5e5;
+}
+
+struct Fp64Shape {
+  int tb, tile, ctas;  // targets per CTA, sources per tile, CTAs per SM planned for
+};
+
+NbodyPlan plan_kind(lpm_context& ctx, int precision, int ndim, int form, bool wu, bool wp,
+                    int64_t ntgt, int64_t nsrc, int kind) {
   NbodyPlan p{};
   p.precision = precision;
   p.ndim = ndim;
@@ -404,19 +425,25 @@ NbodyPlan plan_nbody(lpm_context& ctx, int precision, int ndim, int form,
   p.wp = wp;
   p.ncomp = (wu ? ndim : 0) + (wp ? 1 : 0);
   const bool f32 = precision == LPM_FP32C;
-  const int tb = f32 ? F32_TB : F64_NT * F64_R;
-  const int tile = f32 ? F32_TILE : F64_TILE;
+  Fp64Shape s{F64_NT * F64_R, F64_TILE, f32 ? 4 : 0};
+  if (f32) s = Fp64Shape{F32_TB, F32_TILE, 4};
+  else if (kind == FP64_SPLIT) s = Fp64Shape{SPLIT_NT, SPLIT_TILE, 4};
+  else if (kind == FP64_FINE) s = Fp64Shape{FINE_NT, FINE_TILE, 4};
+  else s.ctas = occupancy(precision);
+  p.split = kind == FP64_SPLIT;
+  p.fine = kind == FP64_FINE;
   p.ntgt = ntgt;
-  p.ntgt_pad = std::max<int64_t>(tb, (ntgt + tb - 1) / tb * tb);
+  p.ntgt_pad = std::max<int64_t>(s.tb, (ntgt + s.tb - 1) / s.tb * s.tb);
   p.nsrc = nsrc;
-  p.nsrc_pad = std::max<int64_t>(tile, (nsrc + tile - 1) / tile * tile);
-  const int64_t ntb = p.ntgt_pad / tb;
-  const int64_t ntiles = p.nsrc_pad / tile;
+  p.nsrc_pad = std::max<int64_t>(s.tile, (nsrc + s.tile - 1) / s.tile * s.tile);
+  const int64_t ntb = p.ntgt_pad / s.tb;
+  const int64_t ntiles = p.nsrc_pad / s.tile;
   // Aim for ~16 waves of CTAs so the tail of the last wave stays small.  The
   // FP32 shapes share one chunking (4 CTAs of 1024 targets per SM) so that the
-  // autotuner can swap shapes without changing the partial layout.
-  const int64_t slots = int64_t(std::max(ctx.num_sms, 1)) * (f32 ? 4 : occupancy(precision));
-  int64_t nch = (16 * slots + ntb - 1) / ntb;
+  // autotuner can swap shapes without changing the partial layout.  The fine
+  // form serves grids of a wave or two: two waves.
+  const int64_t slots = int64_t(std::max(ctx.num_sms, 1)) * s.ctas;
+  int64_t nch = ((p.fine ? 2 : p.split ? 8 : 16) * slots + ntb - 1) / ntb;
   if (ctx.max_part_bytes > 0) {
     const int64_t per_chunk = int64_t(sizeof(double)) * p.ncomp * p.ntgt_pad;
     nch = std::min<int64_t>(nch, int64_t(ctx.max_part_bytes) / per_chunk);
@@ -426,16 +453,49 @@ NbodyPlan plan_nbody(lpm_context& ctx, int precision, int ndim, int form,
   // raise nchunks when ntiles shrinks, but never above nch)
   p.nchunks_max = int(nch);
   const int64_t tiles_per_chunk = (ntiles + nch - 1) / nch;
-  p.chunk_len = int(tiles_per_chunk * tile);
+  p.chunk_len = int(tiles_per_chunk * s.tile);
   p.nchunks = int((ntiles + tiles_per_chunk - 1) / tiles_per_chunk);
   return p;
+}
+
+}  // namespace
+
+NbodyPlan plan_nbody(lpm_context& ctx, int precision, int ndim, int form,
+                     bool wu, bool wp, int64_t ntgt, int64_t nsrc) {
+  int kind = FP64_TILED;
+  if (split_wanted(precision, ndim, ntgt, nsrc)) {
+    kind = FP64_SPLIT;
+  } else if (precision == LPM_FP64) {
+    // tiled grid below two waves: a CTA's serial 256-source tile (2.9e5 clocks
+    // of the FP64 pipe) is the launch's whole time
+    const int64_t ctas = ((ntgt + F64_NT * F64_R - 1) / (F64_NT * F64_R)) *
+                         ((nsrc + F64_TILE - 1) / F64_TILE);
+    if (ctas < 2 * int64_t(std::max(ctx.num_sms, 1)) * occupancy(precision)) kind = FP64_FINE;
+  }
+  return plan_kind(ctx, precision, ndim, form, wu, wp, ntgt, nsrc, kind);
+}
+
+void plan_bounds(lpm_context& ctx, int precision, int ndim, int form, bool wu, bool wp,
+                 int64_t ntgt, int64_t nsrc, PlanBounds* b) {
+  *b = PlanBounds{};
+  for (int kind = FP64_TILED; kind <= FP64_SPLIT; ++kind) {
+    if (kind == FP64_SPLIT && !split_wanted(precision, ndim, ntgt, nsrc)) continue;
+    if (kind == FP64_FINE && precision != LPM_FP64) continue;
+    const NbodyPlan p = plan_kind(ctx, precision, ndim, form, wu, wp, ntgt, nsrc, kind);
+    b->ntgt_pad = std::max(b->ntgt_pad, p.ntgt_pad);
+    b->nsrc_pad = std::max(b->nsrc_pad, p.nsrc_pad);
+    b->part_bytes = std::max(b->part_bytes, p.part_bytes_max());
+    if (p.split) b->split_bytes = split_bytes(ctx, p.ntgt_pad, p.nsrc_pad);
+  }
 }
 
 void launch_nbody(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
                   const int* tself, const void* src, double* part,
                   double eps) {
   const int m = mode_of(p.precision);
-  if (m == M_C32) {
+  if (p.split) {
+    launch_split(ctx, p, tgt, tself, src, part, eps);
+  } else if (m == M_C32) {
     const float c0 = f32_c0(p.ndim, eps);
     if (p.ndim == 3)
       chord_want<float, 3>(ctx, p, tgt, src, part, c0);
@@ -573,21 +633,22 @@ void direct_sum(lpm_context& ctx, const SumSpec& spec, const SrcSpec& src,
 
   ctx.arena.reset();
   // Upper bounds first, so one reservation covers the whole call.
-  NbodyPlan p = plan_nbody(ctx, spec.precision, ndim, spec.form, spec.want_u,
-                           spec.want_psi, ntgt, src.nslots);
+  PlanBounds pb;
+  plan_bounds(ctx, spec.precision, ndim, spec.form, spec.want_u, spec.want_psi, ntgt, src.nslots,
+              &pb);
   const size_t rec = m == M_C32 ? sizeof(float4) : sizeof(double4_16a);  // target record
   const size_t srec = 32;  // source record: SrcF32 or double4_16a
   const size_t need = 4096 + sizeof(int) * (2 * size_t(src.nslots) + 2 * (size_t(src.nslots) / SCAN_BLOCK + 2)) +
-                      srec * size_t(p.nsrc_pad) + rec * size_t(p.ntgt_pad) +
-                      sizeof(int) * size_t(p.ntgt_pad) + p.part_bytes_max() +
-                      sizeof(double) * 300 + 8 * 256;
+                      srec * size_t(pb.nsrc_pad) + rec * size_t(pb.ntgt_pad) +
+                      sizeof(int) * size_t(pb.ntgt_pad) + pb.part_bytes + pb.split_bytes +
+                      sizeof(double) * 300 + 9 * 256;
   ctx.arena.reserve(need);
 
   int* slot2src = static_cast<int*>(ctx.arena.take(sizeof(int) * std::max<int64_t>(1, src.nslots)));
   int* src2slot = static_cast<int*>(ctx.arena.take(sizeof(int) * std::max<int64_t>(1, src.nslots)));
   const int64_t nsrc = compact_sources(ctx, src.mask, src.nslots, slot2src, src2slot);
-  p = plan_nbody(ctx, spec.precision, ndim, spec.form, spec.want_u,
-                 spec.want_psi, ntgt, nsrc);
+  NbodyPlan p = plan_nbody(ctx, spec.precision, ndim, spec.form, spec.want_u, spec.want_psi, ntgt,
+                           nsrc);
   for (int s = 0; s < nseg; ++s)
     if (segs[s].collocated && spec.skip_self) p.skipc = true;
 
@@ -596,6 +657,7 @@ void direct_sum(lpm_context& ctx, const SumSpec& spec, const SrcSpec& src,
   int* tself = static_cast<int*>(ctx.arena.take(sizeof(int) * size_t(p.ntgt_pad)));
   double* part = static_cast<double*>(ctx.arena.take(p.part_bytes()));
   double* sgp = static_cast<double*>(ctx.arena.take(sizeof(double) * 264));
+  if (p.split) p.split_buf = ctx.arena.take(split_bytes(ctx, p.ntgt_pad, p.nsrc_pad));
   if (m == M_C32)
     pack_and_launch<M_C32>(ctx, spec, src, segs, nseg, ntgt, p, slot2src, src2slot, srcp,
                            tgtp, tself, part, sgp);

@@ -483,11 +483,12 @@ struct lpm_ensemble {
     lpm::EnsPk k = packs();
     lpm::Rk4Buf b = bufs();
     lpm::Rk4Par P = params();
-    const int64_t nb = (T + 255) / 256;
-    lpm::k_ens_pack_state<<<nb, 256, 0, ctx->stream>>>(g, k, b.xw);
+    const int th = lpm::sum_threads(T);
+    const int64_t nb = (T + th - 1) / th;
+    lpm::k_ens_pack_state<<<nb, th, 0, ctx->stream>>>(g, k, b.xw);
     ctx->launches++;
     nbody();
-    lpm::k_rk4_final<<<nb, 256, 0, ctx->stream>>>(g, k, b, P);
+    lpm::k_rk4_final<<<nb, th, 0, ctx->stream>>>(g, k, b, P);
     ctx->launches++;
     LPM_CUDA(cudaGetLastError());
   }
@@ -515,16 +516,17 @@ struct lpm_ensemble {
     lpm::EnsPk k = packs();
     lpm::Rk4Buf b = bufs();
     lpm::Rk4Par P = params();
-    const int64_t nb = (T + 255) / 256;
-    lpm::k_rk4_begin<<<nb, 256, 0, ctx->stream>>>(g, k, b, P);
+    const int th = lpm::sum_threads(T);
+    const int64_t nb = (T + th - 1) / th;
+    lpm::k_rk4_begin<<<nb, th, 0, ctx->stream>>>(g, k, b, P);
     ctx->launches++;
     for (int s = 1; s <= 3; ++s) {
       nbody();
-      lpm::k_rk4_stage<<<nb, 256, 0, ctx->stream>>>(g, k, b, P, s);
+      lpm::k_rk4_stage<<<nb, th, 0, ctx->stream>>>(g, k, b, P, s);
       ctx->launches++;
     }
     nbody();
-    lpm::k_rk4_final<<<nb, 256, 0, ctx->stream>>>(g, k, b, P);
+    lpm::k_rk4_final<<<nb, th, 0, ctx->stream>>>(g, k, b, P);
     ctx->launches++;
     LPM_CUDA(cudaGetLastError());
   }
@@ -582,8 +584,9 @@ struct lpm_ensemble {
     if (cands.empty()) cands.push_back(TL);
     lpm::EnsPk k = packs();
     lpm::Rk4Buf b = bufs();
-    const int64_t nb = (T + 255) / 256;
-    lpm::k_ens_pack_state<<<nb, 256, 0, ctx->stream>>>(g, k, b.xw);
+    const int th = lpm::sum_threads(T);
+    const int64_t nb = (T + th - 1) / th;
+    lpm::k_ens_pack_state<<<nb, th, 0, ctx->stream>>>(g, k, b.xw);
     ctx->launches++;
     float best = 1e30f;
     int best_len = cands.front();

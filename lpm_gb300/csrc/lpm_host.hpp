@@ -177,7 +177,10 @@ struct NbodyPlan {
   int chunk_len;
   int nchunks_max;     // bound on nchunks for any nsrc <= this plan's nsrc
   int shape = 0;       // FP32 kernel shape (index into kF32Shapes)
-  bool skipc = false;  // chord stream function: drop coincident (i == j) pairs
+  bool skipc = false;  // the targets' own sources are left out (collocated)
+  bool fine = false;   // LPM_FP64: small grid, one target per thread
+  bool split = false;  // FP64 sums on the FP32 pipe (nbody_split.cuh)
+  void* split_buf = nullptr;  // split_bytes() of scratch for them
   size_t part_bytes() const {
     return sizeof(double) * size_t(ncomp) * size_t(nchunks) * size_t(ntgt_pad);
   }
@@ -187,11 +190,23 @@ struct NbodyPlan {
 };
 NbodyPlan plan_nbody(lpm_context& ctx, int precision, int ndim, int form,
                      bool wu, bool wp, int64_t ntgt, int64_t nsrc);
+// Scratch bounds of the plans for any source count up to nsrc.
+struct PlanBounds {
+  int64_t ntgt_pad = 0, nsrc_pad = 0;
+  size_t part_bytes = 0, split_bytes = 0;
+};
+void plan_bounds(lpm_context& ctx, int precision, int ndim, int form, bool wu, bool wp,
+                 int64_t ntgt, int64_t nsrc, PlanBounds* b);
 // tgt: float4[ntgt_pad] (FP32) or double4_16a[ntgt_pad] (FP64, with tself);
 // src: float4/double4_16a[nsrc_pad].  eps: kernel smoothing.
 void launch_nbody(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
                   const int* tself, const void* src, double* part,
                   double eps);
+// The split FP64 sums (nbody_split.cu): scratch, and the launches of one
+// evaluation (range, source records, pair kernel).
+size_t split_bytes(const lpm_context& ctx, int64_t ntgt_pad, int64_t nsrc_pad);
+void launch_split(lpm_context& ctx, const NbodyPlan& p, const void* tgt, const int* tself,
+                  const void* src, double* part, double eps);
 // FP32 plans: times every kernel shape on the packed arrays (one warm and
 // one timed launch each) and returns the fastest; synchronises.  Results are
 // cached in the context by problem size class.

@@ -788,6 +788,37 @@ __device__ __forceinline__ void ref64_epilogue(const double* a, const double* p,
   }
 }
 
+// Adds the NC partials of nch chunks, chunk after chunk: element (c, k) at
+// p[(c * NC + k) * stride].  Eight chunks' loads are issued before their adds:
+// one at a time the sum waits an L2 latency per chunk (24 us for 40 chunks of
+// 7,682 targets, longer than any other O(n) step of an evaluation).
+template <int NC>
+__device__ __forceinline__ void sum_chunks(const double* __restrict__ p, int nch, int64_t stride,
+                                           double (&a)[NC]) {
+  constexpr int B = 8;
+#pragma unroll
+  for (int k = 0; k < NC; ++k) a[k] = 0.0;
+  int c = 0;
+  for (; c + B <= nch; c += B, p += B * NC * stride) {
+    double v[B][NC];
+#pragma unroll
+    for (int b = 0; b < B; ++b)
+#pragma unroll
+      for (int k = 0; k < NC; ++k) v[b][k] = p[(b * NC + k) * stride];
+#pragma unroll
+    for (int b = 0; b < B; ++b)
+#pragma unroll
+      for (int k = 0; k < NC; ++k) a[k] += v[b][k];
+  }
+#pragma unroll 4
+  for (; c < nch; ++c, p += NC * stride)
+#pragma unroll
+    for (int k = 0; k < NC; ++k) a[k] += p[k * stride];
+}
+// Threads per CTA of the kernels that end in sum_chunks: 64 while that spreads
+// few targets over more SMs (FP64 adds take 64 clocks a warp), 256 otherwise.
+inline int sum_threads(int64_t n) { return n < 65536 ? 64 : 256; }
+
 // Arithmetic modes of the pair sum.
 enum Mode : int {
   M_REF64 = 0,  // LPM_FP64 / LPM_FP64_EXACT: the reference's formulas, FP64
@@ -839,6 +870,12 @@ __device__ __forceinline__ void chord_epilogue(const double* a, const double* p,
 constexpr int F32_NT = 256, F32_R = 4, F32_TILE = 512;
 constexpr int F32_TB = 1024;  // target padding: every FP32 shape divides it
 constexpr int F64_NT = 128, F64_R = 2, F64_TILE = 256;
+// FP64 small grids: one target per thread, 8-source tiles, so that a few
+// thousand targets and sources still give every SM work (a warp's FP64
+// instruction takes 64 clocks of its SM sub-partition).
+constexpr int FINE_NT = 64, FINE_TILE = 8;
+// nbody_split: targets per CTA, sources per tile
+constexpr int SPLIT_NT = 128, SPLIT_TILE = 128;
 
 // FP32 kernel shapes: threads, targets per thread, minimum resident CTAs per
 // SM (a register cap through __launch_bounds__).

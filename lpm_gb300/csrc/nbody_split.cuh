@@ -1,0 +1,454 @@
+// nbody_split.cuh -- the FP64 sphere sums (LPM_FP64) on the FP32 pipe, by
+// error-free transformations.
+//
+// Why: this part executes about 1.7 FP64 FMAs per clock per SM against 128
+// FP32 ones, so the 11 FP64 operations of a pair (nbody_f64h) cost as much
+// pipe time as 700 FP32 operations.  The form below takes about 115 FP32
+// operations per sphere pair and keeps the accuracy of the FP64 kernels:
+//
+//  * Positions are scaled by a power of two into (-1, 1) and cut into three
+//    floats on the common grids 2^-22 and 2^-45 (and the rest): differences of
+//    like parts are exact, so d = x - y is exact before it is rounded to a
+//    float pair (Dh, Dl) of 48 bits.  No cancellation error at all, where
+//    1 - x.y in FP64 loses 1e-16 absolute.
+//  * arg' = 2 (1 - x.y + eps^2) = |d|^2 + C as a float pair (exact products by
+//    FMA, Knuth TwoSum), C = (1 - |x|^2) + (1 - |y|^2) + 2 eps^2; the defects
+//    are taken exactly in FP64 once per point (they carry the reference's
+//    behaviour at stage positions off the sphere).
+//  * q = g / arg' as a float pair: MUFU reciprocal, one Newton step in FP32,
+//    one residual; then q d as float pairs.
+//  * Sums: float pairs over 4 steps, then three-float sums, then FP64 per chunk.
+//  * log(arg') (stream function): m 2^k = arg', 1/m from a 128-entry table,
+//    log1p by its series, all in float pairs.
+//
+// A pair's term carries 5.2e-15 of random relative error (rms) and 1.3e-16 of
+// mean error, which a sum of n like terms averages to 5.2e-15 sqrt(sum t^2) /
+// |sum t|; the FP64 kernel's sum carries the rounding of the running sum and
+// the cancellation in 1 - x.y (1e-16 / (1 - x.y) per pair, so the nearer a
+// pair the more the split form is ahead).  split_wanted() in direct_sum.cu
+// holds the source count from which the split sum's error is the smaller.
+// Pairs closer than 2^-20 of the domain, where the float pairs would run out
+// of bits, are evaluated in FP64 with the arithmetic of nbody_f64h.
+//
+// The planar and chord forms keep their FP64 kernels: they are well
+// conditioned (3e-16 to 5e-16 against FP64 sums), and the same sums in this
+// form measured 5e-16 to 1e-15.
+//
+// Off the sphere |d|^2 and C cancel, which leaves 2^-48 |C| of absolute error in
+// arg'; up to |C| = 1/32 that is below the rounding of 1 - x.y itself.  Pairs
+// with |C| above it and |arg'| < (|C| - 1/32) / 32 are evaluated in FP64 one by
+// one (a run without reprojection drifts, and has stray points late on).
+// Targets of |1 - |x|^2| > 1 or far outside the sources' range take the FP64
+// path for all their pairs; all targets do when a sixteenth of the sources is
+// that far off the sphere or eps is far larger than the domain.
+// Measured on one GB300 (SM clock 2,070 MHz), pair kernel alone, velocity:
+// icosahedral level 4 (7,682 x 5,120 pairs) 169 us, 233 Gpairs/s, against
+// 0.92 ms for nbody_f64h; with the stream function 10 times nbody_f64h's rate.
+// Bound: FP32 issue, 125 lane operations per pair (128 lanes per clock per SM:
+// 76 % of that at level 4, whose 2,440 CTAs end in a ragged second wave).
+#pragma once
+
+#include <type_traits>
+
+#include "f32x2.cuh"
+#include "nbody.cuh"
+
+namespace lpm {
+
+// Two sources, value by value: x hi, mid, lo (2 each), y, z, strength hi, lo,
+// defect hi, lo, source indexes.
+struct __align__(16) SplitPair {
+  float2 xh, xm, xl, yh, ym, yl, zh, zm, zl, gh, gl, ch, cl;
+  int2 slot;
+};
+static_assert(sizeof(SplitPair) == 112, "seven 16-byte loads per pair of sources");
+
+constexpr int kSplitNT = SPLIT_NT;          // targets per CTA, one per thread
+constexpr int kSplitTile = SPLIT_TILE / 2;  // pairs of sources per tile
+constexpr float kSplitTiny = 9.094947e-13f;  // 2^-40: a pair's least scaled arg'
+
+// One target: its three-float position, the constant part of arg' (its defect
+// and 2 eps^2) and whether it lies outside the scaled range (the FP64 path).
+struct __align__(16) SplitTarget {
+  float3 x, y, z;
+  float ch, cl;
+  int exact;
+};
+static_assert(sizeof(SplitTarget) == 48, "three 16-byte loads per target");
+
+// Scales of one evaluation: |position|, eps < 2^e, |strength| < 2^g.  big != 0:
+// out of range, or eps dwarfs the domain: FP64 path.
+struct SplitScale {
+  int e, g, big;
+  int off;  // sources of |1 - |y|^2| > 1 (counted by the record kernel)
+};
+
+// 2^k for |k| <= 1022
+__device__ __forceinline__ double pow2d(int k) {
+  return __longlong_as_double((long long)(1023 + k) << 52);
+}
+
+// X in (-1, 1): x a multiple of 2^-22, y a multiple of 2^-45 with |y| <= 2^-23.
+__device__ __forceinline__ float3 split3(double X) {
+  const double m1 = 1.5 * 1073741824.0;                    // ulp 2^-22
+  const double m2 = 1.5 * 128.0;                           // ulp 2^-45
+  const double h = __dsub_rn(__dadd_rn(X, m1), m1);
+  const double r = __dsub_rn(X, h);
+  const double m = __dsub_rn(__dadd_rn(r, m2), m2);
+  return make_float3(float(h), float(m), float(__dsub_rn(r, m)));
+}
+__device__ __forceinline__ void split2(double v, float& h, float& l) {
+  h = float(v);
+  l = float(v - double(h));
+}
+// 1 - |x|^2 to about 1e-31 absolute, rounded to FP64.
+__device__ __forceinline__ double unit_defect(double x, double y, double z) {
+  double s = 1.0, e = 0.0;
+  const double v[3] = {x, y, z};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double p = __dmul_rn(v[c], v[c]);
+    const double pe = fma(v[c], v[c], -p);
+    const double t = __dsub_rn(s, p);
+    const double bb = __dsub_rn(t, s);
+    e += __dsub_rn(__dsub_rn(s, __dsub_rn(t, bb)), __dadd_rn(p, bb)) - pe;
+    s = t;
+  }
+  return s + e;
+}
+
+__device__ __forceinline__ void two_sum2(u64 a, u64 b, u64& s, u64& e) {
+  s = add2(a, b);
+  const u64 bb = sub2(s, a);
+  e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+__device__ __forceinline__ void two_sum1(float a, float b, float& s, float& e) {
+  s = a + b;
+  const float bb = s - a;
+  e = (a - (s - bb)) + (b - bb);
+}
+__device__ __forceinline__ u64 dup2(float a) { return pk2(a, a); }
+__device__ __forceinline__ u64 pkf2(float2 a) { return pk2(a.x, a.y); }
+
+// Running sum of float pairs: the two lanes' pairs are added first, then a
+// float-pair sum over kSplitRun steps (16 FP32 operations per step), which is
+// merged into a three-float sum.  The rounding of the low words grows with the
+// run's partial sum, so the run is short: 4 steps leave it below the terms' own
+// error (16 steps, or an unbroken three-float sum, left several times it).
+constexpr int kSplitRun = 4;
+struct SplitAcc {
+  float s = 0.f, c = 0.f;
+  float t0 = 0.f, t1 = 0.f, t2 = 0.f;
+  __device__ __forceinline__ void add(u64 h, u64 l) {
+    float h0, h1, l0, l1, e;
+    upk2(h, h0, h1);
+    upk2(l, l0, l1);
+    two_sum1(h0, h1, h0, e);
+    l0 = (l0 + l1) + e;
+    two_sum1(s, h0, s, e);
+    c += l0 + e;
+  }
+  __device__ __forceinline__ void merge() {
+    float e, f;
+    two_sum1(t0, s, t0, e);
+    two_sum1(e, c, e, f);
+    t2 += f;
+    two_sum1(t1, e, t1, f);
+    t2 += f;
+    s = c = 0.f;
+  }
+  __device__ __forceinline__ double value() const { return double(t0) + (double(t1) + double(t2)); }
+};
+
+// log tables: reciprocal f of the interval centre, -log f as a float pair
+// (less ln 2 from sqrt 2 on, where the exponent is one higher); k ln 2 pairs.
+struct SplitLog {
+  float4 m[128];   // f, hi, lo, -
+  float4 k[64];    // (k + offset) ln 2 in three parts for k = -41 .. 22
+};
+constexpr int kSplitLogK0 = -41;
+constexpr int kSplitLogUp = 53;  // intervals from here on lie above sqrt 2
+
+__device__ __forceinline__ void split_log_tables(SplitLog& T, int offset) {
+  for (int i = threadIdx.x; i < 128; i += blockDim.x) {
+    const float f = __frcp_rn(1.f + (float(i) + 0.5f) * (1.f / 128));
+    const double ln2 = 0.69314718055994530942;
+    float h, l;
+    split2(-log(double(f)) - (i >= kSplitLogUp ? ln2 : 0.0), h, l);
+    T.m[i] = make_float4(f, h, l, 0.f);
+  }
+  for (int i = threadIdx.x; i < 64; i += blockDim.x) {
+    const double v = double(i + kSplitLogK0 + offset) * 0.69314718055994530942;
+    float h, l;
+    split2(v, h, l);
+    T.k[i] = make_float4(h, l, float((v - double(h)) - double(l)), 0.f);
+  }
+}
+
+// log(a + al) + offset ln 2 of two values in [2^-40, 2^21] as float pairs.
+__device__ __forceinline__ void split_log2v(const SplitLog& T, u64 a, u64 al, u64& lh, u64& ll) {
+  float a0, a1;
+  upk2(a, a0, a1);
+  const unsigned b0 = __float_as_uint(a0), b1 = __float_as_uint(a1);
+  const int i0 = (b0 >> 16) & 127, i1 = (b1 >> 16) & 127;
+  const float4 e0 = T.m[i0], e1 = T.m[i1];
+  // indexes are kept in range for values outside [2^-40, 2^21] (marked targets)
+  const int x0 = min(max(int(b0 >> 23) - 127 + (i0 >= kSplitLogUp ? 1 : 0) - kSplitLogK0, 0), 63);
+  const int x1 = min(max(int(b1 >> 23) - 127 + (i1 >= kSplitLogUp ? 1 : 0) - kSplitLogK0, 0), 63);
+  const float4 k0 = T.k[x0], k1 = T.k[x1];
+  const u64 m = pk2(__uint_as_float((b0 & 0x7fffffu) | 0x3f800000u),
+                    __uint_as_float((b1 & 0x7fffffu) | 0x3f800000u));
+  const u64 sc = pk2(__uint_as_float(0x7f000000u - (b0 & 0x7f800000u)),
+                     __uint_as_float(0x7f000000u - (b1 & 0x7f800000u)));
+  const u64 f = pk2(e0.x, e1.x);
+  const u64 ml = mul2(al, sc);
+  // t = (m + ml) f - 1, |t| < 2^-7.9
+  const u64 p = mul2(m, f);
+  u64 tl = fma2(ml, f, fma2(m, f, neg2(p)));
+  const u64 t1 = sub2(p, dup2(1.f));
+  const u64 th = add2(t1, tl);
+  tl = sub2(tl, sub2(th, t1));
+  // log1p: th + tl - th^2/2 - th tl + t^3 (1/3 - t/4 + t^2/5 - t^3/6)
+  const u64 nhalf = dup2(-0.5f);
+  const u64 sq = mul2(th, th);
+  const u64 se = fma2(th, th, neg2(sq));
+  u64 P = fma2(th, dup2(-1.f / 6), dup2(0.2f));
+  P = fma2(th, P, dup2(-0.25f));
+  P = fma2(th, P, dup2(1.f / 3));
+  const u64 hs = mul2(sq, nhalf);
+  const u64 r = add2(th, hs);           // |hs| < |th|
+  u64 lo = sub2(hs, sub2(r, th));
+  lo = fma2(se, nhalf, lo);
+  lo = fma2(mul2(sq, th), P, lo);
+  lo = add2(lo, fma2(neg2(th), tl, tl));
+  u64 s, e;
+  two_sum2(pk2(k0.x, k1.x), pk2(e0.y, e1.y), s, e);
+  lo = add2(add2(lo, pk2(k0.z, k1.z)), add2(e, add2(pk2(k0.y, k1.y), pk2(e0.z, e1.z))));
+  two_sum2(s, r, lh, e);
+  ll = add2(lo, e);
+}
+
+// One pair in FP64, the arithmetic of nbody_f64h, added to its partials.
+template <bool WU, bool WP>
+__device__ __forceinline__ void split_pair64(const double4_16a& t, const double4_16a& s,
+                                             double eps2, double* a) {
+  const double arg = eps2 - fma(t.z, s.z, fma(t.y, s.y, fma(t.x, s.x, -1.0)));
+  if (WU) {
+    const double q = div_nr(s.w, arg);
+    a[0] = fma(q, s.x, a[0]);
+    a[1] = fma(q, s.y, a[1]);
+    a[2] = fma(q, s.z, a[2]);
+  }
+  if (WP) a[WU ? 3 : 0] = fma(log(arg), s.w, a[WU ? 3 : 0]);
+}
+// The rare pair of the split loop, out of line.
+template <bool WU, bool WP>
+__device__ __noinline__ void split_near64(const double4_16a* t, const double4_16a* s, double eps2,
+                                          double* a) {
+  split_pair64<WU, WP>(*t, *s, eps2, a);
+}
+
+//   tgt, tself, src, part: as nbody_f64h (sphere forms)
+//   st: SplitTarget per target (ntgt_pad entries)
+//   sp: SplitPair per two sources (nsrc_pad / 2 entries)
+//   SKIP: the pair of tself is left out
+template <bool WU, bool WP, bool SKIP>
+__global__ void __launch_bounds__(kSplitNT, 4)
+    nbody_split(const double4_16a* __restrict__ tgt, const int* __restrict__ tself,
+                const SplitTarget* __restrict__ st, const SplitPair* __restrict__ sp,
+                const double4_16a* __restrict__ src, const SplitScale* __restrict__ scale, int64_t ntgt, int64_t ntgt_pad,
+                int64_t nsrc, int64_t nsrc_pad, int chunk_len, double eps2,
+                double* __restrict__ part, int* err) {
+  constexpr int NC = (WU ? 3 : 0) + (WP ? 1 : 0);
+  __shared__ __align__(128) SplitPair sbuf[2 * kSplitTile];
+  __shared__ __align__(8) uint64_t sbar[2];
+  using Log = typename std::conditional<WP, SplitLog, float4>::type;
+  __shared__ __align__(16) Log slog;
+
+  const int64_t ti = (int64_t)blockIdx.x * kSplitNT + threadIdx.x;
+  const int64_t s0 = (int64_t)blockIdx.y * chunk_len;
+  int64_t slen = nsrc_pad - s0;
+  if (slen > chunk_len) slen = chunk_len;
+  TilePipe<SplitPair, kSplitTile> pipe{sbuf, sbar, sp + s0 / 2, int(slen / (2 * kSplitTile))};
+  pipe.start();
+
+  const SplitScale sc = *scale;
+  const SplitTarget t = st[ti];
+  const int self = SKIP ? tself[ti] : -1;
+  const bool exact = t.exact != 0 || (int64_t(sc.off) * 16 > nsrc && ti < ntgt);
+  // log(arg) = log(arg' 2^(2e)) - ln 2
+  if constexpr (WP) split_log_tables(slog, 2 * sc.e - 1);
+  const u64 XH = dup2(t.x.x), XM = dup2(t.x.y), XL = dup2(t.x.z);
+  const u64 YH = dup2(t.y.x), YM = dup2(t.y.y), YL = dup2(t.y.z);
+  const u64 ZH = dup2(t.z.x), ZM = dup2(t.z.y), ZL = dup2(t.z.z);
+  const u64 CH = dup2(t.ch), CL = dup2(t.cl);
+  SplitAcc acc[NC];
+  double near[NC];  // the pairs evaluated in FP64, in the partials' units
+#pragma unroll
+  for (int k = 0; k < NC; ++k) near[k] = 0.0;
+  // -1/1024 in the scale of arg'; padding targets take out nothing
+  const float tiny = ti < ntgt ? kSplitTiny : -1e30f;
+  const float off = ti < ntgt ? -float(pow2d(-2 * sc.e) / 1024) : -1e30f;
+  const u64 one = dup2(1.f);
+
+  // (a CTA whose targets all do still drains its tiles, without the sums)
+  const bool idle = __syncthreads_and(exact || ti >= ntgt);
+  for (int tl = 0; tl < pipe.ntiles; ++tl) {
+    if (!pipe.acquire(tl)) {
+      pipe.drain(tl, err);
+      return;
+    }
+    const SplitPair* sm = pipe.tile(tl);
+#pragma unroll 1
+    for (int j0 = 0; j0 < kSplitTile && !idle; j0 += kSplitRun) {
+#pragma unroll 1
+      for (int j = j0; j < j0 + kSplitRun; ++j) {
+        const SplitPair s = sm[j];
+        // exact differences, then a float pair
+        u64 dh[3], dl[3], u, v;
+        u = sub2(XH, pkf2(s.xh)), v = sub2(XM, pkf2(s.xm));
+        dh[0] = add2(u, v);
+        dl[0] = add2(sub2(v, sub2(dh[0], u)), sub2(XL, pkf2(s.xl)));
+        u = sub2(YH, pkf2(s.yh)), v = sub2(YM, pkf2(s.ym));
+        dh[1] = add2(u, v);
+        dl[1] = add2(sub2(v, sub2(dh[1], u)), sub2(YL, pkf2(s.yl)));
+        u = sub2(ZH, pkf2(s.zh)), v = sub2(ZM, pkf2(s.zm));
+        dh[2] = add2(u, v);
+        dl[2] = add2(sub2(v, sub2(dh[2], u)), sub2(ZL, pkf2(s.zl)));
+        // |d|^2.  The low words' order matters for the mean error: the residual of
+        // a square has patterned last bits (k^2 mod 4 is 0 or 1) that round down
+        // when summed, so it enters under a product (2 dh dl) that rounds at
+        // random; so do the tiny dl^2, which added to a word would always round
+        // away.  As plain sums the two left 1e-15 of bias, which no averaging
+        // over sources removes.
+        const u64 p0 = mul2(dh[0], dh[0]), p1 = mul2(dh[1], dh[1]), p2 = mul2(dh[2], dh[2]);
+        const u64 sq = fma2(dl[2], dl[2], fma2(dl[0], dl[0], mul2(dl[1], dl[1])));
+        u64 lo = fma2(add2(dh[1], dh[1]), dl[1], sq);
+        lo = add2(lo, fma2(dh[1], dh[1], neg2(p1)));
+        lo = add2(lo, fma2(add2(dh[0], dh[0]), dl[0], fma2(dh[0], dh[0], neg2(p0))));
+        u64 q, e;
+        two_sum2(p0, p1, q, e);
+        lo = add2(lo, e);
+        lo = add2(lo, fma2(add2(dh[2], dh[2]), dl[2], fma2(dh[2], dh[2], neg2(p2))));
+        two_sum2(q, p2, q, e);
+        lo = add2(lo, e);
+        // arg' = |d|^2 + C
+        u64 c, A;
+        two_sum2(CH, pkf2(s.ch), c, e);
+        const u64 cl = add2(add2(CL, pkf2(s.cl)), e);
+        two_sum2(q, c, A, e);
+        u64 Al = add2(lo, add2(e, cl));
+        float a0, a1;
+        upk2(A, a0, a1);
+        // pairs taken out (rare): the closest and those off the sphere,
+        // evaluated in FP64 (with a logarithm also those of a negative arg',
+        // which has none), and the target's own source
+        float c0, c1;
+        upk2(c, c0, c1);
+        bool n0 = (WP ? a0 : fabsf(a0)) < fmaxf(tiny, fmaf(fabsf(c0), 1.f / 32, off));
+        bool n1 = (WP ? a1 : fabsf(a1)) < fmaxf(tiny, fmaf(fabsf(c1), 1.f / 32, off));
+        if (SKIP) {
+          n0 |= s.slot.x == self;
+          n1 |= s.slot.y == self;
+        }
+        u64 gh = pkf2(s.gh), gl = pkf2(s.gl);
+        if (n0 || n1) {
+          if (n0 && s.slot.x >= 0 && !(SKIP && s.slot.x == self))
+            split_near64<WU, WP>(tgt + ti, src + s.slot.x, eps2, near);
+          if (n1 && s.slot.y >= 0 && !(SKIP && s.slot.y == self))
+            split_near64<WU, WP>(tgt + ti, src + s.slot.y, eps2, near);
+          // strength 0 and denominator 1 in the split sum
+          float b0, b1;
+          upk2(Al, b0, b1);
+          a0 = n0 ? 1.f : a0;
+          a1 = n1 ? 1.f : a1;
+          A = pk2(a0, a1);
+          Al = pk2(n0 ? 0.f : b0, n1 ? 0.f : b1);
+          gh = pk2(n0 ? 0.f : s.gh.x, n1 ? 0.f : s.gh.y);
+          gl = pk2(n0 ? 0.f : s.gl.x, n1 ? 0.f : s.gl.y);
+        }
+        if (WU) {
+          // r = -1 / arg': the MUFU's value, one Newton step, its residual
+          u64 r = pk2(rcp_approx(-a0), rcp_approx(-a1));
+          r = fma2(r, fma2(A, r, one), r);
+          e = fma2(Al, r, fma2(A, r, one));
+          const u64 rl = mul2(r, fma2(e, e, e));
+          // the record holds -g: q = g / arg'
+          const u64 qh = mul2(gh, r);
+          u64 ql = fma2(gh, r, neg2(qh));
+          ql = fma2(gh, rl, ql);
+          ql = fma2(gl, r, ql);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const u64 ph = mul2(qh, dh[k]);
+            u64 pl = fma2(qh, dh[k], neg2(ph));
+            pl = fma2(ql, dl[k], fma2(qh, dl[k], pl));
+            pl = fma2(ql, dh[k], pl);
+            acc[k].add(ph, pl);
+          }
+        }
+        if constexpr (WP) {
+          u64 lh, ll;
+          split_log2v(slog, A, Al, lh, ll);
+          const u64 ph = mul2(gh, lh);
+          u64 pl = fma2(gh, lh, neg2(ph));
+          pl = fma2(gh, ll, pl);
+          pl = fma2(gl, lh, pl);
+          acc[NC - 1].add(ph, pl);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c].merge();
+    }
+    pipe.release(tl);
+  }
+
+  double* out = part + (int64_t)blockIdx.y * NC * ntgt_pad;
+  const unsigned lanes = __ballot_sync(0xffffffffu, exact);
+  if (lanes != 0) {
+    // FP64 targets: each by its own thread where they fill half the warp, one
+    // after another by the whole warp where they are few (a lone thread would
+    // hold its warp for 40 times as long)
+    const int64_t j1 = s0 + slen < nsrc ? s0 + slen : nsrc;
+    const int lane = threadIdx.x & 31;
+    const bool own = __popc(lanes) >= 16;
+    for (unsigned rest = own ? 1u : lanes; rest != 0; rest &= rest - 1) {
+      const int b = own ? lane : __ffs(rest) - 1;
+      const int sb = __shfl_sync(0xffffffffu, self, b);
+      const double4_16a x = tgt[ti - lane + b];
+      double a[NC];
+#pragma unroll
+      for (int k = 0; k < NC; ++k) a[k] = 0.0;
+      if (!own || exact) {
+#pragma unroll 2
+        for (int64_t j = s0 + (own ? 0 : lane); j < j1; j += own ? 1 : 32) {
+          const double4_16a y = src[j];
+          if (!(SKIP && j == sb)) split_pair64<WU, WP>(x, y, eps2, a);
+        }
+      }
+      if (!own) {
+#pragma unroll
+        for (int k = 0; k < NC; ++k)
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+      }
+      if (lane == b && exact)
+#pragma unroll
+        for (int k = 0; k < NC; ++k) out[k * ntgt_pad + ti] = a[k];
+    }
+  }
+  if (!exact) {
+    // the sum of g d / arg' in the caller's units; -2 times it equals the sum
+    // of (g / arg) y in the cross product with x
+    if (WU) {
+      const double f = -2.0 * pow2d(sc.g - sc.e);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) near[k] += acc[k].value() * f;
+    }
+    if (WP) near[NC - 1] -= acc[NC - 1].value() * pow2d(sc.g);  // the records hold -g
+#pragma unroll
+    for (int k = 0; k < NC; ++k) out[k * ntgt_pad + ti] = near[k];
+  }
+}
+
+}  // namespace lpm

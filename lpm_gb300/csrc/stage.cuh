@@ -169,16 +169,9 @@ __device__ void combine_t(const PK& k, int64_t t, const double* p, double c0,
                           const double* sg, double* u, double* psi) {
   constexpr int NC = NDIM + (WP ? 1 : 0);
   double a[NC];
-#pragma unroll
-  for (int m = 0; m < NC; ++m) a[m] = 0.0;
   int64_t st;
   const double* b = k.pbase(t, st);
-  const int nch = k.chunks(t);
-  for (int c = 0; c < nch; ++c) {
-    const double* q = b + (int64_t)c * NC * st;
-#pragma unroll
-    for (int m = 0; m < NC; ++m) a[m] += q[m * st];
-  }
+  sum_chunks<NC>(b, k.chunks(t), st, a);
   if (k.mode == M_REF64) {
     if (k.exact) {
       for (int m = 0; m < NDIM; ++m) u[m] = a[m];

@@ -103,6 +103,7 @@ struct lpm_stepper_base {
     src = dalloc(32 * plan.nsrc_pad);  // SrcF32 / double4_16a
     tself = static_cast<int*>(dalloc(sizeof(int) * plan.ntgt_pad));
     part = static_cast<double*>(dalloc(plan.part_bytes()));
+    if (plan.split) plan.split_buf = dalloc(lpm::split_bytes(c, plan.ntgt_pad, plan.nsrc_pad));
     sgbuf = static_cast<double*>(dalloc(sizeof(double) * (8 + 256)));
     // zero the padding records once (never rewritten); tself padding = -1
     zero(tgt, rec * plan.ntgt_pad);
@@ -315,18 +316,19 @@ struct lpm_bve_rk4 : lpm_stepper_base {
     std::memcpy(kk.data(), &g, sizeof(g));
     const void* fd = ff ? static_cast<const void*>(ff->d) : nullptr;
     std::memcpy(kk.data() + sizeof(g), &fd, sizeof(fd));
-    const int64_t nb = (T + 255) / 256;
+    const int th = lpm::sum_threads(T);
+    const int64_t nb = (T + th - 1) / th;
     run(kk, [&]() {
       if (T == 0) return;
-      lpm::k_rk4_begin<<<nb, 256, 0, ctx->stream>>>(g, k, b, P);
+      lpm::k_rk4_begin<<<nb, th, 0, ctx->stream>>>(g, k, b, P);
       ctx->launches++;
       for (int s = 1; s <= 3; ++s) {
         nbody();
-        lpm::k_rk4_stage<<<nb, 256, 0, ctx->stream>>>(g, k, b, P, s);
+        lpm::k_rk4_stage<<<nb, th, 0, ctx->stream>>>(g, k, b, P, s);
         ctx->launches++;
       }
       nbody();
-      lpm::k_rk4_final<<<nb, 256, 0, ctx->stream>>>(g, k, b, P);
+      lpm::k_rk4_final<<<nb, th, 0, ctx->stream>>>(g, k, b, P);
       ctx->launches++;
     });
   }
@@ -356,18 +358,19 @@ struct lpm_ic2d_rk2 : lpm_stepper_base {
     P.sg = sgbuf;
     std::vector<char> kk(sizeof(lpm::Tg));
     std::memcpy(kk.data(), &g, sizeof(g));
-    const int64_t nb = (T + 255) / 256;
+    const int th = lpm::sum_threads(T);
+    const int64_t nb = (T + th - 1) / th;
     run(kk, [&]() {
       if (T == 0) return;
-      lpm::k_rk2_begin<<<nb, 256, 0, ctx->stream>>>(g, k, b, P);
+      lpm::k_rk2_begin<<<nb, th, 0, ctx->stream>>>(g, k, b, P);
       ctx->launches++;
       // the stage-1 stream function is overwritten by the final evaluation
       // (as in Incompressible2DRK2::advance_timestep_impl), so it is not computed
       nbody(false);
-      lpm::k_rk2_mid<<<nb, 256, 0, ctx->stream>>>(g, k, b, P);
+      lpm::k_rk2_mid<<<nb, th, 0, ctx->stream>>>(g, k, b, P);
       ctx->launches++;
       nbody();
-      lpm::k_rk2_final<<<nb, 256, 0, ctx->stream>>>(g, k, b, P);
+      lpm::k_rk2_final<<<nb, th, 0, ctx->stream>>>(g, k, b, P);
       ctx->launches++;
     });
   }

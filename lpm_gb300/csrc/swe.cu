@@ -39,12 +39,6 @@ __device__ __forceinline__ double da(double a, double b) { return __dadd_rn(a, b
 __device__ __forceinline__ double ds(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dd(double a, double b) { return __ddiv_rn(a, b); }
 
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-  u64 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 constexpr int kSweNT = 128;   // targets per CTA
 constexpr int kSweTile = 256;  // sources per shared-memory tile
 constexpr int kSweNC = 9;
