@@ -14,17 +14,16 @@
 // Reducer rules (:559-570): masked sources are skipped; with collocated
 // targets (face sums with eps = 0) the i == j pair is skipped.
 //
-// FP64 in the reference's operation order with non-contracting intrinsics:
-// every term equals the reference's except through exp/log, whose last bits
-// may differ from the host library's.  One CTA = 128 targets x one chunk of
-// the compacted sources (tiles of 256 in shared memory); FP64 partials per
-// (chunk, component, target) are added in fixed order by the epilogue, which
-// also forms the double dot product du/dx^2 + 2 du/dy dv/dx + dv/dy^2.
+// FP64 sums the pair terms as moments of d (k_swe_plane below); FP64 partials
+// per (chunk, component, target) are added in fixed order by the epilogue,
+// which assembles the outputs and the double dot product du/dx^2 +
+// 2 du/dy dv/dx + dv/dy^2.
 #include <algorithm>
 #include <cmath>
 
 #include <cuda_runtime.h>
 
+#include "f64math.cuh"
 #include "lpm_host.hpp"
 #include "nbody.cuh"
 
@@ -37,20 +36,47 @@ namespace {
 __device__ __forceinline__ double dm(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double da(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double ds(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double dd(double a, double b) { return __ddiv_rn(a, b); }
 
 constexpr int kSweNT = 128;   // targets per CTA
-constexpr int kSweTile = 256;  // sources per shared-memory tile
-constexpr int kSweNC = 9;
+constexpr int kSweTile = 256;  // sources per shared-memory tile (FP32)
+// FP64: small tiles and chunks, so that a few thousand points spread evenly
+// (a warp's pair takes 3,500 clocks of its SM sub-partition's FP64 pipe)
+constexpr int kSweTile64 = 64;
 
-struct SweSrc {
+// ---- planar SWE sums, FP64 --------------------------------------------------
+// With r = 1 / R, a = rot r, b = pot r, m = d1^2 - d0^2, the eleven sums
+//   U, V    = sum -a d1 + b d0, sum a d0 + b d1
+//   A1..A3  = sum a r (m, d0 d1, 1),   B1..B3 = sum b r (m, d0 d1, 1)
+//   L       = sum (s_y - s_x) A (40 (1 - p) + 10 p^2 - 2 p^3 / 3) e^-p,
+//             p = |d|^2 / pse_eps^2
+//   P, Q    = sum rot log R, sum pot log R
+// give every output: 2 pi u = U, 2 pi v = V,
+//   2 pi du/dx = 2 A2 + B1 + eps^2 B3,   2 pi du/dy = A1 - eps^2 A3 - 2 B2,
+//   2 pi dv/dx = A1 + eps^2 A3 - 2 B2,   2 pi dv/dy = -2 A2 - B1 + eps^2 B3,
+//   lap = L / (pi pse_eps^2), psi, phi = -P / 4 pi, -Q / 4 pi
+// (R/2 taken from d1^2 and d0^2 pair by pair, so no large sums cancel).
+// The FP64 pipe bounds the kernel: 55 operations per pair (one approximate
+// reciprocal, the logarithm and exponential of f64math.cuh) against about 260
+// for the reference's operation order with its eight divisions, square root
+// and library log and exp: quad level 5, vertices and faces, 19.6 -> 4.7 ms
+// (0.88 of the pipe's measured rate).
+constexpr int kSweNC = 11;
+
+struct __align__(16) SweSrc {
   double x, y, rot, pot, s, area;
-  int slot, pad;
+  int slot, pad[3];
 };
 
+// The last two blocks fill the tables of f64math.cuh.
 __global__ void k_swe_pack(View fx, const double* __restrict__ zeta, const double* __restrict__ sigma,
                            const double* __restrict__ area, const double* __restrict__ sfc,
-                           const int* __restrict__ src2slot, int64_t ns, SweSrc* __restrict__ src) {
+                           const int* __restrict__ src2slot, int64_t ns, SweSrc* __restrict__ src,
+                           F64Tables* __restrict__ tab) {
+  const int tb = int(gridDim.x) - 2;
+  if (int(blockIdx.x) >= tb) {
+    f64_table_entry(tab, (int(blockIdx.x) - tb) * 256 + threadIdx.x);
+    return;
+  }
   const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (k >= ns) return;
   const int64_t j = src2slot[k];
@@ -62,60 +88,75 @@ __global__ void k_swe_pack(View fx, const double* __restrict__ zeta, const doubl
   r.s = sfc[j];
   r.area = area[j];
   r.slot = int(j);
-  r.pad = 0;
+  r.pad[0] = r.pad[1] = r.pad[2] = 0;
   src[k] = r;
 }
+static_assert((1 << kLogBits) == 512, "k_swe_pack fills the tables with two blocks of 256");
 
+__device__ __forceinline__ void load_tables(F64Tables& t, const F64Tables* __restrict__ g) {
+  const auto* s = reinterpret_cast<const double2*>(g);
+  auto* d = reinterpret_cast<double2*>(&t);
+  for (int i = threadIdx.x; i < int(sizeof(F64Tables) / 16); i += blockDim.x) d[i] = s[i];
+}
+
+// COLL: collocated targets, the source in the target's own slot is skipped.
+template <bool COLL>
 __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __restrict__ ts,
                                                       int64_t nt, const SweSrc* __restrict__ src,
-                                                      int64_t ns, int64_t chunk_len, double eps,
-                                                      double pse_eps, int collocated,
+                                                      int64_t ns, int64_t chunk_len, double epssq,
+                                                      double ipse2, const F64Tables* __restrict__ tab,
                                                       double* __restrict__ part, int64_t tpad) {
-  __shared__ SweSrc tile[kSweTile];
+  __shared__ SweSrc tile[kSweTile64];
+  __shared__ F64Tables T;
+  load_tables(T, tab);
   const int64_t i = blockIdx.x * int64_t(kSweNT) + threadIdx.x;
   const int64_t c = blockIdx.y;
   const int64_t j0 = c * chunk_len, j1 = ns < j0 + chunk_len ? ns : j0 + chunk_len;
   const bool valid = i < nt;
   const double x0 = valid ? tx(i, 0) : 0.0, x1 = valid ? tx(i, 1) : 0.0;
   const double si = valid ? ts[i] : 0.0;
-  const double epssq = dm(eps, eps);
-  const double pse2 = dm(pse_eps, pse_eps);
-  const double twopi = 2 * kPI, fourpi = 4 * kPI;
   double r[kSweNC];
 #pragma unroll
   for (int k = 0; k < kSweNC; ++k) r[k] = 0.0;
-  for (int64_t t0 = j0; t0 < j1; t0 += kSweTile) {
-    const int m = int(j1 - t0 < kSweTile ? j1 - t0 : kSweTile);
+  for (int64_t t0 = j0; t0 < j1; t0 += kSweTile64) {
+    const int m = int(j1 - t0 < kSweTile64 ? j1 - t0 : kSweTile64);
     __syncthreads();
-    for (int q = threadIdx.x; q < m; q += kSweNT) tile[q] = src[t0 + q];
+    for (int q = threadIdx.x; q < m * int(sizeof(SweSrc) / 16); q += kSweNT)
+      reinterpret_cast<double2*>(tile)[q] = reinterpret_cast<const double2*>(src + t0)[q];
     __syncthreads();
     if (!valid) continue;
+#pragma unroll 1
     for (int q = 0; q < m; ++q) {
       const SweSrc& y = tile[q];
-      if (collocated && y.slot == i) continue;
-      const double d0 = ds(x0, y.x), d1 = ds(x1, y.y);
-      const double rsq = da(dm(d0, d0), dm(d1, d1));
-      const double R = da(rsq, epssq);
-      const double denom = dm(twopi, R);
-      const double denom2 = dm(kPI, dm(R, R));
-      const double greens = dd(-log(R), fourpi);
-      const double xy = dm(d0, d1);
-      const double d00 = dm(d0, d0), d11 = dm(d1, d1);
-      r[0] = da(r[0], dd(da(dm(-d1, y.rot), dm(d0, y.pot)), denom));
-      r[1] = da(r[1], dd(da(dm(d0, y.rot), dm(d1, y.pot)), denom));
-      r[2] = da(r[2], da(dd(ds(dm(xy, y.rot), dm(d00, y.pot)), denom2), dd(y.pot, denom)));
-      r[3] = da(r[3], ds(dd(ds(dm(d11, y.rot), dm(xy, y.pot)), denom2), dd(y.rot, denom)));
-      r[4] = da(r[4], da(dd(ds(dm(-d00, y.rot), dm(xy, y.pot)), denom2), dd(y.rot, denom)));
-      r[5] = da(r[5], da(dd(ds(dm(-xy, y.rot), dm(d11, y.pot)), denom2), dd(y.pot, denom)));
-      const double e0 = ds(y.x, x0), e1 = ds(y.y, x1);
-      const double pr = dd(__dsqrt_rn(da(dm(e0, e0), dm(e1, e1))), pse_eps);
-      const double p2 = dm(pr, pr);
-      const double p4 = dm(p2, p2);
-      const double pre = ds(da(dm(40.0, ds(1.0, p2)), dm(10.0, p4)), dd(dm(dm(2.0, p2), p4), 3.0));
-      const double lap = dm(pre, dd(exp(-p2), kPI));
-      r[6] = da(r[6], dd(dm(dm(ds(y.s, si), y.area), lap), pse2));
-      r[7] = da(r[7], dm(greens, y.rot));
-      r[8] = da(r[8], dm(greens, y.pot));
+      if (COLL && y.slot == i) continue;
+      const double d0 = x0 - y.x, d1 = x1 - y.y;
+      const double d00 = d0 * d0, d11 = d1 * d1;
+      const double rsq = d00 + d11, R = rsq + epssq;
+      double w, lg;
+      if (f64_plain(R)) {
+        w = f64_rcp(R);
+        lg = f64_log(T, R);
+      } else {  // coincident points, out-of-range values
+        w = 1.0 / R;
+        lg = log(R);
+      }
+      const double a = y.rot * w, b = y.pot * w;
+      r[0] = fma(-a, d1, fma(b, d0, r[0]));
+      r[1] = fma(a, d0, fma(b, d1, r[1]));
+      const double a2 = a * w, b2 = b * w, md = d11 - d00, xy = d0 * d1;
+      r[2] = fma(a2, md, r[2]);
+      r[3] = fma(a2, xy, r[3]);
+      r[4] += a2;
+      r[5] = fma(b2, md, r[5]);
+      r[6] = fma(b2, xy, r[6]);
+      r[7] += b2;
+      const double p = rsq * ipse2;
+      double pre = fma(p, -2.0 / 3, 10.0);
+      pre = fma(p, pre, -40.0);
+      pre = fma(p, pre, 40.0);
+      if (!(p >= 746.0)) r[8] = fma((y.s - si) * y.area, f64_mul_exp_neg(T, pre, p), r[8]);
+      r[9] = fma(y.rot, lg, r[9]);
+      r[10] = fma(y.pot, lg, r[10]);
     }
   }
   if (!valid) return;
@@ -129,29 +170,37 @@ struct SweOut {
   int do_velocity;
 };
 
+// Outputs of one target from its velocity sums (times 2 pi), gradients,
+// Laplacian and stream/potential functions.
+__device__ __forceinline__ void swe_write(const SweOut& o, int64_t i, double u, double v, double g00,
+                                          double g01, double g10, double g11, double lap, double psi,
+                                          double phi) {
+  if (o.do_velocity) {
+    o.u(i, 0) = u;
+    o.u(i, 1) = v;
+  }
+  // square(du/dx) + 2 du/dy dv/dx + square(dv/dy)
+  o.ddot[i] = da(da(dm(g00, g00), dm(dm(2.0, g01), g10)), dm(g11, g11));
+  o.du1dx1[i] = g00;
+  o.du1dx2[i] = g01;
+  o.du2dx1[i] = g10;
+  o.du2dx2[i] = g11;
+  o.laps[i] = lap;
+  o.psi[i] = psi;
+  o.phi[i] = phi;
+}
+
 __global__ void k_swe_out(const double* __restrict__ part, int nchunks, int64_t tpad, int64_t nt,
-                          SweOut o) {
+                          double epssq, double pse_eps, SweOut o) {
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= nt) return;
   double s[kSweNC];
-#pragma unroll
-  for (int k = 0; k < kSweNC; ++k) s[k] = 0.0;
-  for (int c = 0; c < nchunks; ++c)
-#pragma unroll
-    for (int k = 0; k < kSweNC; ++k) s[k] = da(s[k], part[(int64_t(c) * kSweNC + k) * tpad + i]);
-  if (o.do_velocity) {
-    o.u(i, 0) = s[0];
-    o.u(i, 1) = s[1];
-  }
-  // square(du/dx) + 2 du/dy dv/dx + square(dv/dy)
-  o.ddot[i] = da(da(dm(s[2], s[2]), dm(dm(2.0, s[3]), s[4])), dm(s[5], s[5]));
-  o.du1dx1[i] = s[2];
-  o.du1dx2[i] = s[3];
-  o.du2dx1[i] = s[4];
-  o.du2dx2[i] = s[5];
-  o.laps[i] = s[6];
-  o.psi[i] = s[7];
-  o.phi[i] = s[8];
+  sum_chunks<kSweNC>(part + i, nchunks, tpad, s);
+  const double i2pi = 0.5 / kPI, i4pi = 0.25 / kPI;
+  const double ea = epssq * s[4], eb = epssq * s[7], a2 = 2.0 * s[3], b2 = 2.0 * s[6];
+  swe_write(o, i, s[0] * i2pi, s[1] * i2pi, (a2 + s[5] + eb) * i2pi, (s[2] - ea - b2) * i2pi,
+            (s[2] + ea - b2) * i2pi, (eb - a2 - s[5]) * i2pi, s[8] / (kPI * pse_eps * pse_eps),
+            -s[9] * i4pi, -s[10] * i4pi);
 }
 
 // ---- planar SWE sums, FP32 compensated (context precision LPM_FP32C) ------
@@ -335,23 +384,11 @@ __global__ void k_swe_plane32_out(const double* __restrict__ part, int nchunks, 
 #pragma unroll
     for (int k = 0; k < kPl32NC; ++k) w[k] += part[(int64_t(c) * kPl32NC + k) * tpad + i];
   const double ipi = 1.0 / kPI, i2pi = 0.5 / kPI;
-  if (o.do_velocity) {
-    o.u(i, 0) = (w[2] - w[1]) * i2pi;
-    o.u(i, 1) = (w[0] + w[3]) * i2pi;
-  }
-  const double g00 = (w[7] - w[9]) * ipi + w[5] * i2pi;
-  const double g01 = (w[8] - w[10]) * ipi - w[4] * i2pi;
-  const double g10 = -(w[6] + w[10]) * ipi + w[4] * i2pi;
-  const double g11 = -(w[7] + w[11]) * ipi + w[5] * i2pi;
-  o.ddot[i] = da(da(dm(g00, g00), dm(dm(2.0, g01), g10)), dm(g11, g11));
-  o.du1dx1[i] = g00;
-  o.du1dx2[i] = g01;
-  o.du2dx1[i] = g10;
-  o.du2dx2[i] = g11;
-  o.laps[i] = w[12] * ipi / (pse_eps * pse_eps);
   const double k = -0.6931471805599453 / (4 * kPI);
-  o.psi[i] = k * w[13];
-  o.phi[i] = k * w[14];
+  swe_write(o, i, (w[2] - w[1]) * i2pi, (w[0] + w[3]) * i2pi, (w[7] - w[9]) * ipi + w[5] * i2pi,
+            (w[8] - w[10]) * ipi - w[4] * i2pi, -(w[6] + w[10]) * ipi + w[4] * i2pi,
+            -(w[7] + w[11]) * ipi + w[5] * i2pi, w[12] * ipi / (pse_eps * pse_eps), k * w[13],
+            k * w[14]);
 }
 
 // ---- spherical SWE sums ----------------------------------------------------
@@ -365,22 +402,26 @@ __global__ void k_swe_plane32_out(const double* __restrict__ part, int nchunks, 
 //     gkz = D [y]x + c v^T,          v = (1 + eps^2) x - y
 //     gks = -v w^T - D s P,          w = P y = y - s x
 //   (w - D x = -v because s + D = 1 + eps^2).
-// Per target the terms linear in [y]x and P are summed as a vector and a
-// scalar and applied once:
-//   M = sum_j (R c) v^T - (Q v) w^T + [sum_j rot y / (4 pi D)]x
-//       - (sum_j s pot / (4 pi D)) P,      R, Q = rot, pot / (4 pi D^2).
+// With d = x - y every term is a moment of d (c = d cross x, v = eps^2 x + d,
+// w = (1 - s) x - d, identically): writing sz, ss = rot, pot / (4 pi D) and
+// R, Q = rot, pot / (4 pi D^2), the 28 sums
+//   A, B = sum sz d, ss d;  U1, V1 = sum R d, Q d;  U2, V2 = sum R, Q d d^T;
+//   Z, G = sum sz, ss;  H = sum ss (1 - s);  K = sum Q
+// give, with O = sum Q (1 - s) = G - eps^2 K and N = B - eps^2 V1,
+//   u = A x x - B + H x
+//   M = eps^2 (U1 x x) x^T + [U2 columns] x x + V2 - N x^T + eps^2 x V1^T
+//       - eps^2 O x x^T + [Z x - A]x - (G - H) P.
 // FP64: s and D = (1 - s) + eps^2 unfused in the reference's order (D is
 // the ill-conditioned quantity: a one-ulp change of s moves a near pair's D by
 // ~1e-16 / D relative), everything after it contracted, one reciprocal of D per
-// pair (Newton-Raphson from an FP32 seed, two steps: relative error below
-// 1e-28 before the final rounding); about 66 FP64 instructions per pair
-// against ~210 for the non-contracted three-division form.  Agreement with
-// the oracle (which keeps the reference's operation order) is ~1e-14
-// relative.
-constexpr int kSphNC = 16;  // u[3], Mr[9], Yd[3], G
+// pair.  The FP64 pipe bounds the kernel: 51 operations per pair (66 in the form
+// that added c v^T, v w^T, u term by term): icosahedral level 5, vertices and
+// faces, 96.5 -> 81.8 ms (0.91 of the pipe's measured rate); level 2, where
+// 64-source chunks instead of 256-source ones fill the SMs, 1.31 -> 0.38 ms.
+constexpr int kSphNC = 28;  // A3 B3 U1[3] V1[3] U2[6] V2[6] Z G H K
 
-struct SphSrc {
-  double x, y, z, rot, pot;
+struct __align__(16) SphSrc {
+  double x, y, z, rot, pot;  // strengths over 4 pi
   int slot, pad;
 };
 
@@ -395,26 +436,21 @@ __global__ void k_swe_sphere_pack(View fx, const double* __restrict__ zeta,
   r.x = fx(j, 0);
   r.y = fx(j, 1);
   r.z = fx(j, 2);
-  r.rot = -zeta[j] * area[j];
-  r.pot = -sigma[j] * area[j];
+  const double inv4pi = 1.0 / (4 * kPI);
+  r.rot = -zeta[j] * area[j] * inv4pi;
+  r.pot = -sigma[j] * area[j] * inv4pi;
   r.slot = int(j);
   r.pad = 0;
   src[k] = r;
 }
 
-// 1/d by Newton-Raphson, r <- r + r (1 - d r), from the FP32 reciprocal.
-__device__ __forceinline__ double recip_nr(double d) {
-  double r = double(__frcp_rn(float(d)));
-  r = fma(r, fma(-d, r, 1.0), r);
-  return fma(r, fma(-d, r, 1.0), r);
-}
-
+// COLL: collocated targets, the source in the target's own slot is skipped.
+template <bool COLL>
 __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
                                                        const SphSrc* __restrict__ src, int64_t ns,
-                                                       int64_t chunk_len, double eps,
-                                                       int collocated, double* __restrict__ part,
-                                                       int64_t tpad) {
-  __shared__ SphSrc tile[kSweTile];
+                                                       int64_t chunk_len, double epssq,
+                                                       double* __restrict__ part, int64_t tpad) {
+  __shared__ SphSrc tile[kSweTile64];
   const int64_t i = blockIdx.x * int64_t(kSweNT) + threadIdx.x;
   const int64_t c = blockIdx.y;
   const int64_t j0 = c * chunk_len, j1 = ns < j0 + chunk_len ? ns : j0 + chunk_len;
@@ -422,50 +458,49 @@ __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
   double x[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) x[a] = valid ? tx(i, a) : 0.0;
-  const double epssq = eps * eps;
-  const double e1 = 1.0 + epssq;
-  const double inv4pi = 1.0 / (4 * kPI);
-  const double ex[3] = {e1 * x[0], e1 * x[1], e1 * x[2]};
   double r[kSphNC];
 #pragma unroll
   for (int k = 0; k < kSphNC; ++k) r[k] = 0.0;
-  for (int64_t t0 = j0; t0 < j1; t0 += kSweTile) {
-    const int m = int(j1 - t0 < kSweTile ? j1 - t0 : kSweTile);
+  for (int64_t t0 = j0; t0 < j1; t0 += kSweTile64) {
+    const int m = int(j1 - t0 < kSweTile64 ? j1 - t0 : kSweTile64);
     __syncthreads();
-    for (int q = threadIdx.x; q < m; q += kSweNT) tile[q] = src[t0 + q];
+    for (int q = threadIdx.x; q < m * int(sizeof(SphSrc) / 16); q += kSweNT)
+      reinterpret_cast<double2*>(tile)[q] = reinterpret_cast<const double2*>(src + t0)[q];
     __syncthreads();
     if (!valid) continue;
-#pragma unroll 2
+#pragma unroll 1
     for (int q = 0; q < m; ++q) {
-      const SphSrc& sr = tile[q];
-      if (collocated && sr.slot == i) continue;
-      const double y[3] = {sr.x, sr.y, sr.z};
-      // x.y unfused in the reference's order: D = 1 - s cancels, and its
-      // rounding is the reference's
-      const double s = da(da(dm(x[0], y[0]), dm(x[1], y[1])), dm(x[2], y[2]));
-      const double D = da(ds(1.0, s), epssq);
-      const double rd = recip_nr(D);
-      const double inv1 = rd * inv4pi;  // 1 / (4 pi D)
-      const double den2 = inv1 * rd;    // 1 / (4 pi D^2)
-      const double sz = sr.rot * inv1, ss = sr.pot * inv1;
-      const double R = sr.rot * den2, Q = sr.pot * den2;
-      const double cr[3] = {fma(x[1], y[2], -x[2] * y[1]), fma(x[2], y[0], -x[0] * y[2]),
-                            fma(x[0], y[1], -x[1] * y[0])};
-      double w[3], v[3];
+      const SphSrc& y = tile[q];
+      if (COLL && y.slot == i) continue;
+      // x.y unfused in the reference's order: 1 - s cancels, and its rounding
+      // is the reference's
+      const double s = da(da(dm(x[0], y.x), dm(x[1], y.y)), dm(x[2], y.z));
+      const double om = ds(1.0, s), D = da(om, epssq);
+      const double rd = f64_plain(fabs(D)) ? f64_rcp(D) : 1.0 / D;
+      const double d[3] = {x[0] - y.x, x[1] - y.y, x[2] - y.z};
+      const double sz = y.rot * rd, ss = y.pot * rd;
+      const double R = sz * rd, Q = ss * rd;
+      double rr[3], qq[3];
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        w[a] = fma(-s, x[a], y[a]);
-        v[a] = ex[a] - y[a];
-        r[a] = fma(cr[a], sz, fma(w[a], ss, r[a]));
-        r[12 + a] = fma(sz, y[a], r[12 + a]);
+        r[a] = fma(sz, d[a], r[a]);
+        r[3 + a] = fma(ss, d[a], r[3 + a]);
+        rr[a] = R * d[a];
+        qq[a] = Q * d[a];
+        r[6 + a] += rr[a];
+        r[9 + a] += qq[a];
       }
-      r[15] = fma(ss, s, r[15]);
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const double al = R * cr[a], be = Q * v[a];
+      for (int a = 0, k = 0; a < 3; ++a)
 #pragma unroll
-        for (int b = 0; b < 3; ++b) r[3 + 3 * a + b] = fma(al, v[b], fma(-be, w[b], r[3 + 3 * a + b]));
-      }
+        for (int b = a; b < 3; ++b, ++k) {
+          r[12 + k] = fma(rr[a], d[b], r[12 + k]);
+          r[18 + k] = fma(qq[a], d[b], r[18 + k]);
+        }
+      r[24] += sz;
+      r[25] += ss;
+      r[26] = fma(ss, om, r[26]);
+      r[27] += Q;
     }
   }
   if (!valid) return;
@@ -474,32 +509,54 @@ __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
 }
 
 __global__ void k_swe_sphere_out(const double* __restrict__ part, int nchunks, int64_t tpad,
-                                 View tx, int64_t nt, View u, double* __restrict__ ddot,
+                                 View tx, int64_t nt, double eps2, View u, double* __restrict__ ddot,
                                  double* __restrict__ grad, int do_velocity) {
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= nt) return;
   double s[kSphNC];
 #pragma unroll
   for (int k = 0; k < kSphNC; ++k) s[k] = 0.0;
+#pragma unroll 2
   for (int c = 0; c < nchunks; ++c)
 #pragma unroll
     for (int k = 0; k < kSphNC; ++k) s[k] += part[(int64_t(c) * kSphNC + k) * tpad + i];
-  if (do_velocity) {
-    u(i, 0) = s[0];
-    u(i, 1) = s[1];
-    u(i, 2) = s[2];
-  }
   const double x[3] = {tx(i, 0), tx(i, 1), tx(i, 2)};
-  const double* Yd = s + 12;
-  const double Yx[9] = {0.0, -Yd[2], Yd[1], Yd[2], 0.0, -Yd[0], -Yd[1], Yd[0], 0.0};
+  const double *A = s, *B = s + 3, *U1 = s + 6, *V1 = s + 9, *U2 = s + 12, *V2 = s + 18;
+  const double Z = s[24], G = s[25], H = s[26];
+  const int sym[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};  // (a, b) -> packed symmetric index
+  auto cross = [](const double* p, const double* q, double* o) {
+    o[0] = p[1] * q[2] - p[2] * q[1];
+    o[1] = p[2] * q[0] - p[0] * q[2];
+    o[2] = p[0] * q[1] - p[1] * q[0];
+  };
+  if (do_velocity) {
+    double ax[3];
+    cross(A, x, ax);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) u(i, a) = ax[a] - B[a] + H * x[a];
+  }
+  const double O = G - eps2 * s[27];
+  double u1x[3], zy[3], N[3];
+  cross(U1, x, u1x);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    zy[a] = Z * x[a] - A[a];
+    N[a] = B[a] - eps2 * V1[a];
+  }
+  const double Yx[9] = {0.0, -zy[2], zy[1], zy[2], 0.0, -zy[0], -zy[1], zy[0], 0.0};
   double M[9];
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+  for (int b = 0; b < 3; ++b) {
+    const double col[3] = {U2[sym[b]], U2[sym[3 + b]], U2[sym[6 + b]]};
+    double t1[3];
+    cross(col, x, t1);
 #pragma unroll
-    for (int b = 0; b < 3; ++b) {
+    for (int a = 0; a < 3; ++a) {
       const double P = (a == b ? 1.0 : 0.0) - x[a] * x[b];
-      M[3 * a + b] = s[3 + 3 * a + b] + Yx[3 * a + b] - s[15] * P;
+      M[3 * a + b] = eps2 * (u1x[a] * x[b] + x[a] * V1[b] - O * x[a] * x[b]) + t1[a] +
+                     V2[sym[3 * a + b]] - N[a] * x[b] + Yx[3 * a + b] - (G - H) * P;
     }
+  }
   // sum_ij M_ij M_ji in the functors' loop order
   double dsum = 0.0;
 #pragma unroll
@@ -755,8 +812,8 @@ __global__ void k_swe_sphere32_out(const double* __restrict__ part, int nchunks,
 
 // Scratch and chunking shared by the four SWE paths: 128 targets per CTA,
 // sources compacted (masked slots dropped) and split into chunks of whole
-// 256-source tiles, about four waves of CTAs; ncomp FP64 partials per
-// (chunk, target), added in fixed order by the epilogue.
+// tiles, about eight waves of CTAs; ncomp FP64 partials per (chunk, target),
+// added in fixed order by the epilogue.
 struct SwePlan {
   int64_t nb = 0, tpad = 0, ns = 0, chunk_len = 0;
   int nchunks = 1;
@@ -768,17 +825,17 @@ struct SwePlan {
 };
 
 SwePlan swe_plan(lpm_context& ctx, const uint8_t* mask, int64_t nt, int64_t nf, size_t rec_bytes,
-                 int ncomp, bool want_slot) {
+                 int ncomp, bool want_slot, int tile) {
   SwePlan p;
   ctx.arena.reset();
   p.nb = (nt + kSweNT - 1) / kSweNT;
   p.tpad = p.nb * kSweNT;
   const int64_t want = std::max<int64_t>(1, (int64_t(ctx.num_sms) * 4 * 8 + p.nb - 1) / p.nb);
   const int64_t nch_max =
-      std::max<int64_t>(1, std::min<int64_t>(want, (nf + kSweTile - 1) / kSweTile));
+      std::max<int64_t>(1, std::min<int64_t>(want, (nf + tile - 1) / tile));
   ctx.arena.reserve(sizeof(int) * (3 * size_t(nf) + 2 * size_t(nf) / 1024 + 8) +
                     rec_bytes * size_t(nf) + sizeof(double) * ncomp * size_t(nch_max) * p.tpad +
-                    8 * 4096);
+                    sizeof(F64Tables) + 8 * 4096);
   int* slot2src = static_cast<int*>(ctx.arena.take(sizeof(int) * std::max<int64_t>(nf, 1)));
   p.src2slot = static_cast<int*>(ctx.arena.take(sizeof(int) * std::max<int64_t>(nf, 1)));
   p.ns = compact_sources(ctx, mask, nf, slot2src, p.src2slot);
@@ -786,7 +843,7 @@ SwePlan swe_plan(lpm_context& ctx, const uint8_t* mask, int64_t nt, int64_t nf, 
   p.src = ctx.arena.take(rec_bytes * size_t(p.ns + 1));
   if (want_slot) p.slot = static_cast<int*>(ctx.arena.take(sizeof(int) * size_t(p.ns + 1)));
   int64_t len = (p.ns + nch_max - 1) / nch_max;
-  p.chunk_len = std::max<int64_t>(kSweTile, (len + kSweTile - 1) / kSweTile * kSweTile);
+  p.chunk_len = std::max<int64_t>(tile, (len + tile - 1) / tile * tile);
   p.nchunks = int(std::max<int64_t>(1, (p.ns + p.chunk_len - 1) / p.chunk_len));
   p.part = static_cast<double*>(ctx.arena.take(sizeof(double) * ncomp * size_t(p.nchunks) * p.tpad));
   return p;
@@ -800,7 +857,7 @@ void swe_sphere_sums32(lpm_context& ctx, View tx, int64_t nt, View fx, const dou
                        int do_velocity) {
   // one 64-byte pair record per two sources (32 bytes per source, plus one
   // dummy for an odd count); the pair slots take the plan's slot array
-  const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(SphPair32) / 2, kSph32NC, true);
+  const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(SphPair32) / 2, kSph32NC, true, kSweTile);
   auto* src = static_cast<SphPair32*>(p.src);
   auto* pslot = reinterpret_cast<int2*>(p.slot);
   if (p.ns > 0) {
@@ -833,17 +890,22 @@ void swe_sphere_sums(lpm_context& ctx, View tx, int64_t nt, View fx, const doubl
                       do_velocity);
     return;
   }
-  const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(SphSrc), kSphNC, false);
+  const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(SphSrc), kSphNC, false, kSweTile64);
   auto* src = static_cast<SphSrc*>(p.src);
   if (p.ns > 0) {
     k_swe_sphere_pack<<<blocks256(p.ns), 256, 0, ctx.stream>>>(fx, zeta, sigma, area, p.src2slot,
                                                                p.ns, src);
     ctx.launches++;
   }
-  k_swe_sphere<<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, nt, src, p.ns, p.chunk_len, eps,
-                                                    collocated ? 1 : 0, p.part, p.tpad);
-  k_swe_sphere_out<<<blocks256(nt), 256, 0, ctx.stream>>>(p.part, p.nchunks, p.tpad, tx, nt, u,
-                                                          ddot, grad, do_velocity);
+  if (collocated)
+    k_swe_sphere<true><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, nt, src, p.ns, p.chunk_len,
+                                                            eps * eps, p.part, p.tpad);
+  else
+    k_swe_sphere<false><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, nt, src, p.ns, p.chunk_len,
+                                                             eps * eps, p.part, p.tpad);
+  const unsigned th = unsigned(sum_threads(nt));
+  k_swe_sphere_out<<<unsigned((nt + th - 1) / th), th, 0, ctx.stream>>>(
+      p.part, p.nchunks, p.tpad, tx, nt, eps * eps, u, ddot, grad, do_velocity);
   ctx.launches += 2;
   LPM_CUDA(cudaGetLastError());
 }
@@ -860,7 +922,7 @@ void swe_plane_sums32(lpm_context& ctx, View tx, const double* ts, int64_t nt, V
                       const uint8_t* mask, const double* sfc, int64_t nf, double eps,
                       double pse_eps, bool collocated, const SweOut& out) {
   // one 80-byte pair record per two sources (plus one dummy for an odd count)
-  const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(PlPair32) / 2, kPl32NC, false);
+  const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(PlPair32) / 2, kPl32NC, false, kSweTile);
   auto* src = static_cast<PlPair32*>(p.src);
   if (p.ns > 0) {
     k_swe_plane32_pack<<<blocks256((p.ns + 1) / 2), 256, 0, ctx.stream>>>(
@@ -890,16 +952,22 @@ void swe_plane_sums(lpm_context& ctx, View tx, const double* ts, int64_t nt, Vie
                      collocated, out);
     return;
   }
-  const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(SweSrc), kSweNC, false);
+  const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(SweSrc), kSweNC, false, kSweTile64);
   auto* src = static_cast<SweSrc*>(p.src);
-  if (p.ns > 0) {
-    k_swe_pack<<<blocks256(p.ns), 256, 0, ctx.stream>>>(fx, zeta, sigma, area, sfc, p.src2slot,
-                                                        p.ns, src);
-    ctx.launches++;
-  }
-  k_swe_plane<<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, ts, nt, src, p.ns, p.chunk_len, eps, pse_eps,
-                                                   collocated ? 1 : 0, p.part, p.tpad);
-  k_swe_out<<<blocks256(nt), 256, 0, ctx.stream>>>(p.part, p.nchunks, p.tpad, nt, out);
+  auto* tab = static_cast<F64Tables*>(ctx.arena.take(sizeof(F64Tables)));
+  k_swe_pack<<<blocks256(p.ns) + 2, 256, 0, ctx.stream>>>(fx, zeta, sigma, area, sfc, p.src2slot,
+                                                          p.ns, src, tab);
+  ctx.launches++;
+  const double epssq = eps * eps, ipse2 = 1.0 / (pse_eps * pse_eps);
+  if (collocated)
+    k_swe_plane<true><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, ts, nt, src, p.ns, p.chunk_len, epssq,
+                                                           ipse2, tab, p.part, p.tpad);
+  else
+    k_swe_plane<false><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, ts, nt, src, p.ns, p.chunk_len,
+                                                            epssq, ipse2, tab, p.part, p.tpad);
+  const unsigned th = unsigned(sum_threads(nt));
+  k_swe_out<<<unsigned((nt + th - 1) / th), th, 0, ctx.stream>>>(p.part, p.nchunks, p.tpad, nt, epssq,
+                                                                pse_eps, out);
   ctx.launches += 2;
   LPM_CUDA(cudaGetLastError());
 }
