@@ -422,13 +422,13 @@ __global__ void __launch_bounds__(128) k_ff_eval(
 }  // namespace
 
 FFDevice::~FFDevice() {
-  for (void* p : allocs) cudaFree(p);
+  for (auto& c : caps) cudaFree(*c.first);
 }
-void* FFDevice::alloc(size_t bytes) {
-  void* p = nullptr;
-  LPM_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 256)));
-  allocs.push_back(p);
-  return p;
+void FFDevice::reserve(void** p, size_t bytes) {
+  if (*p) cudaFree(*p);  // waits for the device
+  *p = nullptr;
+  caps[p] = 0;
+  LPM_CUDA(cudaMalloc(p, bytes));
 }
 
 void ff_cells(lpm_context& ctx, const float4* ys, const int4* cells, int ncells, float* cd) {
@@ -467,49 +467,22 @@ lpm_farfield::~lpm_farfield() {
 
 bool lpm_farfield::built() const { return d != nullptr && d->ncells > 0; }
 
-void lpm_farfield::build(const double* src_xyz, int64_t nsrc, const double* tgt_xyz, int64_t ntgt) {
+void lpm_farfield::enter() {
   using namespace lpm;
-  TreeTopo tp = build_tree(src_xyz, nsrc, tgt_xyz, ntgt, leaf_max);
+  if (used && last_stream != ctx->stream) LPM_CUDA(cudaDeviceSynchronize());
+  last_stream = ctx->stream;
+  used = true;
+}
+
+void lpm_farfield::build(const double* src, int src_stride, int64_t nsrc, const double* tgt,
+                         int tgt_stride, int64_t ntgt) {
+  using namespace lpm;
+  enter();
   ff_prepare_kernels();
-  FFDevice* nd = new FFDevice();
-  try {
-    nd->nsrc = nsrc;
-    nd->ntgt = ntgt;
-    nd->ncells = int(tp.start.size());
-    nd->nblocks = tp.nblocks;
-    double r2 = 0;
-    for (int64_t i = 0; i < ntgt; ++i)
-      r2 = std::max(r2, tgt_xyz[3 * i] * tgt_xyz[3 * i] + tgt_xyz[3 * i + 1] * tgt_xyz[3 * i + 1] +
-                            tgt_xyz[3 * i + 2] * tgt_xyz[3 * i + 2]);
-    // targets move between tree builds: keep a generous margin
-    nd->rmax = float(1.1 * std::sqrt(r2) + 0.1);
-    nd->perm = static_cast<int*>(nd->alloc(sizeof(int) * nsrc));
-    nd->tslot = static_cast<int*>(nd->alloc(sizeof(int) * kTargetBlock * size_t(std::max<int64_t>(nd->nblocks, 1))));
-    nd->cells = static_cast<int4*>(nd->alloc(sizeof(int4) * nd->ncells));
-    nd->ys = static_cast<float4*>(nd->alloc(sizeof(float4) * nsrc));
-    nd->cd = static_cast<float*>(nd->alloc(sizeof(float) * kCellF * size_t(nd->ncells)));
-    nd->xt = static_cast<float4*>(nd->alloc(sizeof(float4) * kTargetBlock * size_t(nd->nblocks)));
-    nd->box = static_cast<float4*>(nd->alloc(sizeof(float4) * size_t(nd->nblocks)));
-    nd->far = static_cast<int*>(nd->alloc(sizeof(int) * kFarCap * size_t(nd->nblocks)));
-    nd->near = static_cast<int*>(nd->alloc(sizeof(int) * kNearCap * size_t(nd->nblocks)));
-    nd->lrn = static_cast<int*>(nd->alloc(sizeof(int) * kLearnCap * size_t(nd->nblocks)));
-    nd->cnt = static_cast<int4*>(nd->alloc(sizeof(int4) * size_t(nd->nblocks)));
-    nd->counter = static_cast<int*>(nd->alloc(sizeof(int) * 4));
-    std::vector<int4> ci(nd->ncells);
-    for (int i = 0; i < nd->ncells; ++i) ci[i] = make_int4(tp.start[i], tp.count[i], tp.child0[i], tp.nchild[i]);
-    cudaStream_t st = ctx->stream;
-    LPM_CUDA(cudaMemcpyAsync(nd->perm, tp.perm.data(), sizeof(int) * nsrc, cudaMemcpyHostToDevice, st));
-    if (nd->nblocks > 0)
-      LPM_CUDA(cudaMemcpyAsync(nd->tslot, tp.tslot.data(), sizeof(int) * tp.tslot.size(),
-                               cudaMemcpyHostToDevice, st));
-    LPM_CUDA(cudaMemcpyAsync(nd->cells, ci.data(), sizeof(int4) * nd->ncells, cudaMemcpyHostToDevice, st));
-    LPM_CUDA(cudaStreamSynchronize(st));
-  } catch (...) {
-    delete nd;
-    throw;
-  }
-  delete d;
-  d = nd;
+  if (!d) d = new FFDevice();
+  ++generation;
+  d->ncells = 0;  // not built until the end
+  build_tree_device(*ctx, *d, src, src_stride, nsrc, tgt, tgt_stride, ntgt, leaf_max);
 }
 
 void lpm_farfield::evaluate(const void* tgt, const void* src, double* wout, int64_t wstride,

@@ -85,12 +85,22 @@ struct lpm_farfield {
   int64_t last_far = 0, last_near = 0, last_learn = 0, last_fallback = 0, last_rows = 0;
   // optional CUDA-event timing of evaluations (not inside graph capture)
   bool timing = false;
+  bool used = false;
+  void* last_stream = nullptr;
   std::vector<void*> events;  // cudaEvent_t triples: start, tree done, network done
   void timings(double* tree_ms, double* net_ms, int64_t* evals);
 
   ~lpm_farfield();
-  // Tree over the sources (nsrc x 3, host) and targets (ntgt x 3, host).
-  void build(const double* src_xyz, int64_t nsrc, const double* tgt_xyz, int64_t ntgt);
+  // Tree over the sources and targets: device positions, rows `stride` doubles
+  // apart.  The caller has reserved lpm::tree_build_bytes() in the context's arena
+  // beyond what it has taken.
+  void build(const double* src, int src_stride, int64_t nsrc, const double* tgt, int tgt_stride,
+             int64_t ntgt);
+  // The tree's buffers are reused from build to build: a caller that switched the
+  // context to another stream waits for the work queued on the old one (outside
+  // stream capture).
+  void enter();
+  int64_t generation = 0;  // builds so far
   bool built() const;
   // w[c * wstride + t] = sum over sources of g (x_t - y) / (|x_t - y|^2 + c0)
   // up to terms parallel to x_t (the chord-form sum whose cross product with

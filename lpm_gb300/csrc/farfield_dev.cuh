@@ -2,7 +2,9 @@
 // entry points shared by farfield.cu and mlp.cu.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
+#include <map>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -26,10 +28,30 @@ struct FFDevice {
   int *far = nullptr, *near = nullptr, *lrn = nullptr;  // per-block lists
   int4* cnt = nullptr;    // (far, near, learned, overflow) per block
   int* counter = nullptr; // [0] work counter of the network kernel, [2..3] rows (u64)
-  std::vector<void*> allocs;
   ~FFDevice();
-  void* alloc(size_t bytes);
+  // Room for n elements; a later build that needs no more keeps the buffer (an
+  // allocation and a release per buffer and build took 1 ms of a far-field call).
+  // Contents are lost when it grows.
+  template <class T>
+  void grow(T*& p, size_t n) {
+    size_t& cap = caps[reinterpret_cast<void**>(&p)];
+    const size_t bytes = (n * sizeof(T) + 255) / 256 * 256;
+    if (p && bytes <= cap) return;
+    reserve(reinterpret_cast<void**>(&p), std::max<size_t>(bytes, 256));
+    cap = std::max<size_t>(bytes, 256);
+  }
+
+ private:
+  std::map<void**, size_t> caps;  // capacity of each member buffer
+  void reserve(void** p, size_t bytes);
 };
+
+// Builds the tree of device positions (`stride` doubles apart) into d, buffers
+// included; two short synchronisations.  The caller has reserved
+// tree_build_bytes() in the context's arena beyond what it has taken.
+size_t tree_build_bytes(int64_t nsrc, int64_t ntgt);
+void build_tree_device(lpm_context& ctx, FFDevice& d, const double* src, int src_stride, int64_t nsrc,
+                       const double* tgt, int tgt_stride, int64_t ntgt, int leaf_max);
 
 // Network weights on the device: BF16 in the tensor-core tile layout
 // (W1 128x48, W2 128x128, W3 128x128, W4 16x128, each row-major in core

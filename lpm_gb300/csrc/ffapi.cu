@@ -170,7 +170,8 @@ int lpm_farfield_velocity(lpm_farfield* ff, lpm_view u, lpm_view x, int64_t nx, 
     lpm::DeviceGuard device_guard(c.device);
     c.arena.reset();
     c.arena.reserve(sizeof(int) * (2 * size_t(nf) + 2 * size_t(nf) / 1024 + 8) +
-                    sizeof(double4_16a) * size_t(nf + nx) + sizeof(double) * 3 * size_t(nx) + 8192);
+                    sizeof(double4_16a) * size_t(nf + nx) + sizeof(double) * 3 * size_t(nx) +
+                    lpm::tree_build_bytes(nf, nx) + 8192);
     int* slot2src = static_cast<int*>(c.arena.take(sizeof(int) * std::max<int64_t>(nf, 1)));
     int* src2slot = static_cast<int*>(c.arena.take(sizeof(int) * std::max<int64_t>(nf, 1)));
     const int64_t ns = lpm::compact_sources(c, mask, nf, slot2src, src2slot);
@@ -187,14 +188,7 @@ int lpm_farfield_velocity(lpm_farfield* ff, lpm_view u, lpm_view x, int64_t nx, 
                                                                      src2slot, ns, src);
     k_ff_pack_tgt<<<unsigned((nx + 255) / 256), 256, 0, c.stream>>>(lpm::to_view(x), nx, tgt);
     c.launches += 2;
-    std::vector<double4_16a> hs(ns), ht(nx);
-    LPM_CUDA(cudaMemcpyAsync(hs.data(), src, sizeof(double4_16a) * ns, cudaMemcpyDeviceToHost, c.stream));
-    LPM_CUDA(cudaMemcpyAsync(ht.data(), tgt, sizeof(double4_16a) * nx, cudaMemcpyDeviceToHost, c.stream));
-    LPM_CUDA(cudaStreamSynchronize(c.stream));
-    std::vector<double> sx(3 * ns), tx(3 * nx);
-    for (int64_t i = 0; i < ns; ++i) sx[3 * i] = hs[i].x, sx[3 * i + 1] = hs[i].y, sx[3 * i + 2] = hs[i].z;
-    for (int64_t i = 0; i < nx; ++i) tx[3 * i] = ht[i].x, tx[3 * i + 1] = ht[i].y, tx[3 * i + 2] = ht[i].z;
-    ff->build(sx.data(), ns, tx.data(), nx);
+    ff->build(reinterpret_cast<const double*>(src), 4, ns, reinterpret_cast<const double*>(tgt), 4, nx);
     ff->evaluate(tgt, src, w, nx, lpm::chord_c0(3, eps), eps);
     k_ff_velocity<<<unsigned((nx + 255) / 256), 256, 0, c.stream>>>(w, nx, lpm::to_view(x),
                                                                      lpm::to_view(u));

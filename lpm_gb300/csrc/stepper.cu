@@ -24,7 +24,7 @@
 
 #include "lpm_host.hpp"
 #include "nbody.cuh"
-#include "farfield.hpp"
+#include "farfield_dev.cuh"
 #include "stage.cuh"
 
 
@@ -168,20 +168,18 @@ struct lpm_stepper_base {
   // (first step, then every ff_every steps); outside any graph capture.
   void ff_prepare(const lpm::Tg& g) {
     if (!ff) return;
+    ff->enter();
     const bool due = !ff->built() || (ff_every > 0 && ff_steps % ff_every == 0);
     ff_steps++;
     if (!due) return;
     lpm_context& c = *ctx;
-    c.arena.reset();
-    c.arena.reserve(sizeof(double) * 3 * size_t(T + nsrc) + 4096);
-    double* d = static_cast<double*>(c.arena.take(sizeof(double) * 3 * size_t(T + nsrc)));
     const int64_t n = T + nsrc;
+    c.arena.reset();
+    c.arena.reserve(sizeof(double) * 3 * size_t(n) + lpm::tree_build_bytes(nsrc, T) + 4096);
+    double* d = static_cast<double*>(c.arena.take(sizeof(double) * 3 * size_t(n)));
     lpm::k_snapshot<<<unsigned((n + 255) / 256), 256, 0, c.stream>>>(g, src2slot, nsrc, d, d + 3 * T);
     c.launches++;
-    std::vector<double> h(3 * size_t(n));
-    LPM_CUDA(cudaMemcpyAsync(h.data(), d, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c.stream));
-    LPM_CUDA(cudaStreamSynchronize(c.stream));
-    ff->build(h.data() + 3 * T, nsrc, h.data(), T);
+    ff->build(d + 3 * T, 3, nsrc, d, 3, T);
   }
   // One N-body evaluation; with_psi = false evaluates the velocity only (a
   // plan without the stream-function component) even if the stepper wants psi.
@@ -312,10 +310,10 @@ struct lpm_bve_rk4 : lpm_stepper_base {
     P.c0 = c0();
 
     ff_prepare(g);
-    std::vector<char> kk(sizeof(lpm::Tg) + sizeof(void*));
+    std::vector<char> kk(sizeof(lpm::Tg) + sizeof(int64_t));
     std::memcpy(kk.data(), &g, sizeof(g));
-    const void* fd = ff ? static_cast<const void*>(ff->d) : nullptr;
-    std::memcpy(kk.data() + sizeof(g), &fd, sizeof(fd));
+    const int64_t tree = ff ? ff->generation : -1;  // a rebuilt tree: other sizes, buffers
+    std::memcpy(kk.data() + sizeof(g), &tree, sizeof(tree));
     const int th = lpm::sum_threads(T);
     const int64_t nb = (T + th - 1) / th;
     run(kk, [&]() {
