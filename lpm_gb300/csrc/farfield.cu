@@ -89,6 +89,9 @@ __global__ void __launch_bounds__(128) k_ff_cells(const float4* __restrict__ ys,
   const int s0 = ci.x, n = ci.y, t = threadIdx.x;
   // pass 1: centre, S, sum g
   float a[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  // (loads eight points ahead: the few largest cells are read by one CTA, which
+  // waited a memory latency per point of a thread; the sums keep their order)
+#pragma unroll 8
   for (int i = t; i < n; i += 128) {
     const float4 p = ys[s0 + i];
     a[0] += p.x;
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(128) k_ff_cells(const float4* __restrict__ ys,
   const double cn = cnorm;
   // pass 2: radius about the (FP32) centre
   float hmax = 0.f;
+#pragma unroll 8
   for (int i = t; i < n; i += 128) {
     const float4 p = ys[s0 + i];
     const float x0 = p.x - cf[0], x1 = p.y - cf[1], x2 = p.z - cf[2];
@@ -215,6 +219,7 @@ __global__ void __launch_bounds__(128) k_ff_tblocks(const double4_16a* __restric
                                                     const int* __restrict__ tslot,
                                                     float4* __restrict__ xt, float4* __restrict__ box) {
   __shared__ double sh[5 * 8];
+  __shared__ float fsh[4], ctr[3];
   const int64_t b = blockIdx.x;
   const int t = threadIdx.x;
   const int64_t i = b * kTargetBlock + t;
@@ -224,50 +229,63 @@ __global__ void __launch_bounds__(128) k_ff_tblocks(const double4_16a* __restric
     x = make_float4(float(p.x), float(p.y), float(p.z), 1.f);
   }
   xt[i] = x;
-  double a[4] = {x.x, x.y, x.z, x.w};
-  block_sum128<4>(a, sh);
-  const float c0 = float(a[0] / a[3]), c1 = float(a[1] / a[3]), c2 = float(a[2] / a[3]);
-  double r = 0;
+  // FP64 sums (64 clocks a warp and operation): only of the coordinates, and
+  // divided once per block
+  const int count = __syncthreads_count(x.w > 0.f);
+  double a[3] = {x.x, x.y, x.z};
+  block_sum128<3>(a, sh);
+  if (t < 3) ctr[t] = float((t == 0 ? a[0] : t == 1 ? a[1] : a[2]) / double(count));
+  __syncthreads();
+  const float c0 = ctr[0], c1 = ctr[1], c2 = ctr[2];
+  float r = 0.f;
   if (x.w > 0) {
     const float e0 = x.x - c0, e1 = x.y - c1, e2 = x.z - c2;
     r = sqrtf(e0 * e0 + e1 * e1 + e2 * e2);
   }
-  r = block_max128(r, sh);
-  if (t == 0) box[b] = make_float4(c0, c1, c2, float(r) * (1.f + 1e-6f) + 1e-7f);
+  r = block_max128(r, fsh);
+  if (t == 0) box[b] = make_float4(c0, c1, c2, r * (1.f + 1e-6f) + 1e-7f);
 }
 
-// One thread per target block: depth-first walk from the root.
-__global__ void k_ff_lists(const float* __restrict__ cd, const int4* __restrict__ cells,
-                           const float4* __restrict__ box, int64_t nblocks, float theta,
-                           float rho_min, int learn, int* __restrict__ far, int* __restrict__ near,
-                           int* __restrict__ lrn, int4* __restrict__ cnt) {
-  const int64_t b = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (b >= nblocks) return;
-  const float4 bx = box[b];
+// The walk's verdict on a cell for one target block.
+struct Verdict {
+  bool far, learn, near;  // none: descend
+};
+__device__ __forceinline__ Verdict judge(const float* __restrict__ r, const int4 ci, const float4 bx,
+                                         float theta, float rho_min, int learn) {
+  const float e0 = bx.x - r[0], e1 = bx.y - r[1], e2 = bx.z - r[2];
+  const float D = sqrtf(e0 * e0 + e1 * e1 + e2 * e2) - bx.w;
+  const float h = r[4];
+  const bool accept = D > 0.f && h <= theta * D;
+  Verdict v;
+  v.far = accept && ci.y >= kExactMax;
+  v.learn = v.far && learn && h >= rho_min * D;
+  // a leaf that is near, or far but small enough to sum exactly
+  v.near = !v.far && ci.w == 0;
+  return v;
+}
+
+// Depth-first walk from the root by one thread (a block whose list outgrows the
+// warp's buffers).
+__device__ __noinline__ int4 walk_serial(const float* __restrict__ cd, const int4* __restrict__ cells,
+                                         float4 bx, float theta, float rho_min, int learn,
+                                         int* __restrict__ F, int* __restrict__ N,
+                                         int* __restrict__ L) {
   int stk[8 * 22];
   int sp = 0;
   stk[sp++] = 0;
   int nf = 0, nn = 0, nl = 0, over = 0;
-  int* F = far + b * kFarCap;
-  int* N = near + b * kNearCap;
-  int* L = lrn + b * kLearnCap;
   while (sp > 0) {
     const int c = stk[--sp];
-    const float* r = cd + int64_t(c) * kCellF;
-    const float e0 = bx.x - r[0], e1 = bx.y - r[1], e2 = bx.z - r[2];
-    const float D = sqrtf(e0 * e0 + e1 * e1 + e2 * e2) - bx.w;
-    const float h = r[4];
     const int4 ci = cells[c];
-    const bool accept = D > 0.f && h <= theta * D;
-    if (accept && ci.y >= kExactMax) {
+    const Verdict v = judge(cd + int64_t(c) * kCellF, ci, bx, theta, rho_min, learn);
+    if (v.far) {
       if (nf < kFarCap) F[nf] = c;
       nf++;
-      if (learn && h >= rho_min * D) {
+      if (v.learn) {
         if (nl < kLearnCap) L[nl] = c;
         nl++;
       }
-    } else if (ci.w == 0) {
-      // a leaf that is near, or far but small enough to sum exactly
+    } else if (v.near) {
       if (nn < kNearCap) N[nn] = c;
       nn++;
     } else {
@@ -278,8 +296,106 @@ __global__ void k_ff_lists(const float* __restrict__ cd, const int4* __restrict_
       for (int k = ci.w - 1; k >= 0; --k) stk[sp++] = ci.z + k;
     }
   }
-  if (nf > kFarCap || nn > kNearCap || nl > kLearnCap) over = 1;
-  cnt[b] = make_int4(min(nf, kFarCap), min(nn, kNearCap), min(nl, kLearnCap), over);
+  return make_int4(nf, nn, nl, over);
+}
+
+// One warp per target block.  The walk keeps an ordered list of cells and, level
+// by level, judges 32 of them at a time: a far cell or a near leaf stays in place
+// with a tag, any other is replaced by its children, so the list ends in the
+// depth-first order of the serial walk.  A thread walking alone waited two memory
+// latencies per cell: 253 us at icosahedral level 6, theta 0.4 (1,600 blocks),
+// where the warp takes 22.
+constexpr int kListCap = 2048;  // entries of the ordered list; beyond, walk_serial
+constexpr int kListWarps = 2;
+constexpr int kTagFar = 1 << 30, kTagNear = 1 << 29, kTagLearn = 1 << 28;  // cells < 2^28
+
+__global__ void __launch_bounds__(32 * kListWarps) k_ff_lists(
+    const float* __restrict__ cd, const int4* __restrict__ cells, const float4* __restrict__ box,
+    int64_t nblocks, float theta, float rho_min, int learn, int* __restrict__ far,
+    int* __restrict__ near, int* __restrict__ lrn, int4* __restrict__ cnt) {
+  __shared__ int list[kListWarps][2][kListCap];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const int64_t b = blockIdx.x * int64_t(kListWarps) + w;
+  if (b >= nblocks) return;
+  const float4 bx = box[b];
+  int* F = far + b * kFarCap;
+  int* N = near + b * kNearCap;
+  int* L = lrn + b * kLearnCap;
+  int* in = list[w][0];
+  int* out = list[w][1];
+  if (lane == 0) in[0] = 0;
+  __syncwarp();
+  int len = 1;
+  bool fits = true, open = true;
+  while (open && fits) {
+    open = false;
+    int n = 0;
+    for (int base = 0; base < len; base += 32) {
+      int e = base + lane < len ? in[base + lane] : 0;
+      int put = base + lane < len ? 1 : 0, child = -1;
+      if (put && e < kTagLearn) {
+        const int4 ci = cells[e];
+        const Verdict v = judge(cd + int64_t(e) * kCellF, ci, bx, theta, rho_min, learn);
+        if (v.far) {
+          e |= kTagFar | (v.learn ? kTagLearn : 0);
+        } else if (v.near) {
+          e |= kTagNear;
+        } else {
+          child = ci.z;
+          put = ci.w;
+        }
+      }
+      open |= child >= 0;
+      int x = put;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      const int total = __shfl_sync(0xffffffffu, x, 31);
+      if (n + total > kListCap) {
+        fits = false;
+        break;
+      }
+      const int at = n + x - put;
+      if (child < 0) {
+        if (put) out[at] = e;
+      } else {
+        for (int k = 0; k < put; ++k) out[at + k] = child + k;
+      }
+      n += total;
+    }
+    open = __any_sync(0xffffffffu, open);
+    __syncwarp();
+    int* s = in;
+    in = out;
+    out = s;
+    len = n;
+  }
+  int4 c = make_int4(0, 0, 0, 0);
+  if (fits) {
+    for (int base = 0; base < len; base += 32) {
+      const int e = base + lane < len ? in[base + lane] : 0;
+      const int id = e & (kTagLearn - 1);
+      const unsigned mf = __ballot_sync(0xffffffffu, (e & kTagFar) != 0);
+      const unsigned mn = __ballot_sync(0xffffffffu, (e & kTagNear) != 0);
+      const unsigned ml = __ballot_sync(0xffffffffu, (e & kTagLearn) != 0);
+      int p = c.x + __popc(mf & below);
+      if ((e & kTagFar) && p < kFarCap) F[p] = id;
+      p = c.y + __popc(mn & below);
+      if ((e & kTagNear) && p < kNearCap) N[p] = id;
+      p = c.z + __popc(ml & below);
+      if ((e & kTagLearn) && p < kLearnCap) L[p] = id;
+      c.x += __popc(mf), c.y += __popc(mn), c.z += __popc(ml);
+    }
+  } else if (lane == 0) {
+    c = walk_serial(cd, cells, bx, theta, rho_min, learn, F, N, L);
+  }
+  if (lane == 0) {
+    const int over = c.w || c.x > kFarCap || c.y > kNearCap || c.z > kLearnCap;
+    cnt[b] = make_int4(min(c.x, kFarCap), min(c.y, kNearCap), min(c.z, kLearnCap), over);
+  }
 }
 
 constexpr int kNearBuf = 512;
@@ -295,7 +411,10 @@ __device__ __forceinline__ void chord_acc(float x0, float x1, float x2, float4 s
   w2 = fmaf(r, d2, w2);
 }
 
-// One CTA (128 threads, one target each) per target block.
+// One CTA (128 threads, one target each) per target block and part: part 0 sums
+// the near leaves, and the far batches go to the parts in turn; the parts' FP64
+// partials are added by the epilogue.  One part while the blocks fill the GPU for
+// many waves, more where the last wave would leave it idle (ff_parts).
 __global__ void __launch_bounds__(128) k_ff_eval(
     const float4* __restrict__ xt, const int* __restrict__ tslot,
     const float4* __restrict__ ys, int64_t nsrc, const float* __restrict__ cd,
@@ -305,13 +424,13 @@ __global__ void __launch_bounds__(128) k_ff_eval(
   __shared__ float cell[kFarBatch][kCellF];
   __shared__ int4 lf[8];
   const int64_t b = blockIdx.x;
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, part = blockIdx.y, parts = gridDim.y;
   const float4 x = xt[b * kTargetBlock + t];
   const int4 nc = cnt[b];
   float S0 = 0.f, S1 = 0.f, S2 = 0.f, C0 = 0.f, C1 = 0.f, C2 = 0.f;
   if (nc.w) {
-    // lists overflowed: full direct sum (fallback)
-    for (int64_t j0 = 0; j0 < nsrc; j0 += kNearBuf) {
+    // lists overflowed: full direct sum (fallback), by part 0
+    for (int64_t j0 = 0; j0 < (part == 0 ? nsrc : 0); j0 += kNearBuf) {
       const int m = int(nsrc - j0 < kNearBuf ? nsrc - j0 : kNearBuf);
       __syncthreads();
       for (int i = t; i < m; i += 128) buf[i] = ys[j0 + i];
@@ -326,7 +445,7 @@ __global__ void __launch_bounds__(128) k_ff_eval(
     // near leaves, up to 8 per batch (<= 512 sources); the 8 leaf records are
     // loaded by 8 threads at once
     const int* N = near + b * kNearCap;
-    for (int l0 = 0; l0 < nc.y; l0 += 8) {
+    for (int l0 = 0; l0 < (part == 0 ? nc.y : 0); l0 += 8) {
       const int nl = min(8, nc.y - l0);
       __syncthreads();
       if (t < nl) lf[t] = cells[N[l0 + t]];
@@ -388,7 +507,7 @@ __global__ void __launch_bounds__(128) k_ff_eval(
     }
     // far cells: order-4 expansion, kFarBatch cells per batch
     const int* F = far + b * kFarCap;
-    for (int f0 = 0; f0 < nc.x; f0 += kFarBatch) {
+    for (int f0 = part * kFarBatch; f0 < nc.x; f0 += parts * kFarBatch) {
       const int nb = min(kFarBatch, nc.x - f0);
       __syncthreads();
       for (int i = t; i < nb * kCellF; i += 128) {
@@ -413,9 +532,10 @@ __global__ void __launch_bounds__(128) k_ff_eval(
   }
   const int64_t tt = tslot[b * kTargetBlock + t];
   if (tt >= 0) {
-    wout[tt] = double(S0) + double(C0);
-    wout[wstride + tt] = double(S1) + double(C1);
-    wout[2 * wstride + tt] = double(S2) + double(C2);
+    double* w = wout + 3 * part * wstride;
+    w[tt] = double(S0) + double(C0);
+    w[wstride + tt] = double(S1) + double(C1);
+    w[2 * wstride + tt] = double(S2) + double(C2);
   }
 }
 
@@ -437,6 +557,15 @@ void ff_cells(lpm_context& ctx, const float4* ys, const int4* cells, int ncells,
   LPM_CUDA(cudaGetLastError());
 }
 
+// Parts of an evaluation: at least kPartWaves waves of CTAs (seven resident per
+// SM).  Icosahedral level 6, theta 0.4 (1,600 blocks: 1.5 waves in one part):
+// 470 us in one part, 407 in four; level 8 (25,557 blocks) runs one part.
+int ff_parts(const lpm_context& ctx, int64_t nblocks) {
+  constexpr int64_t kPartWaves = 6;
+  const int64_t slots = int64_t(std::max(ctx.num_sms, 1)) * 7;
+  return int(std::max<int64_t>(1, std::min<int64_t>(kFFMaxParts, kPartWaves * slots / std::max<int64_t>(nblocks, 1))));
+}
+
 void ff_launch_tree(lpm_context& ctx, FFDevice& d, const void* tgt, const void* src, double* wout,
                     int64_t wstride, double c0, double theta, double rho_min, bool learn) {
   cudaStream_t st = ctx.stream;
@@ -445,10 +574,10 @@ void ff_launch_tree(lpm_context& ctx, FFDevice& d, const void* tgt, const void* 
   k_ff_cells<<<d.ncells, 128, 0, st>>>(d.ys, d.cells, d.ncells, float(theta), d.rmax, d.cd);
   k_ff_tblocks<<<unsigned(d.nblocks), 128, 0, st>>>(static_cast<const double4_16a*>(tgt), d.tslot,
                                                     d.xt, d.box);
-  k_ff_lists<<<unsigned((d.nblocks + 63) / 64), 64, 0, st>>>(d.cd, d.cells, d.box, d.nblocks,
-                                                            float(theta), float(rho_min), learn,
-                                                            d.far, d.near, d.lrn, d.cnt);
-  k_ff_eval<<<unsigned(d.nblocks), 128, 0, st>>>(d.xt, d.tslot, d.ys, d.nsrc, d.cd,
+  k_ff_lists<<<unsigned((d.nblocks + kListWarps - 1) / kListWarps), 32 * kListWarps, 0, st>>>(
+      d.cd, d.cells, d.box, d.nblocks, float(theta), float(rho_min), learn, d.far, d.near, d.lrn,
+      d.cnt);
+  k_ff_eval<<<dim3(unsigned(d.nblocks), unsigned(ff_parts(ctx, d.nblocks))), 128, 0, st>>>(d.xt, d.tslot, d.ys, d.nsrc, d.cd,
                                                  d.cells, d.far, d.near, d.cnt, float(c0), wout,
                                                  wstride);
   ctx.launches += 5;
@@ -464,6 +593,8 @@ lpm_farfield::~lpm_farfield() {
   for (void* e : events) cudaEventDestroy(static_cast<cudaEvent_t>(e));
   delete d;
 }
+
+int lpm_farfield::parts() const { return lpm::ff_parts(*ctx, d->nblocks); }
 
 bool lpm_farfield::built() const { return d != nullptr && d->ncells > 0; }
 

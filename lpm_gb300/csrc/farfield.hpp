@@ -20,6 +20,7 @@ constexpr int kTargetBlock = 128;   // targets per block = rows of one MMA tile
 constexpr int kFarCap = 2048;       // far cells per target block
 constexpr int kNearCap = 4096;      // near leaves per target block
 constexpr int kLearnCap = 1024;     // learned (cell, block) pairs per block
+constexpr int kFFMaxParts = 4;      // partial sums per target of an evaluation
 constexpr int kExactMax = 32;       // accepted cells with fewer points are summed exactly
 
 // Cell record: kCellF floats per cell.
@@ -102,7 +103,9 @@ struct lpm_farfield {
   void enter();
   int64_t generation = 0;  // builds so far
   bool built() const;
-  // w[c * wstride + t] = sum over sources of g (x_t - y) / (|x_t - y|^2 + c0)
+  // Partial sums an evaluation of the built tree writes (at most kFFMaxParts).
+  int parts() const;
+  // The sum over parts p of w[(3 p + c) * wstride + t] = sum over sources of g (x_t - y) / (|x_t - y|^2 + c0)
   // up to terms parallel to x_t (the chord-form sum whose cross product with
   // x_t gives the velocity), for packed double4_16a targets (x, y, z, _) and
   // sources (x, y, z, g) in the order given to build().

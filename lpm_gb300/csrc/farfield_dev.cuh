@@ -64,6 +64,7 @@ struct FFNet {
   void* alloc(size_t bytes);
 };
 
+int ff_parts(const lpm_context& ctx, int64_t nblocks);
 void ff_launch_tree(lpm_context& ctx, FFDevice& d, const void* tgt, const void* src, double* wout,
                     int64_t wstride, double c0, double theta, double rho_min, bool learn);
 // Shared-memory limits of the network kernels (call outside stream capture,

@@ -33,10 +33,16 @@ __global__ void k_ff_pack_tgt(lpm::View x, int64_t n, double4_16a* __restrict__ 
 }
 
 // u = -(1/2pi) w cross x
-__global__ void k_ff_velocity(const double* __restrict__ w, int64_t n, lpm::View x, lpm::View u) {
+__global__ void k_ff_velocity(const double* __restrict__ w, int parts, int64_t n, lpm::View x,
+                              lpm::View u) {
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= n) return;
-  const double w0 = w[i], w1 = w[n + i], w2 = w[2 * n + i];
+  double w0 = w[i], w1 = w[n + i], w2 = w[2 * n + i];
+  for (int p = 1; p < parts; ++p, w += 3 * n) {
+    w0 += w[3 * n + i];
+    w1 += w[4 * n + i];
+    w2 += w[5 * n + i];
+  }
   const double x0 = x(i, 0), x1 = x(i, 1), x2 = x(i, 2);
   const double k = -1.0 / lpm::kTWOPI;
   u(i, 0) = k * (w1 * x2 - w2 * x1);
@@ -170,7 +176,7 @@ int lpm_farfield_velocity(lpm_farfield* ff, lpm_view u, lpm_view x, int64_t nx, 
     lpm::DeviceGuard device_guard(c.device);
     c.arena.reset();
     c.arena.reserve(sizeof(int) * (2 * size_t(nf) + 2 * size_t(nf) / 1024 + 8) +
-                    sizeof(double4_16a) * size_t(nf + nx) + sizeof(double) * 3 * size_t(nx) +
+                    sizeof(double4_16a) * size_t(nf + nx) + sizeof(double) * 3 * lpm::kFFMaxParts * size_t(nx) +
                     lpm::tree_build_bytes(nf, nx) + 8192);
     int* slot2src = static_cast<int*>(c.arena.take(sizeof(int) * std::max<int64_t>(nf, 1)));
     int* src2slot = static_cast<int*>(c.arena.take(sizeof(int) * std::max<int64_t>(nf, 1)));
@@ -183,14 +189,14 @@ int lpm_farfield_velocity(lpm_farfield* ff, lpm_view u, lpm_view x, int64_t nx, 
     }
     double4_16a* src = static_cast<double4_16a*>(c.arena.take(sizeof(double4_16a) * ns));
     double4_16a* tgt = static_cast<double4_16a*>(c.arena.take(sizeof(double4_16a) * nx));
-    double* w = static_cast<double*>(c.arena.take(sizeof(double) * 3 * nx));
+    double* w = static_cast<double*>(c.arena.take(sizeof(double) * 3 * lpm::kFFMaxParts * nx));
     k_ff_pack_src<<<unsigned((ns + 255) / 256), 256, 0, c.stream>>>(lpm::to_view(fx), zeta, area,
                                                                      src2slot, ns, src);
     k_ff_pack_tgt<<<unsigned((nx + 255) / 256), 256, 0, c.stream>>>(lpm::to_view(x), nx, tgt);
     c.launches += 2;
     ff->build(reinterpret_cast<const double*>(src), 4, ns, reinterpret_cast<const double*>(tgt), 4, nx);
     ff->evaluate(tgt, src, w, nx, lpm::chord_c0(3, eps), eps);
-    k_ff_velocity<<<unsigned((nx + 255) / 256), 256, 0, c.stream>>>(w, nx, lpm::to_view(x),
+    k_ff_velocity<<<unsigned((nx + 255) / 256), 256, 0, c.stream>>>(w, ff->parts(), nx, lpm::to_view(x),
                                                                      lpm::to_view(u));
     c.launches++;
     LPM_CUDA(cudaGetLastError());

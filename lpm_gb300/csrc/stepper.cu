@@ -102,7 +102,11 @@ struct lpm_stepper_base {
     tgt = dalloc(rec * plan.ntgt_pad);
     src = dalloc(32 * plan.nsrc_pad);  // SrcF32 / double4_16a
     tself = static_cast<int*>(dalloc(sizeof(int) * plan.ntgt_pad));
-    part = static_cast<double*>(dalloc(plan.part_bytes()));
+    // (a far field writes at most kFFMaxParts partials of the velocity)
+    const size_t ff_bytes = precision == LPM_FP64_CHORD
+                                ? sizeof(double) * 3 * lpm::kFFMaxParts * size_t(plan.ntgt_pad)
+                                : 0;
+    part = static_cast<double*>(dalloc(std::max(plan.part_bytes(), ff_bytes)));
     if (plan.split) plan.split_buf = dalloc(lpm::split_bytes(c, plan.ntgt_pad, plan.nsrc_pad));
     sgbuf = static_cast<double*>(dalloc(sizeof(double) * (8 + 256)));
     // zero the padding records once (never rewritten); tself padding = -1
@@ -160,7 +164,7 @@ struct lpm_stepper_base {
     k.tself = tself;
     k.src = src;
     k.part = part;
-    k.nchunks = ff ? 1 : plan.nchunks;
+    k.nchunks = ff ? ff->parts() : plan.nchunks;
     k.tpad = plan.ntgt_pad;
     return k;
   }
@@ -295,6 +299,7 @@ struct lpm_bve_rk4 : lpm_stepper_base {
       buf = static_cast<double*>(dalloc(sizeof(double) * size_t(T) * (4 * 3 + 4 + 3)));
     }
     lpm::Tg g = targets(vx, vzeta, vvel, nullptr, fx, fzeta, fvel, nullptr, farea);
+    ff_prepare(g);
     lpm::Pk k = packs();
     lpm::Rk4Buf b;
     for (int s = 0; s < 4; ++s) {
@@ -309,7 +314,6 @@ struct lpm_bve_rk4 : lpm_stepper_base {
     P.reproject = flags & LPM_STEP_REPROJECT;
     P.c0 = c0();
 
-    ff_prepare(g);
     std::vector<char> kk(sizeof(lpm::Tg) + sizeof(int64_t));
     std::memcpy(kk.data(), &g, sizeof(g));
     const int64_t tree = ff ? ff->generation : -1;  // a rebuilt tree: other sizes, buffers

@@ -71,3 +71,17 @@ def test_reuse_grows_and_shrinks(gpu_ctx, oracle):
         a = _check(gpu_ctx, oracle, ff, x, y, z, 64)
         b = _check(gpu_ctx, oracle, FarField(theta=0.3, ctx=gpu_ctx), x, y, z, 64)
         assert a == b and a < 1e-3
+
+
+@pytest.mark.parametrize("theta", [0.05, 0.12])
+def test_long_lists(gpu_ctx, oracle, theta):
+    """Interaction lists longer than a warp's ordered list (2,048 cells): those
+    blocks walk serially; leaves of one point make the lists long.  Every pair is
+    then a near one or an accepted cell of fewer than 32 points: the FP32 direct
+    sum, within 1e-5."""
+    from lpm_gb300.farfield import FarField
+
+    rng = np.random.default_rng(6)
+    ff = FarField(theta=theta, leaf_max=1, rho_min=0.0, ctx=gpu_ctx)
+    err = _check(gpu_ctx, oracle, ff, _points(rng, 300), _points(rng, 3500), rng.normal(size=3500), 1)
+    assert err < (1e-5 if theta < 0.1 else 1e-3)
