@@ -148,6 +148,68 @@ __global__ void k_pack_tgt(int64_t off, int64_t n, View x, int ndim,
   }
 }
 
+// Compaction and packing of a small call in one launch, without the host learning
+// the source count: each CTA counts the unmasked slots before its own 256 itself
+// (masks of at most kPrepSlots bytes), packs its sources and its targets; the CTA
+// of the last slot writes the count and the padding records (strength 0, away from
+// any target).  Separate counting, scanning, mapping, packing and padding launches
+// with a host read of the count in between took 36 of the 52 us of a call of 162
+// vertices and 320 sources.
+constexpr int64_t kPrepSlots = 32768;
+
+template <int MODE>
+__global__ void __launch_bounds__(256)
+    k_prep_small(const uint8_t* __restrict__ mask, int64_t nslots, int64_t npad, View sx, int ndim,
+                 const double* __restrict__ zeta, const double* __restrict__ area, int form,
+                 View tx, int64_t nt, int64_t ntpad, bool collocated, bool skip,
+                 void* __restrict__ src, void* __restrict__ tgt, int* __restrict__ tself,
+                 int* __restrict__ nreal) {
+  __shared__ int wsum[8], wcnt[8];
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  const int64_t b0 = int64_t(blockIdx.x) * 256, i = b0 + t;
+  int before = 0;
+  for (int64_t j = t; j < min(b0, nslots); j += 256) before += mask[j] == 0;
+  before = __reduce_add_sync(0xffffffffu, before);
+  const bool keep = i < nslots && !mask[i];
+  const unsigned m = __ballot_sync(0xffffffffu, keep);
+  if (lane == 0) wsum[w] = before, wcnt[w] = __popc(m);
+  __syncthreads();
+  int k = __popc(m & ((1u << lane) - 1u)), total = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    total += wsum[q] + wcnt[q];
+    k += wsum[q] + (q < w ? wcnt[q] : 0);
+  }
+  auto put_src = [&](int64_t at, double p0, double p1, double p2, double g) {
+    if (MODE == M_C32)
+      reinterpret_cast<SrcF32*>(src)[at] = make_src_f32(float(p0), float(p1), float(p2), float(g));
+    else
+      reinterpret_cast<double4_16a*>(src)[at] = make_double4_16a(p0, p1, p2, g);
+  };
+  if (keep)
+    put_src(k, sx(i, 0), sx(i, 1), ndim == 3 ? sx(i, 2) : 0.0,
+            (form == FORM_BVE && MODE == M_REF64) ? (-zeta[i]) * area[i] : zeta[i] * area[i]);
+  if (b0 <= max(nslots - 1, int64_t(0)) && max(nslots - 1, int64_t(0)) < b0 + 256) {
+    if (t == 0) *nreal = total;
+    const double far = ndim == 3 ? 0.0 : (MODE == M_C32 ? 1e18 : 1e100);
+    for (int64_t q = total + t; q < npad; q += 256) put_src(q, far, far, 0.0, 0.0);
+  }
+  if (i < ntpad) {
+    const bool real = i < nt;
+    const double p0 = real ? tx(i, 0) : 0.0, p1 = real ? tx(i, 1) : 0.0;
+    const double p2 = real && ndim == 3 ? tx(i, 2) : 0.0;
+    const int self = real && collocated && skip && keep ? k : -1;
+    const double gs = self >= 0 ? zeta[i] * area[i] : 0.0;
+    if (MODE == M_C32) {
+      reinterpret_cast<float4*>(tgt)[i] = make_float4(float(p0), float(p1), float(p2), float(gs));
+    } else {
+      reinterpret_cast<double4_16a*>(tgt)[i] =
+          make_double4_16a(p0, p1, p2, MODE == M_C64 ? gs : 0.0);
+      if (MODE == M_REF64) tself[i] = self;
+    }
+  }
+}
+
 __global__ void k_fill_pad_tgt(int64_t from, int64_t to, bool f32, void* out,
                                int* tself) {
   const int64_t i = from + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -176,12 +238,13 @@ __global__ void k_sum_g_partial(const void* src, bool f32, int64_t n, double* pa
   }
   if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
+// One warp, fixed order (a single thread's chain of 256 FP64 adds took 10 us).
 __global__ void k_sum_final(const double* part, int n, double* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0;
-    for (int i = 0; i < n; ++i) s += part[i];
-    *out = s;
-  }
+  double s = 0;
+  for (int i = threadIdx.x; i < n; i += 32) s += part[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) *out = s;
 }
 
 // Combine the chunk partials of one segment and write its outputs.
@@ -254,7 +317,7 @@ void launch_chord_shape(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
   dim3 grid(unsigned(p.ntgt_pad / (NT * R)), unsigned(p.nchunks));
   nbody_chord<T, NDIM, WU, WP, SKIPC, R, NT, TILE, MINB><<<grid, NT, 0, ctx.stream>>>(
       static_cast<const V4*>(tgt), static_cast<const Rec*>(src), p.ntgt_pad, p.nsrc_pad,
-      p.chunk_len, c0, part, ctx.d_err);
+      p.nreal, p.chunk_len, c0, part, ctx.d_err);
   ctx.launches++;
 }
 
@@ -310,7 +373,7 @@ void launch_f64(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
     dim3 g(unsigned(p.ntgt_pad / FINE_NT), unsigned(p.nchunks));
     nbody_f64h<FORM, WU, WP, 1, FINE_NT, FINE_TILE><<<g, FINE_NT, 0, ctx.stream>>>(
         static_cast<const double4_16a*>(tgt), tself, static_cast<const double4_16a*>(src),
-        p.ntgt_pad, p.nsrc_pad, p.chunk_len, eps2, part, ctx.d_err);
+        p.ntgt_pad, p.nsrc_pad, p.nreal, p.chunk_len, eps2, part, ctx.d_err);
     ctx.launches++;
     return;
   }
@@ -318,11 +381,11 @@ void launch_f64(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
   if (ref64_exact(p.precision))
     nbody_f64<FORM, WU, WP, F64_R, F64_NT, F64_TILE><<<grid, F64_NT, 0, ctx.stream>>>(
         static_cast<const double4_16a*>(tgt), tself, static_cast<const double4_16a*>(src),
-        p.ntgt_pad, p.nsrc_pad, p.chunk_len, eps2, part, ctx.d_err);
+        p.ntgt_pad, p.nsrc_pad, p.nreal, p.chunk_len, eps2, part, ctx.d_err);
   else
     nbody_f64h<FORM, WU, WP, F64_R, F64_NT, F64_TILE><<<grid, F64_NT, 0, ctx.stream>>>(
         static_cast<const double4_16a*>(tgt), tself, static_cast<const double4_16a*>(src),
-        p.ntgt_pad, p.nsrc_pad, p.chunk_len, eps2, part, ctx.d_err);
+        p.ntgt_pad, p.nsrc_pad, p.nreal, p.chunk_len, eps2, part, ctx.d_err);
   ctx.launches++;
 }
 
@@ -572,6 +635,35 @@ void sum_strengths(lpm_context& ctx, const void* src, bool f32, int64_t nsrc,
 }
 
 namespace {
+// Launches after packing: strength sum, pair kernel, combine.
+template <int MODE>
+void sum_and_combine(lpm_context& ctx, const SumSpec& spec, const TgtSeg* segs, int nseg,
+                     const NbodyPlan& p, void* srcp, void* tgtp, int* tself, double* part,
+                     double* sgp) {
+  const int ndim = spec.ndim;
+  if (MODE != M_REF64 && spec.want_psi && ndim == 3)
+    sum_strengths(ctx, srcp, MODE == M_C32, p.nsrc, sgp, sgp + 8);
+  LPM_CUDA(cudaGetLastError());
+
+  NbodyPlan pt = p;
+  pt.shape = tune_shape(ctx, p, tgtp, tself, srcp, part, spec.eps);
+  launch_nbody(ctx, pt, tgtp, tself, srcp, part, spec.eps);
+
+  const double c0 = MODE == M_C32 ? double(f32_c0(ndim, spec.eps)) : chord_c0(ndim, spec.eps);
+  int64_t off = 0;
+  for (int s = 0; s < nseg; ++s) {
+    const TgtSeg& g = segs[s];
+    if (g.n > 0) {
+      if (ndim == 3)
+        combine_dispatch<MODE, 3>(ctx, p, part, off, g, tgtp, sgp, c0);
+      else
+        combine_dispatch<MODE, 2>(ctx, p, part, off, g, tgtp, sgp, c0);
+    }
+    off += g.n;
+  }
+  LPM_CUDA(cudaGetLastError());
+}
+
 template <int MODE>
 void pack_and_launch(lpm_context& ctx, const SumSpec& spec, const SrcSpec& src,
                      const TgtSeg* segs, int nseg, int64_t ntgt, const NbodyPlan& p,
@@ -599,27 +691,27 @@ void pack_and_launch(lpm_context& ctx, const SumSpec& spec, const SrcSpec& src,
         ntgt, p.ntgt_pad, MODE == M_C32, tgtp, tself);
     ctx.launches++;
   }
-  if (MODE != M_REF64 && spec.want_psi && ndim == 3)
-    sum_strengths(ctx, srcp, MODE == M_C32, p.nsrc, sgp, sgp + 8);
-  LPM_CUDA(cudaGetLastError());
+  sum_and_combine<MODE>(ctx, spec, segs, nseg, p, srcp, tgtp, tself, part, sgp);
+}
 
-  NbodyPlan pt = p;
-  pt.shape = tune_shape(ctx, p, tgtp, tself, srcp, part, spec.eps);
-  launch_nbody(ctx, pt, tgtp, tself, srcp, part, spec.eps);
+template <int MODE>
+void prep_and_launch(lpm_context& ctx, const SumSpec& spec, const SrcSpec& src, const TgtSeg& g,
+                     const NbodyPlan& p, void* srcp, void* tgtp, int* tself, int* nreal,
+                     double* part, double* sgp) {
+  const int64_t n = std::max(src.nslots, p.ntgt_pad);
+  k_prep_small<MODE><<<unsigned((n + 255) / 256), 256, 0, ctx.stream>>>(
+      src.mask, src.nslots, p.nsrc_pad, src.x, spec.ndim, src.zeta, src.area, spec.form, g.x, g.n,
+      p.ntgt_pad, g.collocated, spec.skip_self, srcp, tgtp, tself, nreal);
+  ctx.launches++;
+  sum_and_combine<MODE>(ctx, spec, &g, 1, p, srcp, tgtp, tself, part, sgp);
+}
 
-  const double c0 = MODE == M_C32 ? double(f32_c0(ndim, spec.eps)) : chord_c0(ndim, spec.eps);
-  off = 0;
-  for (int s = 0; s < nseg; ++s) {
-    const TgtSeg& g = segs[s];
-    if (g.n > 0) {
-      if (ndim == 3)
-        combine_dispatch<MODE, 3>(ctx, p, part, off, g, tgtp, sgp, c0);
-      else
-        combine_dispatch<MODE, 2>(ctx, p, part, off, g, tgtp, sgp, c0);
-    }
-    off += g.n;
-  }
-  LPM_CUDA(cudaGetLastError());
+// Calls that run without the host learning the source count: few enough slots for
+// k_prep_small, too few pairs for tuning the kernel shape, and no choice that
+// depends on the count (the split sums' least source count).
+bool prep_small(const SumSpec& spec, int64_t ntgt, int64_t nslots, int nseg) {
+  return nseg == 1 && nslots <= kPrepSlots && double(ntgt + 1024) * double(nslots + 512) < 2e9 &&
+         !split_wanted(spec.precision, spec.ndim, ntgt, nslots);
 }
 }  // namespace
 
@@ -632,12 +724,33 @@ void direct_sum(lpm_context& ctx, const SumSpec& spec, const SrcSpec& src,
   const int ndim = spec.ndim;
 
   ctx.arena.reset();
+  const size_t rec = m == M_C32 ? sizeof(float4) : sizeof(double4_16a);  // target record
+  const size_t srec = 32;  // source record: SrcF32 or double4_16a
+  if (prep_small(spec, ntgt, src.nslots, nseg)) {
+    NbodyPlan p = plan_nbody(ctx, spec.precision, ndim, spec.form, spec.want_u, spec.want_psi, ntgt,
+                             src.nslots);
+    p.skipc = segs[0].collocated && spec.skip_self;
+    ctx.arena.reserve(4096 + srec * size_t(p.nsrc_pad) + (rec + sizeof(int)) * size_t(p.ntgt_pad) +
+                      p.part_bytes() + sizeof(double) * 300 + 8 * 256);
+    void* srcp = ctx.arena.take(srec * size_t(p.nsrc_pad));
+    void* tgtp = ctx.arena.take(rec * size_t(p.ntgt_pad));
+    int* tself = static_cast<int*>(ctx.arena.take(sizeof(int) * size_t(p.ntgt_pad)));
+    double* part = static_cast<double*>(ctx.arena.take(p.part_bytes()));
+    double* sgp = static_cast<double*>(ctx.arena.take(sizeof(double) * 264));
+    int* nreal = static_cast<int*>(ctx.arena.take(sizeof(int)));
+    p.nreal = nreal;
+    if (m == M_C32)
+      prep_and_launch<M_C32>(ctx, spec, src, segs[0], p, srcp, tgtp, tself, nreal, part, sgp);
+    else if (m == M_C64)
+      prep_and_launch<M_C64>(ctx, spec, src, segs[0], p, srcp, tgtp, tself, nreal, part, sgp);
+    else
+      prep_and_launch<M_REF64>(ctx, spec, src, segs[0], p, srcp, tgtp, tself, nreal, part, sgp);
+    return;
+  }
   // Upper bounds first, so one reservation covers the whole call.
   PlanBounds pb;
   plan_bounds(ctx, spec.precision, ndim, spec.form, spec.want_u, spec.want_psi, ntgt, src.nslots,
               &pb);
-  const size_t rec = m == M_C32 ? sizeof(float4) : sizeof(double4_16a);  // target record
-  const size_t srec = 32;  // source record: SrcF32 or double4_16a
   const size_t need = 4096 + sizeof(int) * (2 * size_t(src.nslots) + 2 * (size_t(src.nslots) / SCAN_BLOCK + 2)) +
                       srec * size_t(pb.nsrc_pad) + rec * size_t(pb.ntgt_pad) +
                       sizeof(int) * size_t(pb.ntgt_pad) + pb.part_bytes + pb.split_bytes +

@@ -178,6 +178,7 @@ struct NbodyPlan {
   int nchunks_max;     // bound on nchunks for any nsrc <= this plan's nsrc
   int shape = 0;       // FP32 kernel shape (index into kF32Shapes)
   bool skipc = false;  // the targets' own sources are left out (collocated)
+  const int* nreal = nullptr;  // device: the source count, where nsrc is a bound
   bool fine = false;   // LPM_FP64: small grid, one target per thread
   bool split = false;  // FP64 sums on the FP32 pipe (nbody_split.cuh)
   void* split_buf = nullptr;  // split_bytes() of scratch for them

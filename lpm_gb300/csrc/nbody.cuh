@@ -462,13 +462,22 @@ __device__ __forceinline__ bool chord_chunk(
   }
 }
 
+// Sources of the chunk at s0, whole tiles.  nreal (optional): the source count on
+// the device where the host planned with an upper bound; chunks beyond it are empty.
+template <int TILE>
+__device__ __forceinline__ int64_t chunk_sources(int64_t s0, int64_t nsrc_pad, const int* nreal,
+                                                 int chunk_len) {
+  if (nreal) nsrc_pad = min(nsrc_pad, (int64_t(*nreal) + TILE - 1) / TILE * TILE);
+  return max(int64_t(0), min(nsrc_pad - s0, int64_t(chunk_len)));
+}
+
 template <typename T, int NDIM, bool WU, bool WP, bool SKIPC, int R, int NT, int TILE,
           int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     nbody_chord(const typename Vec4<T>::type* __restrict__ tgt,
                 const typename SrcRec<T>::type* __restrict__ src, int64_t ntgt_pad,
-                int64_t nsrc_pad, int chunk_len, T c0, double* __restrict__ part,
-                int* err) {
+                int64_t nsrc_pad, const int* __restrict__ nreal, int chunk_len, T c0,
+                double* __restrict__ part, int* err) {
   using V4 = typename Vec4<T>::type;
   using Rec = typename SrcRec<T>::type;
   constexpr int NC = ChordAcc<T, NDIM, WU, WP>::NC;
@@ -478,8 +487,7 @@ __global__ void __launch_bounds__(NT, MINB)
   const int tid = threadIdx.x;
   const int64_t tbase = (int64_t)blockIdx.x * (NT * R);
   const int64_t s0 = (int64_t)blockIdx.y * chunk_len;
-  int64_t slen = nsrc_pad - s0;
-  if (slen > chunk_len) slen = chunk_len;
+  const int64_t slen = chunk_sources<TILE>(s0, nsrc_pad, nreal, chunk_len);
 
   T tx[R], ty[R], tz[R];
 #pragma unroll
@@ -536,7 +544,7 @@ template <int FORM, bool WU, bool WP, int R, int NT, int TILE>
 __global__ void __launch_bounds__(NT)
     nbody_f64(const double4_16a* __restrict__ tgt, const int* __restrict__ tself,
               const double4_16a* __restrict__ src, int64_t ntgt_pad,
-              int64_t nsrc_pad, int chunk_len, double eps2,
+              int64_t nsrc_pad, const int* __restrict__ nreal, int chunk_len, double eps2,
               double* __restrict__ part, int* err) {
   constexpr int ND = (FORM == 2) ? 2 : 3;
   constexpr int NC = (WU ? ND : 0) + (WP ? 1 : 0);
@@ -546,8 +554,7 @@ __global__ void __launch_bounds__(NT)
   const int tid = threadIdx.x;
   const int64_t tbase = (int64_t)blockIdx.x * (NT * R);
   const int64_t s0 = (int64_t)blockIdx.y * chunk_len;
-  int64_t slen = nsrc_pad - s0;
-  if (slen > chunk_len) slen = chunk_len;
+  const int64_t slen = chunk_sources<TILE>(s0, nsrc_pad, nreal, chunk_len);
 
   double x0[R], x1[R], x2[R];
   int self[R];
@@ -679,7 +686,7 @@ template <int FORM, bool WU, bool WP, int R, int NT, int TILE>
 __global__ void __launch_bounds__(NT)
     nbody_f64h(const double4_16a* __restrict__ tgt, const int* __restrict__ tself,
                const double4_16a* __restrict__ src, int64_t ntgt_pad,
-               int64_t nsrc_pad, int chunk_len, double eps2,
+               int64_t nsrc_pad, const int* __restrict__ nreal, int chunk_len, double eps2,
                double* __restrict__ part, int* err) {
   constexpr int ND = (FORM == 2) ? 2 : 3;
   constexpr int NC = (WU ? ND : 0) + (WP ? 1 : 0);
@@ -689,8 +696,7 @@ __global__ void __launch_bounds__(NT)
   const int tid = threadIdx.x;
   const int64_t tbase = (int64_t)blockIdx.x * (NT * R);
   const int64_t s0 = (int64_t)blockIdx.y * chunk_len;
-  int64_t slen = nsrc_pad - s0;
-  if (slen > chunk_len) slen = chunk_len;
+  const int64_t slen = chunk_sources<TILE>(s0, nsrc_pad, nreal, chunk_len);
 
   double x0[R], x1[R], x2[R];
   int self[R];
