@@ -308,10 +308,10 @@ void combine_dispatch(lpm_context& ctx, const NbodyPlan& p, const double* part,
     launch_combine<MODE, NDIM, false, true>(ctx, p, part, off, seg, tgt, sg, c0);
 }
 
-template <typename T, int NDIM, bool WU, bool WP, bool SKIPC, int R, int NT, int MINB>
+template <typename T, int NDIM, bool WU, bool WP, bool SKIPC, int R, int NT, int MINB,
+          int TILE = std::is_same<T, float>::value ? F32_TILE : F64_TILE>
 void launch_chord_shape(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
                         const void* src, double* part, T c0) {
-  constexpr int TILE = std::is_same<T, float>::value ? F32_TILE : F64_TILE;
   using V4 = typename Vec4<T>::type;
   using Rec = typename SrcRec<T>::type;
   dim3 grid(unsigned(p.ntgt_pad / (NT * R)), unsigned(p.nchunks));
@@ -352,6 +352,8 @@ void launch_chord_k(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
       default:
         launch_chord_shape<T, NDIM, WU, WP, SKIPC, 4, 256, 3>(ctx, p, tgt, src, part, c0);
     }
+  } else if (p.fine) {
+    launch_chord_shape<T, NDIM, WU, WP, SKIPC, 1, FINE_NT, 4, FINE_TILE>(ctx, p, tgt, src, part, c0);
   } else {
     launch_chord_shape<T, NDIM, WU, WP, SKIPC, F64_R, F64_NT, 4>(ctx, p, tgt, src, part, c0);
   }
@@ -369,23 +371,17 @@ void launch_chord(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
 template <int FORM, bool WU, bool WP>
 void launch_f64(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
                 const int* tself, const void* src, double* part, double eps2) {
-  if (p.fine) {
-    dim3 g(unsigned(p.ntgt_pad / FINE_NT), unsigned(p.nchunks));
-    nbody_f64h<FORM, WU, WP, 1, FINE_NT, FINE_TILE><<<g, FINE_NT, 0, ctx.stream>>>(
-        static_cast<const double4_16a*>(tgt), tself, static_cast<const double4_16a*>(src),
-        p.ntgt_pad, p.nsrc_pad, p.nreal, p.chunk_len, eps2, part, ctx.d_err);
-    ctx.launches++;
-    return;
-  }
-  dim3 grid(unsigned(p.ntgt_pad / (F64_NT * F64_R)), unsigned(p.nchunks));
-  if (ref64_exact(p.precision))
-    nbody_f64<FORM, WU, WP, F64_R, F64_NT, F64_TILE><<<grid, F64_NT, 0, ctx.stream>>>(
-        static_cast<const double4_16a*>(tgt), tself, static_cast<const double4_16a*>(src),
-        p.ntgt_pad, p.nsrc_pad, p.nreal, p.chunk_len, eps2, part, ctx.d_err);
-  else
-    nbody_f64h<FORM, WU, WP, F64_R, F64_NT, F64_TILE><<<grid, F64_NT, 0, ctx.stream>>>(
-        static_cast<const double4_16a*>(tgt), tself, static_cast<const double4_16a*>(src),
-        p.ntgt_pad, p.nsrc_pad, p.nreal, p.chunk_len, eps2, part, ctx.d_err);
+  const int nt = p.fine ? FINE_NT : F64_NT, tb = p.fine ? FINE_NT : F64_NT * F64_R;
+  const bool exact = ref64_exact(p.precision);
+  auto* kernel =
+      p.fine ? (exact ? nbody_f64<FORM, WU, WP, 1, FINE_NT, FINE_TILE>
+                      : nbody_f64h<FORM, WU, WP, 1, FINE_NT, FINE_TILE>)
+             : (exact ? nbody_f64<FORM, WU, WP, F64_R, F64_NT, F64_TILE>
+                      : nbody_f64h<FORM, WU, WP, F64_R, F64_NT, F64_TILE>);
+  dim3 grid(unsigned(p.ntgt_pad / tb), unsigned(p.nchunks));
+  kernel<<<grid, nt, 0, ctx.stream>>>(static_cast<const double4_16a*>(tgt), tself,
+                                      static_cast<const double4_16a*>(src), p.ntgt_pad, p.nsrc_pad,
+                                      p.nreal, p.chunk_len, eps2, part, ctx.d_err);
   ctx.launches++;
 }
 
@@ -461,8 +457,8 @@ int64_t compact_sources(lpm_context& ctx, const uint8_t* mask, int64_t nslots,
 
 namespace {
 
-// FP64 kernels of a plan: nbody_split, the one-target-per-thread form of
-// nbody_f64h for grids too small for the tiled one, or the tiled kernels.
+// FP64 kernels of a plan: nbody_split, the one-target-per-thread form of the tiled
+// kernels for grids too small for them, or those.
 enum Fp64Kind : int { FP64_TILED = 0, FP64_FINE = 1, FP64_SPLIT = 2 };
 
 // Whether the split sums (nbody_split.cuh) replace nbody_f64h: the sphere
@@ -528,7 +524,7 @@ NbodyPlan plan_nbody(lpm_context& ctx, int precision, int ndim, int form,
   int kind = FP64_TILED;
   if (split_wanted(precision, ndim, ntgt, nsrc)) {
     kind = FP64_SPLIT;
-  } else if (precision == LPM_FP64) {
+  } else if (precision != LPM_FP32C) {
     // tiled grid below two waves: a CTA's serial 256-source tile (2.9e5 clocks
     // of the FP64 pipe) is the launch's whole time
     const int64_t ctas = ((ntgt + F64_NT * F64_R - 1) / (F64_NT * F64_R)) *
@@ -543,7 +539,7 @@ void plan_bounds(lpm_context& ctx, int precision, int ndim, int form, bool wu, b
   *b = PlanBounds{};
   for (int kind = FP64_TILED; kind <= FP64_SPLIT; ++kind) {
     if (kind == FP64_SPLIT && !split_wanted(precision, ndim, ntgt, nsrc)) continue;
-    if (kind == FP64_FINE && precision != LPM_FP64) continue;
+    if (kind == FP64_FINE && precision == LPM_FP32C) continue;
     const NbodyPlan p = plan_kind(ctx, precision, ndim, form, wu, wp, ntgt, nsrc, kind);
     b->ntgt_pad = std::max(b->ntgt_pad, p.ntgt_pad);
     b->nsrc_pad = std::max(b->nsrc_pad, p.nsrc_pad);
@@ -594,13 +590,20 @@ int tune_shape(lpm_context& ctx, const NbodyPlan& p0, const void* tgt, const int
   const uint64_t key = (uint64_t(p0.ndim) << 60) | (uint64_t(p0.wu) << 59) |
                        (uint64_t(p0.wp) << 58) | (uint64_t(p0.skipc) << 57) |
                        (lg(p0.ntgt_pad) << 8) | lg(p0.nsrc_pad);
+  // below ~2e9 pairs a launch lasts a few hundred microseconds: not timed.  512
+  // targets per CTA (shape 3) where that leaves SMs idle all the same -- a CTA's
+  // serial tile is then the launch's time -- and for the sphere's stream function
+  // (its extra MUFU work hides behind more warps); else 1,024 at 2 CTAs per SM.
+  // Measured, us per step or call at icosahedral levels 2 / 3 / 4 / 5: velocity
+  // RK4 117 / 123 / 164 / 997 (shape 3), 140 / 145 / 151 / 977 (shape 5), 170 /
+  // 176 / 180 / 1057 (shape 0); with stream function, levels 2 / 4 / 5: 95 / 111 /
+  // 456 (shape 3), 123 / 136 / 479 (shape 5), 140 / 152 / 490 (shape 0).
+  if (!ctx.autotune || double(p0.ntgt_pad) * double(p0.nsrc_pad) < 2e9) {
+    const int64_t ctas = p0.ntgt_pad / 512 * p0.nchunks;
+    return (p0.wp && p0.ndim == 3) || ctas < ctx.num_sms ? 3 : 5;
+  }
   auto it = ctx.tuned.find(key);
   if (it != ctx.tuned.end()) return it->second;
-  // below ~2e9 pairs a launch lasts a few hundred microseconds: keep the default
-  if (!ctx.autotune || double(p0.ntgt_pad) * double(p0.nsrc_pad) < 2e9) {
-    ctx.tuned[key] = 0;
-    return 0;
-  }
   cudaEvent_t e0, e1;
   LPM_CUDA(cudaEventCreate(&e0));
   LPM_CUDA(cudaEventCreate(&e1));

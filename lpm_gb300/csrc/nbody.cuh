@@ -876,7 +876,7 @@ __device__ __forceinline__ void chord_epilogue(const double* a, const double* p,
 constexpr int F32_NT = 256, F32_R = 4, F32_TILE = 512;
 constexpr int F32_TB = 1024;  // target padding: every FP32 shape divides it
 constexpr int F64_NT = 128, F64_R = 2, F64_TILE = 256;
-// FP64 small grids: one target per thread, 8-source tiles, so that a few
+// FP64 small grids (all FP64 forms): one target per thread, 8-source tiles, so that a few
 // thousand targets and sources still give every SM work (a warp's FP64
 // instruction takes 64 clocks of its SM sub-partition).
 constexpr int FINE_NT = 64, FINE_TILE = 8;
