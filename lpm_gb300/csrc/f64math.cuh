@@ -1,38 +1,61 @@
 // f64math.cuh -- FP64 logarithm, exponential and reciprocal for pair loops that
-// the FP64 pipe bounds (about 1.7 operations per clock per SM): table lookups and
-// integer operations, which run beside it, take the place of FP64 ones.
+// the FP64 pipe bounds (about 1.7 operations per clock per SM: 64 clocks of a
+// sub-partition's pipe per warp instruction).  The other pipes' issue slots are
+// free there, so the values are formed in 64-bit fixed point (integer operations,
+// FP32 for the last terms) and tables, and rounded to FP64 once:
 //
-// log x: x = 2^k m; f = 1/c for the centre c of m's interval of width 2^-9 (table),
-// r = m f - 1 (fused), log x = k ln 2 - log f + log1p(r), the series to r^5 / 5 for
-// |r| <= 2^-10: 9 FP64 operations.
-// exp(-p): -p = (256 n + j) ln 2 / 256 + f, 2^(j/256) from a table, exp(f) by its
-// series to f^5 / 120 for |f| <= ln 2 / 512: 11 FP64 operations.
-// Both from the textbook reductions (Cody and Waite; Tang's table-driven
-// methods); absolute error of log about 2e-16 (1 + |log x| / 2), relative error of
-// exp about 3e-16.
+// 1/x: FP32 reciprocal y of the mantissa m, e = 1 - m y exactly (integers modulo
+// 2^64), y (1 + e + e^2): no FP64 operation.
+// log x: x = 2^k m; f = 1/c to 22 bits for the centre c of m's interval of width
+// 2^-12 (table), r = m f - 1 exactly (integers modulo 2^64), log x = (k ln 2 - log f)
+// + log1p(r), the series to r^4 / 4 in fixed point of 74 bits: 2 FP64 additions.
+// exp(-p): p = n ln 2 / 8192 + r in fixed point of 76 bits, 2^(-n/8192) from a table of
+// 63 bits, exp(-r) by its series to the cube: no FP64 operation.
+// The range reductions are those of Cody and Waite, and Tang's table-driven
+// methods.  Errors: 1/x and exp about half a unit in the last place, log two
+// roundings of its parts.  The tables (145 KB) are read through L1.
 #pragma once
+
+#include <cstdint>
 
 #include <cuda_runtime.h>
 
 namespace lpm {
 
-constexpr int kLogBits = 9;
-struct F64Tables {
-  double2 lg[1 << kLogBits];  // f, -log f (less ln 2 above sqrt 2)
-  double ex[256];             // 2^(j/256)
-};
+constexpr int kLogBits = 12, kExpBits = 13;
+constexpr int kF64Entries = 1 << kExpBits;  // of the largest table
 constexpr double kLn2 = 0.69314718055994530942;
+struct __align__(16) F64LogEntry {
+  double y;    // -log f, less ln 2 above sqrt 2
+  unsigned f;  // 2^22 f
+  unsigned up;  // 1 above sqrt 2: the exponent counts one more
+};
+struct __align__(16) F64Tables {
+  F64LogEntry lg[1 << kLogBits];
+  uint64_t ex[1 << kExpBits];  // 2^63 2^(-j / 2^kExpBits)
+  double kl[2050];             // (e - 1023) ln 2
+};
 
-constexpr double kMagic = 6755399441055744.0;  // 2^52 + 2^51: integers in the low word
-
-// Entry i of the tables, i in [0, 2^kLogBits).
+// Entry i of the tables, i in [0, kF64Entries).
 __device__ __forceinline__ void f64_table_entry(F64Tables* T, int i) {
-  {
+  if (i < 1 << kLogBits) {
     const double c = 1.0 + (i + 0.5) / (1 << kLogBits);
-    const double f = 1.0 / c;
-    T->lg[i] = make_double2(f, -log(f) - (c > 1.41421356237309504880 ? kLn2 : 0.0));
+    const unsigned f = unsigned(rint(0x1p22 / c));
+    const bool up = c > 1.41421356237309504880;
+    T->lg[i] = F64LogEntry{-log(f * 0x1p-22) - (up ? kLn2 : 0.0), f, unsigned(up)};
   }
-  if (i < 256) T->ex[i] = exp2(i / 256.0);
+  if (i < 2050) T->kl[i] = (i - 1023) * kLn2;
+  // 2^64 2^(-2^k / 8192), multiplied over the bits of i
+  constexpr uint64_t root[kExpBits] = {
+      0xfffa747ea0040664ull, 0xfff4e91bff1b8c3eull, 0xffe9d2b2f7db2756ull, 0xffd3a751c0f7e10cull,
+      0xffa756521c8daed2ull, 0xff4ecb59511ec8a5ull, 0xfe9e115c7b8f884cull, 0xfd3e0c0cf486c175ull,
+      0xfa83b2db722a033aull, 0xf5257d152486cc2cull, 0xeac0c6e7dd24392full, 0xd744fccad69d6af4ull,
+      0xb504f333f9de6484ull};
+  uint64_t t = uint64_t(1) << 63;
+#pragma unroll
+  for (int k = 0; k < kExpBits; ++k)
+    if (i >> k & 1) t = __umul64hi(t, root[k]);
+  T->ex[i] = t;
 }
 
 // Whether x is a positive normal number in [2^-1000, 2^1000).
@@ -41,49 +64,64 @@ __device__ __forceinline__ bool f64_plain(double x) {
   return h - (23u << 20) < (2000u << 20);
 }
 
-// 1/d, d as f64_plain: the approximate reciprocal (relative error e below
-// 2^-20) times 1 + e + e^2.
+__device__ __forceinline__ uint64_t f64_mantissa(double x) {  // 2^52 m, m in [1, 2)
+  return (uint64_t(__double_as_longlong(x)) & 0xfffffffffffffull) | 0x10000000000000ull;
+}
+// 1/d, |d| as f64_plain.
 __device__ __forceinline__ double f64_rcp(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  return fma(r, fma(e, e, e), r);
+  const unsigned h = unsigned(__double2hiint(d)), l = unsigned(__double2loint(d));
+  const float mh = __int_as_float(int(__funnelshift_l(l, h & 0xfffff, 3)) | 0x3f800000);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(mh));
+  y = fminf(y, 0x1.fffffep-1f);
+  const unsigned Y = (unsigned(__float_as_int(y)) & 0x7fffff) | 0x800000;  // 2^24 y
+  const int64_t E = -int64_t(f64_mantissa(d) * Y);                         // 2^76 (1 - m y)
+  const int e = int(E >> 32);                                              // 2^44 e
+  const int64_t e2 = (int64_t(e) * e) >> 24;                               // 2^64 e^2
+  // 2^63 / m
+  const uint64_t W = (uint64_t(Y) << 39) + uint64_t((int64_t(Y) * (E >> 16)) >> 21) +
+                     ((uint64_t(unsigned(e2)) * Y) >> 25);
+  const uint64_t b = ((W + 0x200) >> 10) + (uint64_t(2044 - ((h >> 20) & 0x7ff)) << 52);
+  return __hiloint2double(int(unsigned(b >> 32) | (h & 0x80000000u)), int(unsigned(b)));
 }
 
-__device__ __forceinline__ double f64_log(const F64Tables& T, double x) {
+// log x, x as f64_plain.
+__device__ __forceinline__ double f64_log(const F64Tables* __restrict__ T, double x) {
   const int h = __double2hiint(x);
-  const int i = (h >> (20 - kLogBits)) & ((1 << kLogBits) - 1);
-  const double2 t = T.lg[i];
-  // above sqrt 2 the table holds -log f - ln 2 and the exponent counts one more
-  const int k = (h >> 20) - 1023 + (t.y < 0.0 ? 1 : 0);
-  const double m = __hiloint2double((h & 0xfffff) | 0x3ff00000, __double2loint(x));
-  const double kd = __hiloint2double(0x43380000, k + 2048) - (kMagic + 2048.0);
-  const double r = fma(m, t.x, -1.0);
-  double p = fma(r, 0.2, -0.25);
-  p = fma(r, p, 1.0 / 3);
-  p = fma(r, p, -0.5);
-  return fma(kd, kLn2, t.y) + fma(r * r, p, r);
+  const int4 t4 = reinterpret_cast<const int4*>(T->lg)[(h >> (20 - kLogBits)) & ((1 << kLogBits) - 1)];
+  const double base = T->kl[(h >> 20) + t4.w] + __hiloint2double(t4.y, t4.x);
+  const int64_t r = int64_t(f64_mantissa(x) * unsigned(t4.z));  // 2^74 r, |r| < 2^-12.9
+  const int r1 = int((r + (int64_t(1) << 30)) >> 31);           // 2^43 r
+  const float rf = float(r1) * 0x1p-43f;
+  const int c = __float2int_rn(rf * rf * rf * fmaf(rf, -0.25f, 1.f / 3) * 0x1p66f);
+  const int64_t v = r - ((int64_t(r1) * r1) >> 13) + (int64_t(c) << 8);  // 2^74 log1p(r)
+  const uint64_t a = uint64_t(v < 0 ? -v : v);
+  const int z = __clzll(int64_t(a));
+  const uint64_t b = ((a << z) >> 11) + (uint64_t(unsigned(1023 - 12 - z)) << 52);
+  return base + __hiloint2double(int(unsigned(b >> 32) | (unsigned(v >> 32) & 0x80000000u)),
+                                 int(unsigned(b)));
 }
 
 // q exp(-p) for 0 <= p < 746 (beyond, exp(-p) is 0 in FP64); q finite.
-__device__ __forceinline__ double f64_mul_exp_neg(const F64Tables& T, double q, double p) {
-  const double z = fma(p, -369.3299304675746, kMagic);  // -256 / ln 2
-  const int n = __double2loint(z);
-  const double zf = z - kMagic;
-  // ln 2 / 256 in two parts, the first of 29 bits: zf times it is exact
-  double f = fma(zf, -0x1.62e42fep-9, -p);
-  f = fma(zf, -0x1.f473de6af278fp-38, f);
-  double e = fma(f, 1.0 / 120, 1.0 / 24);
-  e = fma(f, e, 1.0 / 6);
-  e = fma(f, e, 0.5);
-  e = fma(f * f, e, f);
-  // 2^k into the exponent of the table value, as far as it stays normal
-  const double t0 = T.ex[n & 255];
-  const int k = n >> 8, k1 = max(k, -1000);
-  const double t = __hiloint2double(__double2hiint(t0) + (k1 << 20), __double2loint(t0));
-  double v = q * fma(t, e, t);
-  if (k < k1) v *= __hiloint2double((1023 + k - k1) << 20, 0);
-  return v;
+__device__ __forceinline__ double f64_mul_exp_neg(const F64Tables* __restrict__ T, double q,
+                                                  double p) {
+  const int ep = int((unsigned(__double2hiint(p)) >> 20) & 0x7ff) - 1023;  // <= 9
+  const uint64_t P = (f64_mantissa(p) << 11) >> min(unsigned(9 - ep), 63u);  // 2^54 p
+  const unsigned n = unsigned((uint64_t(unsigned(P >> 32)) * 12102203u) >> 32);
+  const int64_t r = int64_t((P << 22) - n * 0x58b90bfbe8e7bcd6ull);  // 2^76 r, r < 2^-13.4
+  const int r1 = int((r + (int64_t(1) << 31)) >> 32);                // 2^44 r
+  const float rf = float(r1) * 0x1p-44f;
+  const int c = __float2int_rn(rf * rf * rf * fmaf(rf, -1.f / 24, 1.f / 6) * 0x1p70f);
+  const int64_t v = ((int64_t(r1) * r1) >> 13) - r - (int64_t(c) << 6);  // 2^76 (exp(-r) - 1)
+  const uint64_t t = T->ex[n & ((1 << kExpBits) - 1)];
+  const uint64_t E = t + uint64_t(__mul64hi(int64_t(t >> 1), v) >> 11);  // 2^63 2^(-j/8192 - r)
+  const int z = __clzll(int64_t(E));
+  const int e = 1023 - z - int(n >> kExpBits), e1 = max(e, 23);
+  const uint64_t a = E << z;
+  const uint64_t b = (a >> 11) + (a >> 10 & 1) + (uint64_t(unsigned(e1 - 1)) << 52);
+  double w = q * __longlong_as_double(int64_t(b));
+  if (e < e1) w *= __hiloint2double((1023 + e - e1) << 20, 0);
+  return w;
 }
 
 }  // namespace lpm

@@ -40,13 +40,13 @@ __device__ __forceinline__ double ds(double a, double b) { return __dsub_rn(a, b
 constexpr int kSweNT = 128;   // targets per CTA
 constexpr int kSweTile = 256;  // sources per shared-memory tile (FP32)
 // FP64: small tiles and chunks, so that a few thousand points spread evenly
-// (a warp's pair takes 3,500 clocks of its SM sub-partition's FP64 pipe)
+// (a warp's pair takes 2,000 to 3,000 clocks of its sub-partition's FP64 pipe)
 constexpr int kSweTile64 = 64;
 
 // ---- planar SWE sums, FP64 --------------------------------------------------
-// With r = 1 / R, a = rot r, b = pot r, m = d1^2 - d0^2, the eleven sums
-//   U, V    = sum -a d1 + b d0, sum a d0 + b d1
-//   A1..A3  = sum a r (m, d0 d1, 1),   B1..B3 = sum b r (m, d0 d1, 1)
+// With e = d / R, the eleven sums
+//   U, V    = sum -rot e1 + pot e0, sum rot e0 + pot e1
+//   A1..A3  = sum rot (e1^2 - e0^2, e0 e1, 1 / R^2),   B1..B3 the same with pot
 //   L       = sum (s_y - s_x) A (40 (1 - p) + 10 p^2 - 2 p^3 / 3) e^-p,
 //             p = |d|^2 / pse_eps^2
 //   P, Q    = sum rot log R, sum pot log R
@@ -54,12 +54,13 @@ constexpr int kSweTile64 = 64;
 //   2 pi du/dx = 2 A2 + B1 + eps^2 B3,   2 pi du/dy = A1 - eps^2 A3 - 2 B2,
 //   2 pi dv/dx = A1 + eps^2 A3 - 2 B2,   2 pi dv/dy = -2 A2 - B1 + eps^2 B3,
 //   lap = L / (pi pse_eps^2), psi, phi = -P / 4 pi, -Q / 4 pi
-// (R/2 taken from d1^2 and d0^2 pair by pair, so no large sums cancel).
-// The FP64 pipe bounds the kernel: 55 operations per pair (one approximate
-// reciprocal, the logarithm and exponential of f64math.cuh) against about 260
-// for the reference's operation order with its eight divisions, square root
-// and library log and exp: quad level 5, vertices and faces, 19.6 -> 4.7 ms
-// (0.88 of the pipe's measured rate).
+// (R/2 taken from e1^2 and e0^2 pair by pair, so no large sums cancel).
+// The FP64 pipe bounds the kernel, 64 clocks of a sub-partition per operation of a
+// warp: 33 operations per pair, the reciprocal, logarithm and exponential in
+// integers (f64math.cuh), against about 260 for the reference's operation order
+// with its eight divisions, square root and library log and exp.  Quad level 5,
+// vertices and faces: 19.6 ms in that order, 4.73 ms with 55 operations (Newton
+// steps and series in FP64), 2.89 ms now (0.9 of the pipe's measured rate).
 constexpr int kSweNC = 11;
 
 struct __align__(16) SweSrc {
@@ -67,12 +68,14 @@ struct __align__(16) SweSrc {
   int slot, pad[3];
 };
 
-// The last two blocks fill the tables of f64math.cuh.
+// The last kTabBlocks blocks fill the tables of f64math.cuh.
+constexpr int kTabBlocks = kF64Entries / 256;
+
 __global__ void k_swe_pack(View fx, const double* __restrict__ zeta, const double* __restrict__ sigma,
                            const double* __restrict__ area, const double* __restrict__ sfc,
                            const int* __restrict__ src2slot, int64_t ns, SweSrc* __restrict__ src,
                            F64Tables* __restrict__ tab) {
-  const int tb = int(gridDim.x) - 2;
+  const int tb = int(gridDim.x) - kTabBlocks;
   if (int(blockIdx.x) >= tb) {
     f64_table_entry(tab, (int(blockIdx.x) - tb) * 256 + threadIdx.x);
     return;
@@ -91,14 +94,6 @@ __global__ void k_swe_pack(View fx, const double* __restrict__ zeta, const doubl
   r.pad[0] = r.pad[1] = r.pad[2] = 0;
   src[k] = r;
 }
-static_assert((1 << kLogBits) == 512, "k_swe_pack fills the tables with two blocks of 256");
-
-__device__ __forceinline__ void load_tables(F64Tables& t, const F64Tables* __restrict__ g) {
-  const auto* s = reinterpret_cast<const double2*>(g);
-  auto* d = reinterpret_cast<double2*>(&t);
-  for (int i = threadIdx.x; i < int(sizeof(F64Tables) / 16); i += blockDim.x) d[i] = s[i];
-}
-
 // COLL: collocated targets, the source in the target's own slot is skipped.
 template <bool COLL>
 __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __restrict__ ts,
@@ -107,8 +102,6 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
                                                       double ipse2, const F64Tables* __restrict__ tab,
                                                       double* __restrict__ part, int64_t tpad) {
   __shared__ SweSrc tile[kSweTile64];
-  __shared__ F64Tables T;
-  load_tables(T, tab);
   const int64_t i = blockIdx.x * int64_t(kSweNT) + threadIdx.x;
   const int64_t c = blockIdx.y;
   const int64_t j0 = c * chunk_len, j1 = ns < j0 + chunk_len ? ns : j0 + chunk_len;
@@ -130,31 +123,33 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
       const SweSrc& y = tile[q];
       if (COLL && y.slot == i) continue;
       const double d0 = x0 - y.x, d1 = x1 - y.y;
-      const double d00 = d0 * d0, d11 = d1 * d1;
-      const double rsq = d00 + d11, R = rsq + epssq;
+      const double rsq = fma(d1, d1, d0 * d0), R = rsq + epssq;
       double w, lg;
       if (f64_plain(R)) {
         w = f64_rcp(R);
-        lg = f64_log(T, R);
+        lg = f64_log(tab, R);
       } else {  // coincident points, out-of-range values
         w = 1.0 / R;
         lg = log(R);
       }
-      const double a = y.rot * w, b = y.pot * w;
-      r[0] = fma(-a, d1, fma(b, d0, r[0]));
-      r[1] = fma(a, d0, fma(b, d1, r[1]));
-      const double a2 = a * w, b2 = b * w, md = d11 - d00, xy = d0 * d1;
-      r[2] = fma(a2, md, r[2]);
-      r[3] = fma(a2, xy, r[3]);
-      r[4] += a2;
-      r[5] = fma(b2, md, r[5]);
-      r[6] = fma(b2, xy, r[6]);
-      r[7] += b2;
+      const double e0 = d0 * w, e1 = d1 * w;
+      r[0] = fma(-y.rot, e1, fma(y.pot, e0, r[0]));
+      r[1] = fma(y.rot, e0, fma(y.pot, e1, r[1]));
+      const double w2 = w * w, md = fma(e1, e1, -(e0 * e0)), xy = e0 * e1;
+      r[2] = fma(y.rot, md, r[2]);
+      r[3] = fma(y.rot, xy, r[3]);
+      r[4] = fma(y.rot, w2, r[4]);
+      r[5] = fma(y.pot, md, r[5]);
+      r[6] = fma(y.pot, xy, r[6]);
+      r[7] = fma(y.pot, w2, r[7]);
       const double p = rsq * ipse2;
       double pre = fma(p, -2.0 / 3, 10.0);
       pre = fma(p, pre, -40.0);
       pre = fma(p, pre, 40.0);
-      if (!(p >= 746.0)) r[8] = fma((y.s - si) * y.area, f64_mul_exp_neg(T, pre, p), r[8]);
+      // p < 746 or NaN, by the high word (p >= 0)
+      const unsigned hp = unsigned(__double2hiint(p));
+      if (hp < 0x40875000u || hp > 0x7ff00000u)
+        r[8] = fma((y.s - si) * y.area, f64_mul_exp_neg(tab, pre, p), r[8]);
       r[9] = fma(y.rot, lg, r[9]);
       r[10] = fma(y.pot, lg, r[10]);
     }
@@ -414,10 +409,12 @@ __global__ void k_swe_plane32_out(const double* __restrict__ part, int nchunks, 
 // FP64: s and D = (1 - s) + eps^2 unfused in the reference's order (D is
 // the ill-conditioned quantity: a one-ulp change of s moves a near pair's D by
 // ~1e-16 / D relative), everything after it contracted, one reciprocal of D per
-// pair.  The FP64 pipe bounds the kernel: 51 operations per pair (66 in the form
-// that added c v^T, v w^T, u term by term): icosahedral level 5, vertices and
-// faces, 96.5 -> 81.8 ms (0.91 of the pipe's measured rate); level 2, where
-// 64-source chunks instead of 256-source ones fill the SMs, 1.31 -> 0.38 ms.
+// pair in integers (f64math.cuh).  The FP64 pipe bounds the kernel: 48 operations
+// per pair (66 in the form that added c v^T, v w^T, u term by term): icosahedral
+// level 5, vertices and faces, 96.5 -> 68.9 ms (81.8 ms with the reciprocal by the
+// hardware's FP64 approximation and three operations, which costs eight);
+// level 2, where 64-source chunks instead of 256-source ones fill the SMs,
+// 1.31 -> 0.34 ms.
 constexpr int kSphNC = 28;  // A3 B3 U1[3] V1[3] U2[6] V2[6] Z G H K
 
 struct __align__(16) SphSrc {
@@ -955,7 +952,7 @@ void swe_plane_sums(lpm_context& ctx, View tx, const double* ts, int64_t nt, Vie
   const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(SweSrc), kSweNC, false, kSweTile64);
   auto* src = static_cast<SweSrc*>(p.src);
   auto* tab = static_cast<F64Tables*>(ctx.arena.take(sizeof(F64Tables)));
-  k_swe_pack<<<blocks256(p.ns) + 2, 256, 0, ctx.stream>>>(fx, zeta, sigma, area, sfc, p.src2slot,
+  k_swe_pack<<<blocks256(p.ns) + kTabBlocks, 256, 0, ctx.stream>>>(fx, zeta, sigma, area, sfc, p.src2slot,
                                                           p.ns, src, tab);
   ctx.launches++;
   const double epssq = eps * eps, ipse2 = 1.0 / (pse_eps * pse_eps);
