@@ -185,6 +185,7 @@ int lpm_context_create(lpm_context** out, int device) {
     c->num_sms = prop.multiProcessorCount;
     LPM_CUDA(cudaMalloc(&c->d_err, sizeof(int)));
     LPM_CUDA(cudaMemset(c->d_err, 0, sizeof(int)));
+    c->f64_tab = lpm::make_f64_tables();
     *out = c;
     return LPM_OK;
   } catch (...) {
@@ -198,6 +199,7 @@ int lpm_context_destroy(lpm_context* ctx) {
   cudaStreamSynchronize(ctx->stream);
   ctx->arena.release();
   if (ctx->d_err) cudaFree(ctx->d_err);
+  if (ctx->f64_tab) cudaFree(ctx->f64_tab);
   delete ctx;
   return LPM_OK;
 }

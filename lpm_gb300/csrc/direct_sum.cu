@@ -317,7 +317,7 @@ void launch_chord_shape(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
   dim3 grid(unsigned(p.ntgt_pad / (NT * R)), unsigned(p.nchunks));
   nbody_chord<T, NDIM, WU, WP, SKIPC, R, NT, TILE, MINB><<<grid, NT, 0, ctx.stream>>>(
       static_cast<const V4*>(tgt), static_cast<const Rec*>(src), p.ntgt_pad, p.nsrc_pad,
-      p.nreal, p.chunk_len, c0, part, ctx.d_err);
+      p.nreal, p.chunk_len, c0, part, ctx.d_err, ctx.f64_tab);
   ctx.launches++;
 }
 
@@ -372,16 +372,20 @@ template <int FORM, bool WU, bool WP>
 void launch_f64(lpm_context& ctx, const NbodyPlan& p, const void* tgt,
                 const int* tself, const void* src, double* part, double eps2) {
   const int nt = p.fine ? FINE_NT : F64_NT, tb = p.fine ? FINE_NT : F64_NT * F64_R;
-  const bool exact = ref64_exact(p.precision);
-  auto* kernel =
-      p.fine ? (exact ? nbody_f64<FORM, WU, WP, 1, FINE_NT, FINE_TILE>
-                      : nbody_f64h<FORM, WU, WP, 1, FINE_NT, FINE_TILE>)
-             : (exact ? nbody_f64<FORM, WU, WP, F64_R, F64_NT, F64_TILE>
-                      : nbody_f64h<FORM, WU, WP, F64_R, F64_NT, F64_TILE>);
-  dim3 grid(unsigned(p.ntgt_pad / tb), unsigned(p.nchunks));
-  kernel<<<grid, nt, 0, ctx.stream>>>(static_cast<const double4_16a*>(tgt), tself,
-                                      static_cast<const double4_16a*>(src), p.ntgt_pad, p.nsrc_pad,
-                                      p.nreal, p.chunk_len, eps2, part, ctx.d_err);
+  const dim3 grid(unsigned(p.ntgt_pad / tb), unsigned(p.nchunks));
+  const auto* t = static_cast<const double4_16a*>(tgt);
+  const auto* y = static_cast<const double4_16a*>(src);
+  if (ref64_exact(p.precision)) {
+    auto* kernel = p.fine ? nbody_f64<FORM, WU, WP, 1, FINE_NT, FINE_TILE>
+                          : nbody_f64<FORM, WU, WP, F64_R, F64_NT, F64_TILE>;
+    kernel<<<grid, nt, 0, ctx.stream>>>(t, tself, y, p.ntgt_pad, p.nsrc_pad, p.nreal, p.chunk_len,
+                                        eps2, part, ctx.d_err);
+  } else {
+    auto* kernel = p.fine ? nbody_f64h<FORM, WU, WP, 1, FINE_NT, FINE_TILE>
+                          : nbody_f64h<FORM, WU, WP, F64_R, F64_NT, F64_TILE>;
+    kernel<<<grid, nt, 0, ctx.stream>>>(t, tself, y, p.ntgt_pad, p.nsrc_pad, p.nreal, p.chunk_len,
+                                        eps2, part, ctx.d_err, ctx.f64_tab);
+  }
   ctx.launches++;
 }
 
@@ -427,6 +431,21 @@ int occupancy(int precision) {
 }
 
 }  // namespace
+
+namespace {
+__global__ void k_f64_tables(F64Tables* t) {
+  f64_table_entry(t, int(blockIdx.x * blockDim.x + threadIdx.x));
+}
+}  // namespace
+
+F64Tables* make_f64_tables() {
+  F64Tables* t = nullptr;
+  LPM_CUDA(cudaMalloc(&t, sizeof(F64Tables)));
+  k_f64_tables<<<kF64Entries / 256, 256>>>(t);
+  LPM_CUDA(cudaGetLastError());
+  LPM_CUDA(cudaStreamSynchronize(nullptr));
+  return t;
+}
 
 float f32_c0(int ndim, double eps) { return float(chord_c0(ndim, eps)); }
 
@@ -500,9 +519,13 @@ NbodyPlan plan_kind(lpm_context& ctx, int precision, int ndim, int form, bool wu
   // Aim for ~16 waves of CTAs so the tail of the last wave stays small.  The
   // FP32 shapes share one chunking (4 CTAs of 1024 targets per SM) so that the
   // autotuner can swap shapes without changing the partial layout.  The fine
-  // form serves grids of a wave or two: two waves.
+  // form: two waves (16 warps per SM), and up to eight, which hide the latency of
+  // a pair's chain of operations, while a chunk keeps 64 sources (chord form,
+  // 14,336 targets x 6,144 sources: two waves 2.23 ms, eight 1.91; 1,089 x 1,024:
+  // 43 and 61 us).
   const int64_t slots = int64_t(std::max(ctx.num_sms, 1)) * s.ctas;
   int64_t nch = ((p.fine ? 2 : p.split ? 8 : 16) * slots + ntb - 1) / ntb;
+  if (p.fine) nch = std::max(nch, std::min(4 * nch, ntiles / (64 / FINE_TILE)));
   if (ctx.max_part_bytes > 0) {
     const int64_t per_chunk = int64_t(sizeof(double)) * p.ncomp * p.ntgt_pad;
     nch = std::min<int64_t>(nch, int64_t(ctx.max_part_bytes) / per_chunk);

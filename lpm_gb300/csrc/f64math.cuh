@@ -8,7 +8,7 @@
 // 2^64), y (1 + e + e^2): no FP64 operation.
 // log x: x = 2^k m; f = 1/c to 22 bits for the centre c of m's interval of width
 // 2^-12 (table), r = m f - 1 exactly (integers modulo 2^64), log x = (k ln 2 - log f)
-// + log1p(r), the series to r^4 / 4 in fixed point of 74 bits: 2 FP64 additions.
+// + log1p(r), the series to r^5 / 5 in fixed point of 74 bits: 2 FP64 additions.
 // exp(-p): p = n ln 2 / 8192 + r in fixed point of 76 bits, 2^(-n/8192) from a table of
 // 63 bits, exp(-r) by its series to the cube: no FP64 operation.
 // The range reductions are those of Cody and Waite, and Tang's table-driven
@@ -39,10 +39,11 @@ struct __align__(16) F64Tables {
 // Entry i of the tables, i in [0, kF64Entries).
 __device__ __forceinline__ void f64_table_entry(F64Tables* T, int i) {
   if (i < 1 << kLogBits) {
-    const double c = 1.0 + (i + 0.5) / (1 << kLogBits);
+    // f = 1 beside 1 and 1/2 beside 2: log x stays accurate relative to x - 1
+    const double c = i == 0 ? 1.0 : i == (1 << kLogBits) - 1 ? 2.0 : 1.0 + (i + 0.5) / (1 << kLogBits);
     const unsigned f = unsigned(rint(0x1p22 / c));
     const bool up = c > 1.41421356237309504880;
-    T->lg[i] = F64LogEntry{-log(f * 0x1p-22) - (up ? kLn2 : 0.0), f, unsigned(up)};
+    T->lg[i] = F64LogEntry{-log(f * (up ? 0x1p-21 : 0x1p-22)), f, unsigned(up)};
   }
   if (i < 2050) T->kl[i] = (i - 1023) * kLn2;
   // 2^64 2^(-2^k / 8192), multiplied over the bits of i
@@ -85,21 +86,37 @@ __device__ __forceinline__ double f64_rcp(double d) {
   return __hiloint2double(int(unsigned(b >> 32) | (h & 0x80000000u)), int(unsigned(b)));
 }
 
-// log x, x as f64_plain.
+// 1/d for any d.  The rare case is a call: inlined, its FP64 operations are issued
+// for every pair and the result selected.
+static __device__ __noinline__ double f64_inv_any(double d) { return 1.0 / d; }
+__device__ __forceinline__ double f64_inv(double d) {
+  return f64_plain(fabs(d)) ? f64_rcp(d) : f64_inv_any(d);
+}
+
+// log x, x as f64_plain and not within 2^-16 of 1 (where the error, 2^-67, outgrows
+// the result's last place).
 __device__ __forceinline__ double f64_log(const F64Tables* __restrict__ T, double x) {
   const int h = __double2hiint(x);
   const int4 t4 = reinterpret_cast<const int4*>(T->lg)[(h >> (20 - kLogBits)) & ((1 << kLogBits) - 1)];
   const double base = T->kl[(h >> 20) + t4.w] + __hiloint2double(t4.y, t4.x);
-  const int64_t r = int64_t(f64_mantissa(x) * unsigned(t4.z));  // 2^74 r, |r| < 2^-12.9
-  const int r1 = int((r + (int64_t(1) << 30)) >> 31);           // 2^43 r
-  const float rf = float(r1) * 0x1p-43f;
-  const int c = __float2int_rn(rf * rf * rf * fmaf(rf, -0.25f, 1.f / 3) * 0x1p66f);
-  const int64_t v = r - ((int64_t(r1) * r1) >> 13) + (int64_t(c) << 8);  // 2^74 log1p(r)
+  const int64_t r = int64_t(f64_mantissa(x) * unsigned(t4.z));  // 2^74 r, |r| < 2^-12
+  const float rf = float(int(r >> 32)) * 0x1p-42f;
+  const int c = __float2int_rn(rf * rf * rf * fmaf(rf, fmaf(rf, 0.2f, -0.25f), 1.f / 3) * 0x1p66f);
+  const int64_t v = r - (__mul64hi(r << 1, r << 1) >> 13) + (int64_t(c) << 8);  // 2^74 log1p(r)
   const uint64_t a = uint64_t(v < 0 ? -v : v);
-  const int z = __clzll(int64_t(a));
+  const int z = __clzll(int64_t(a | 1));
   const uint64_t b = ((a << z) >> 11) + (uint64_t(unsigned(1023 - 12 - z)) << 52);
   return base + __hiloint2double(int(unsigned(b >> 32) | (unsigned(v >> 32) & 0x80000000u)),
                                  int(unsigned(b)));
+}
+// Whether x is one that f64_log takes.
+__device__ __forceinline__ bool f64_log_plain(double x) {
+  return f64_plain(x) && unsigned(__double2hiint(x)) - 0x3fefffe0u >= 0x30u;
+}
+// log x for any x.
+static __device__ __noinline__ double f64_ln_any(double x) { return log(x); }
+__device__ __forceinline__ double f64_ln(const F64Tables* __restrict__ T, double x) {
+  return f64_log_plain(x) ? f64_log(T, x) : f64_ln_any(x);
 }
 
 // q exp(-p) for 0 <= p < 746 (beyond, exp(-p) is 0 in FP64); q finite.

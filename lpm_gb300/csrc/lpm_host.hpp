@@ -110,12 +110,19 @@ struct Arena {
 
 }  // namespace lpm
 
+namespace lpm {
+struct F64Tables;
+F64Tables* make_f64_tables();  // allocated and filled on the current device
+}  // namespace lpm
+
 struct lpm_context {
   int device = 0;
   cudaStream_t stream = nullptr;
   int precision = LPM_FP64;
   int num_sms = 0;
   int* d_err = nullptr;  // device flag: nonzero after a bounded wait gave up
+  // tables of the FP64 logarithm and exponential (f64math.cuh), filled once
+  lpm::F64Tables* f64_tab = nullptr;
   lpm::Arena arena;
   int64_t launches = 0;
   size_t max_part_bytes = 0;  // cap on chunk-partial scratch (0 = none)

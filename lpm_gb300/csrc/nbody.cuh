@@ -25,9 +25,13 @@
 // FP64 path (LPM_FP64, parity form within 1e-12).  The reference's kernels
 // (1 - x.y [+ eps^2] on the sphere, |x - y|^2 + eps^2 on the plane) with the
 // cross product hoisted out of the sum: per target B = sum_j (g_j / arg_j) y_j
-// and u = s (x cross B) in the epilogue; one quotient per pair by Newton's
-// method from the hardware's approximate reciprocal.  11 FP64 operations per
-// sphere pair (eps form), against ~32 with three correctly rounded divisions.
+// and u = s (x cross B) in the epilogue.  The reciprocal and the logarithm are
+// formed in integers (f64math.cuh), beside the FP64 pipe that bounds the loop: 8
+// FP64 operations per sphere pair (eps form), 7 per planar pair, against ~32 with
+// three correctly rounded divisions, and 3 more for the stream function.
+// Planar quad level 5, vertices and faces: velocity 0.96 -> 0.65 ms, with
+// stream function 3.81 -> 0.90 ms (against the hardware's FP64 approximation with
+// four operations, and the library's logarithm).
 //
 // FP64 exact path (LPM_FP64_EXACT).  Every pair term is computed with the
 // reference's formula and operation order using non-contracting intrinsics
@@ -42,6 +46,7 @@
 #include <cuda_runtime.h>
 
 #include "f32x2.cuh"
+#include "f64math.cuh"
 #include "lpm_gb300.h"
 
 namespace lpm {
@@ -194,7 +199,7 @@ struct TilePipe {
 //   src: vec4 (x, y, z, g) per source (plane: z = 0), nsrc_pad entries
 //   part: [chunk][comp][ntgt_pad] doubles; comps = (WU ? NDIM : 0) +
 //         (WP ? 1 : 0): (w0 w1 [w2] [L]) with L = sum g lg2 q
-// FP32 uses the MUFU reciprocal and log2; FP64 divides and calls log2.
+// FP32 uses the MUFU reciprocal and log2; FP64 takes both from f64math.cuh.
 // ---------------------------------------------------------------------------
 template <typename T> struct Vec4;
 template <> struct Vec4<float> { using type = float4; };
@@ -214,9 +219,11 @@ template <> struct SrcRec<float> { using type = SrcF32; };
 template <> struct SrcRec<double> { using type = double4_16a; };
 
 __device__ __forceinline__ float chord_rcp(float q) { return rcp_approx(q); }
-__device__ __forceinline__ double chord_rcp(double q) { return 1.0 / q; }
-__device__ __forceinline__ float chord_lg2(float q) { return lg2_approx(q); }
-__device__ __forceinline__ double chord_lg2(double q) { return log2(q); }
+__device__ __forceinline__ double chord_rcp(double q) { return f64_inv(q); }
+__device__ __forceinline__ float chord_lg2(float q, const F64Tables*) { return lg2_approx(q); }
+__device__ __forceinline__ double chord_lg2(double q, const F64Tables* tab) {
+  return 1.4426950408889634074 * f64_ln(tab, q);
+}
 __device__ __forceinline__ float chord_fma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double chord_fma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ void two_sum_acc(double& s, double& c, double p) {
@@ -328,7 +335,8 @@ template <typename T, int NDIM, bool WU, bool WP, bool SKIPC, int R, int TILE>
 __device__ __forceinline__ bool chord_chunk(
     TilePipe<typename SrcRec<T>::type, TILE>& pipe, const T (&tx)[R], const T (&ty)[R],
     const T (&tz)[R], T (&S)[ChordAcc<T, NDIM, WU, WP>::NC][R],
-    T (&C)[ChordAcc<T, NDIM, WU, WP>::NC][R], T c0, int* err) {
+    T (&C)[ChordAcc<T, NDIM, WU, WP>::NC][R], T c0, int* err,
+    const F64Tables* __restrict__ tab = nullptr) {
   using Rec = typename SrcRec<T>::type;
   constexpr int NC = ChordAcc<T, NDIM, WU, WP>::NC;
   if constexpr (std::is_same<T, float>::value) {
@@ -412,17 +420,19 @@ __device__ __forceinline__ bool chord_chunk(
     }
     return true;
   } else {
+    // merged by TwoSum every 64 sources, or every tile of more
+    constexpr int kMerge = TILE < 64 ? 64 / TILE : 1;
+    T P[NC][R];
+#pragma unroll
+    for (int k = 0; k < NC; ++k)
+#pragma unroll
+      for (int r = 0; r < R; ++r) P[k][r] = T(0);
     for (int t = 0; t < pipe.ntiles; ++t) {
       if (!pipe.acquire(t)) {
         pipe.drain(t, err);
         return false;
       }
       const Rec* sm = pipe.tile(t);
-      T P[NC][R];
-#pragma unroll
-      for (int k = 0; k < NC; ++k)
-#pragma unroll
-        for (int r = 0; r < R; ++r) P[k][r] = T(0);
 
 #pragma unroll 4
       for (int j = 0; j < TILE; ++j) {
@@ -446,16 +456,21 @@ __device__ __forceinline__ bool chord_chunk(
             if (NDIM == 3) P[2][r] = chord_fma(w, dz, P[2][r]);
           }
           if (WP) {
-            T lg = chord_lg2(q);
+            T lg = chord_lg2(q, tab);
             if (SKIPC) lg = (q == c0) ? T(0) : lg;
             P[NC - 1][r] = chord_fma(s.w, lg, P[NC - 1][r]);
           }
         }
       }
+      if ((t + 1) % kMerge == 0 || t + 1 == pipe.ntiles) {
 #pragma unroll
-      for (int k = 0; k < NC; ++k)
+        for (int k = 0; k < NC; ++k)
 #pragma unroll
-        for (int r = 0; r < R; ++r) two_sum_acc(S[k][r], C[k][r], P[k][r]);
+          for (int r = 0; r < R; ++r) {
+            two_sum_acc(S[k][r], C[k][r], P[k][r]);
+            P[k][r] = T(0);
+          }
+      }
       pipe.release(t);
     }
     return true;
@@ -477,7 +492,7 @@ __global__ void __launch_bounds__(NT, MINB)
     nbody_chord(const typename Vec4<T>::type* __restrict__ tgt,
                 const typename SrcRec<T>::type* __restrict__ src, int64_t ntgt_pad,
                 int64_t nsrc_pad, const int* __restrict__ nreal, int chunk_len, T c0,
-                double* __restrict__ part, int* err) {
+                double* __restrict__ part, int* err, const F64Tables* __restrict__ tab) {
   using V4 = typename Vec4<T>::type;
   using Rec = typename SrcRec<T>::type;
   constexpr int NC = ChordAcc<T, NDIM, WU, WP>::NC;
@@ -508,7 +523,7 @@ __global__ void __launch_bounds__(NT, MINB)
 
   TilePipe<Rec, TILE> pipe{sbuf, sbar, src + s0, int(slen / TILE)};
   pipe.start();
-  if (!chord_chunk<T, NDIM, WU, WP, SKIPC, R, TILE>(pipe, tx, ty, tz, S, C, c0, err)) return;
+  if (!chord_chunk<T, NDIM, WU, WP, SKIPC, R, TILE>(pipe, tx, ty, tz, S, C, c0, err, tab)) return;
 
   double* out = part + (int64_t)blockIdx.y * NC * ntgt_pad;
 #pragma unroll
@@ -672,9 +687,9 @@ __global__ void __launch_bounds__(NT)
 // multiply-add), n / d = n r / (1 - e) = n r (1 + e + e^2) + O(e0^3), so
 // q = q0 + q0 (e + e^2), q0 = n r -- the second-order Newton-Raphson
 // (Halley-type) correction of the quotient, four FP64 operations.  Within
-// about one ulp of n / d for the finite, normal d that occur here; d = 0
-// gives NaN.
-__device__ __forceinline__ double div_nr(double n, double d) {
+// about one ulp of n / d for finite, normal d; d = 0 gives NaN.  For the arguments
+// that f64_rcp does not take.
+static __device__ __noinline__ double div_nr(double n, double d) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
   const double q0 = n * r;
@@ -687,7 +702,7 @@ __global__ void __launch_bounds__(NT)
     nbody_f64h(const double4_16a* __restrict__ tgt, const int* __restrict__ tself,
                const double4_16a* __restrict__ src, int64_t ntgt_pad,
                int64_t nsrc_pad, const int* __restrict__ nreal, int chunk_len, double eps2,
-               double* __restrict__ part, int* err) {
+               double* __restrict__ part, int* err, const F64Tables* __restrict__ tab) {
   constexpr int ND = (FORM == 2) ? 2 : 3;
   constexpr int NC = (WU ? ND : 0) + (WP ? 1 : 0);
   __shared__ __align__(128) double4_16a sbuf[2 * TILE];
@@ -742,7 +757,7 @@ __global__ void __launch_bounds__(NT)
           arg = (FORM == 1) ? eps2 - dm1 : -dm1;
         }
         if (WU) {
-          const double q = div_nr(s.w, arg);
+          const double q = f64_plain(fabs(arg)) ? s.w * f64_rcp(arg) : div_nr(s.w, arg);
           const double g = skip ? 0.0 : q;
           if (FORM == 2) {
             A[0][r] = fma(-m1, g, A[0][r]);
@@ -754,7 +769,7 @@ __global__ void __launch_bounds__(NT)
           }
         }
         if (WP) {
-          const double l = fma(log(arg), s.w, A[NC - 1][r]);
+          const double l = fma(f64_ln(tab, arg), s.w, A[NC - 1][r]);
           A[NC - 1][r] = skip ? A[NC - 1][r] : l;
         }
       }

@@ -68,18 +68,9 @@ struct __align__(16) SweSrc {
   int slot, pad[3];
 };
 
-// The last kTabBlocks blocks fill the tables of f64math.cuh.
-constexpr int kTabBlocks = kF64Entries / 256;
-
 __global__ void k_swe_pack(View fx, const double* __restrict__ zeta, const double* __restrict__ sigma,
                            const double* __restrict__ area, const double* __restrict__ sfc,
-                           const int* __restrict__ src2slot, int64_t ns, SweSrc* __restrict__ src,
-                           F64Tables* __restrict__ tab) {
-  const int tb = int(gridDim.x) - kTabBlocks;
-  if (int(blockIdx.x) >= tb) {
-    f64_table_entry(tab, (int(blockIdx.x) - tb) * 256 + threadIdx.x);
-    return;
-  }
+                           const int* __restrict__ src2slot, int64_t ns, SweSrc* __restrict__ src) {
   const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (k >= ns) return;
   const int64_t j = src2slot[k];
@@ -125,10 +116,10 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
       const double d0 = x0 - y.x, d1 = x1 - y.y;
       const double rsq = fma(d1, d1, d0 * d0), R = rsq + epssq;
       double w, lg;
-      if (f64_plain(R)) {
+      if (f64_log_plain(R)) {
         w = f64_rcp(R);
         lg = f64_log(tab, R);
-      } else {  // coincident points, out-of-range values
+      } else {  // coincident points, out-of-range values, R beside 1
         w = 1.0 / R;
         lg = log(R);
       }
@@ -473,7 +464,7 @@ __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
       // is the reference's
       const double s = da(da(dm(x[0], y.x), dm(x[1], y.y)), dm(x[2], y.z));
       const double om = ds(1.0, s), D = da(om, epssq);
-      const double rd = f64_plain(fabs(D)) ? f64_rcp(D) : 1.0 / D;
+      const double rd = f64_inv(D);
       const double d[3] = {x[0] - y.x, x[1] - y.y, x[2] - y.z};
       const double sz = y.rot * rd, ss = y.pot * rd;
       const double R = sz * rd, Q = ss * rd;
@@ -832,7 +823,7 @@ SwePlan swe_plan(lpm_context& ctx, const uint8_t* mask, int64_t nt, int64_t nf, 
       std::max<int64_t>(1, std::min<int64_t>(want, (nf + tile - 1) / tile));
   ctx.arena.reserve(sizeof(int) * (3 * size_t(nf) + 2 * size_t(nf) / 1024 + 8) +
                     rec_bytes * size_t(nf) + sizeof(double) * ncomp * size_t(nch_max) * p.tpad +
-                    sizeof(F64Tables) + 8 * 4096);
+                    8 * 4096);
   int* slot2src = static_cast<int*>(ctx.arena.take(sizeof(int) * std::max<int64_t>(nf, 1)));
   p.src2slot = static_cast<int*>(ctx.arena.take(sizeof(int) * std::max<int64_t>(nf, 1)));
   p.ns = compact_sources(ctx, mask, nf, slot2src, p.src2slot);
@@ -951,17 +942,18 @@ void swe_plane_sums(lpm_context& ctx, View tx, const double* ts, int64_t nt, Vie
   }
   const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(SweSrc), kSweNC, false, kSweTile64);
   auto* src = static_cast<SweSrc*>(p.src);
-  auto* tab = static_cast<F64Tables*>(ctx.arena.take(sizeof(F64Tables)));
-  k_swe_pack<<<blocks256(p.ns) + kTabBlocks, 256, 0, ctx.stream>>>(fx, zeta, sigma, area, sfc, p.src2slot,
-                                                          p.ns, src, tab);
-  ctx.launches++;
+  if (p.ns > 0) {
+    k_swe_pack<<<blocks256(p.ns), 256, 0, ctx.stream>>>(fx, zeta, sigma, area, sfc, p.src2slot, p.ns,
+                                                        src);
+    ctx.launches++;
+  }
   const double epssq = eps * eps, ipse2 = 1.0 / (pse_eps * pse_eps);
   if (collocated)
     k_swe_plane<true><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, ts, nt, src, p.ns, p.chunk_len, epssq,
-                                                           ipse2, tab, p.part, p.tpad);
+                                                           ipse2, ctx.f64_tab, p.part, p.tpad);
   else
     k_swe_plane<false><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, ts, nt, src, p.ns, p.chunk_len,
-                                                            epssq, ipse2, tab, p.part, p.tpad);
+                                                            epssq, ipse2, ctx.f64_tab, p.part, p.tpad);
   const unsigned th = unsigned(sum_threads(nt));
   k_swe_out<<<unsigned((nt + th - 1) / th), th, 0, ctx.stream>>>(p.part, p.nchunks, p.tpad, nt, epssq,
                                                                 pse_eps, out);
