@@ -689,13 +689,15 @@ __global__ void __launch_bounds__(NT)
 // (Halley-type) correction of the quotient, four FP64 operations.  Within
 // about one ulp of n / d for finite, normal d; d = 0 gives NaN.  For the arguments
 // that f64_rcp does not take.
-static __device__ __noinline__ double div_nr(double n, double d) {
+__device__ __forceinline__ double div_nr(double n, double d) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
   const double q0 = n * r;
   const double e = fma(-d, r, 1.0);
   return fma(q0, fma(e, e, e), q0);
 }
+// (out of line, as f64_inv_any)
+static __device__ __noinline__ double div_nr_any(double n, double d) { return div_nr(n, d); }
 
 template <int FORM, bool WU, bool WP, int R, int NT, int TILE>
 __global__ void __launch_bounds__(NT)
@@ -757,7 +759,7 @@ __global__ void __launch_bounds__(NT)
           arg = (FORM == 1) ? eps2 - dm1 : -dm1;
         }
         if (WU) {
-          const double q = f64_plain(fabs(arg)) ? s.w * f64_rcp(arg) : div_nr(s.w, arg);
+          const double q = f64_plain(fabs(arg)) ? s.w * f64_rcp(arg) : div_nr_any(s.w, arg);
           const double g = skip ? 0.0 : q;
           if (FORM == 2) {
             A[0][r] = fma(-m1, g, A[0][r]);
@@ -895,8 +897,12 @@ constexpr int F64_NT = 128, F64_R = 2, F64_TILE = 256;
 // thousand targets and sources still give every SM work (a warp's FP64
 // instruction takes 64 clocks of its SM sub-partition).
 constexpr int FINE_NT = 64, FINE_TILE = 8;
-// nbody_split: targets per CTA, sources per tile
-constexpr int SPLIT_NT = 128, SPLIT_TILE = 128;
+// nbody_split: targets per CTA, sources per tile.  128 targets with the stream
+// function (a CTA copies the log tables), 64 without: icosahedral level 4's 7,682
+// targets leave 4,840 CTAs, four waves, where 128 leave 2,440, four waves and eight
+// CTAs (RK4 step 776 -> 740 us; with stream function 64 cost 1.4 %).
+__host__ __device__ constexpr int split_nt(bool wp) { return wp ? 128 : 64; }
+constexpr int SPLIT_TILE = 128;
 
 // FP32 kernel shapes: threads, targets per thread, minimum resident CTAs per
 // SM (a register cap through __launch_bounds__).

@@ -163,13 +163,13 @@ struct SplitBufs {
 template <bool WU, bool WP>
 void launch(lpm_context& ctx, const NbodyPlan& p, const SplitBufs& b, const double4_16a* tgt,
             const int* tself, const double4_16a* src, double* part, double eps) {
-  dim3 grid(unsigned(p.ntgt_pad / kSplitNT), unsigned(p.nchunks));
+  dim3 grid(unsigned(p.ntgt_pad / split_nt(WP)), unsigned(p.nchunks));
   if (p.skipc)
-    nbody_split<WU, WP, true><<<grid, kSplitNT, 0, ctx.stream>>>(
+    nbody_split<WU, WP, true><<<grid, split_nt(WP), 0, ctx.stream>>>(
         tgt, tself, b.st, b.sp, src, b.scale, p.ntgt, p.ntgt_pad, p.nsrc, p.nsrc_pad, p.chunk_len,
         eps * eps, part, ctx.d_err);
   else
-    nbody_split<WU, WP, false><<<grid, kSplitNT, 0, ctx.stream>>>(
+    nbody_split<WU, WP, false><<<grid, split_nt(WP), 0, ctx.stream>>>(
         tgt, tself, b.st, b.sp, src, b.scale, p.ntgt, p.ntgt_pad, p.nsrc, p.nsrc_pad, p.chunk_len,
         eps * eps, part, ctx.d_err);
   ctx.launches++;
@@ -201,11 +201,11 @@ void launch_split(lpm_context& ctx, const NbodyPlan& p, const void* tgt_, const 
   b.scale = reinterpret_cast<SplitScale*>(w);
   b.range = reinterpret_cast<int4*>(w + 256);
   b.st = reinterpret_cast<SplitTarget*>(w + 256 + range_bytes(ctx));
-  b.sp = reinterpret_cast<SplitPair*>(b.st + p.ntgt_pad);  // ntgt_pad is a multiple of 128
+  b.sp = reinterpret_cast<SplitPair*>(b.st + p.ntgt_pad);  // ntgt_pad is a multiple of 64
   const int nb = range_blocks(ctx, p);
   k_split_range<<<nb, kRangeThreads, 0, ctx.stream>>>(tgt, p.ntgt, src, p.nsrc, b.range, b.scale);
   const int64_t npairs = p.nsrc_pad / 2;
-  k_split_pack<<<unsigned((npairs + 127) / 128 + p.ntgt_pad / 128), 128, 0, ctx.stream>>>(
+  k_split_pack<<<unsigned((npairs + 127) / 128 + (p.ntgt_pad + 127) / 128), 128, 0, ctx.stream>>>(
       src, p.nsrc, npairs, tgt, p.ntgt, p.ntgt_pad, eps, b.range, nb, b.sp, b.st, b.scale);
   ctx.launches += 2;
   if (p.wu && p.wp)

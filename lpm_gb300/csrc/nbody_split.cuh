@@ -63,7 +63,6 @@ struct __align__(16) SplitPair {
 };
 static_assert(sizeof(SplitPair) == 112, "seven 16-byte loads per pair of sources");
 
-constexpr int kSplitNT = SPLIT_NT;          // targets per CTA, one per thread
 constexpr int kSplitTile = SPLIT_TILE / 2;  // pairs of sources per tile
 constexpr float kSplitTiny = 9.094947e-13f;  // 2^-40: a pair's least scaled arg'
 
@@ -253,7 +252,7 @@ __device__ __noinline__ void split_near64(const double4_16a* t, const double4_16
 //   sp: SplitPair per two sources (nsrc_pad / 2 entries)
 //   SKIP: the pair of tself is left out
 template <bool WU, bool WP, bool SKIP>
-__global__ void __launch_bounds__(kSplitNT, 4)
+__global__ void __launch_bounds__(split_nt(WP), 512 / split_nt(WP))
     nbody_split(const double4_16a* __restrict__ tgt, const int* __restrict__ tself,
                 const SplitTarget* __restrict__ st, const SplitPair* __restrict__ sp,
                 const double4_16a* __restrict__ src, const SplitScale* __restrict__ scale, int64_t ntgt, int64_t ntgt_pad,
@@ -265,7 +264,7 @@ __global__ void __launch_bounds__(kSplitNT, 4)
   using Log = typename std::conditional<WP, SplitLog, float4>::type;
   __shared__ __align__(16) Log slog;
 
-  const int64_t ti = (int64_t)blockIdx.x * kSplitNT + threadIdx.x;
+  const int64_t ti = (int64_t)blockIdx.x * split_nt(WP) + threadIdx.x;
   const int64_t s0 = (int64_t)blockIdx.y * chunk_len;
   int64_t slen = nsrc_pad - s0;
   if (slen > chunk_len) slen = chunk_len;
@@ -291,8 +290,10 @@ __global__ void __launch_bounds__(kSplitNT, 4)
   const float off = ti < ntgt ? -float(pow2d(-2 * sc.e) / 1024) : -1e30f;
   const u64 one = dup2(1.f);
 
-  // (a CTA whose targets all do still drains its tiles, without the sums)
-  const bool idle = __syncthreads_and(exact || ti >= ntgt);
+  // (a warp whose targets all do, or are padding, still passes its tiles, without
+  // the sums)
+  const bool idle = __all_sync(0xffffffffu, exact || ti >= ntgt);
+  __syncthreads();  // the tables
   for (int tl = 0; tl < pipe.ntiles; ++tl) {
     if (!pipe.acquire(tl)) {
       pipe.drain(tl, err);
