@@ -60,7 +60,7 @@ constexpr int kSweTile64 = 64;
 // integers (f64math.cuh), against about 260 for the reference's operation order
 // with its eight divisions, square root and library log and exp.  Quad level 5,
 // vertices and faces: 19.6 ms in that order, 4.73 ms with 55 operations (Newton
-// steps and series in FP64), 2.89 ms now (0.9 of the pipe's measured rate).
+// steps and series in FP64), 2.64 ms now (0.95 of the pipe's measured rate).
 constexpr int kSweNC = 11;
 
 struct __align__(16) SweSrc {
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
                                                       double ipse2, const F64Tables* __restrict__ tab,
                                                       double* __restrict__ part, int64_t tpad) {
   __shared__ SweSrc tile[kSweTile64];
-  const int64_t i = blockIdx.x * int64_t(kSweNT) + threadIdx.x;
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   const int64_t c = blockIdx.y;
   const int64_t j0 = c * chunk_len, j1 = ns < j0 + chunk_len ? ns : j0 + chunk_len;
   const bool valid = i < nt;
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
   for (int64_t t0 = j0; t0 < j1; t0 += kSweTile64) {
     const int m = int(j1 - t0 < kSweTile64 ? j1 - t0 : kSweTile64);
     __syncthreads();
-    for (int q = threadIdx.x; q < m * int(sizeof(SweSrc) / 16); q += kSweNT)
+    for (int q = threadIdx.x; q < m * int(sizeof(SweSrc) / 16); q += blockDim.x)
       reinterpret_cast<double2*>(tile)[q] = reinterpret_cast<const double2*>(src + t0)[q];
     __syncthreads();
     if (!valid) continue;
@@ -176,12 +176,12 @@ __device__ __forceinline__ void swe_write(const SweOut& o, int64_t i, double u, 
   o.phi[i] = phi;
 }
 
-__global__ void k_swe_out(const double* __restrict__ part, int nchunks, int64_t tpad, int64_t nt,
-                          double epssq, double pse_eps, SweOut o) {
+__global__ void k_swe_out(const double* __restrict__ part, int64_t tpad, int64_t nt, double epssq, double pse_eps, SweOut o) {
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= nt) return;
   double s[kSweNC];
-  sum_chunks<kSweNC>(part + i, nchunks, tpad, s);
+#pragma unroll
+  for (int k = 0; k < kSweNC; ++k) s[k] = part[k * tpad + i];
   const double i2pi = 0.5 / kPI, i4pi = 0.25 / kPI;
   const double ea = epssq * s[4], eb = epssq * s[7], a2 = 2.0 * s[3], b2 = 2.0 * s[6];
   swe_write(o, i, s[0] * i2pi, s[1] * i2pi, (a2 + s[5] + eb) * i2pi, (s[2] - ea - b2) * i2pi,
@@ -359,16 +359,12 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane32(View tx, const double* _
   for (int k = 0; k < kPl32NC; ++k) part[(c * kPl32NC + k) * tpad + i] = double(S[k]) + double(C[k]);
 }
 
-__global__ void k_swe_plane32_out(const double* __restrict__ part, int nchunks, int64_t tpad,
-                                  int64_t nt, double pse_eps, SweOut o) {
+__global__ void k_swe_plane32_out(const double* __restrict__ part, int64_t tpad, int64_t nt, double pse_eps, SweOut o) {
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= nt) return;
   double w[kPl32NC];
 #pragma unroll
-  for (int k = 0; k < kPl32NC; ++k) w[k] = 0.0;
-  for (int c = 0; c < nchunks; ++c)
-#pragma unroll
-    for (int k = 0; k < kPl32NC; ++k) w[k] += part[(int64_t(c) * kPl32NC + k) * tpad + i];
+  for (int k = 0; k < kPl32NC; ++k) w[k] = part[k * tpad + i];
   const double ipi = 1.0 / kPI, i2pi = 0.5 / kPI;
   const double k = -0.6931471805599453 / (4 * kPI);
   swe_write(o, i, (w[2] - w[1]) * i2pi, (w[0] + w[3]) * i2pi, (w[7] - w[9]) * ipi + w[5] * i2pi,
@@ -402,10 +398,10 @@ __global__ void k_swe_plane32_out(const double* __restrict__ part, int nchunks, 
 // ~1e-16 / D relative), everything after it contracted, one reciprocal of D per
 // pair in integers (f64math.cuh).  The FP64 pipe bounds the kernel: 48 operations
 // per pair (66 in the form that added c v^T, v w^T, u term by term): icosahedral
-// level 5, vertices and faces, 96.5 -> 68.9 ms (81.8 ms with the reciprocal by the
+// level 5, vertices and faces, 96.5 -> 68.6 ms (81.8 ms with the reciprocal by the
 // hardware's FP64 approximation and three operations, which costs eight);
-// level 2, where 64-source chunks instead of 256-source ones fill the SMs,
-// 1.31 -> 0.34 ms.
+// level 2, where chunks of 8 to 64 sources instead of 256 fill the SMs, 1.31 ->
+// 0.14 ms.
 constexpr int kSphNC = 28;  // A3 B3 U1[3] V1[3] U2[6] V2[6] Z G H K
 
 struct __align__(16) SphSrc {
@@ -439,7 +435,7 @@ __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
                                                        int64_t chunk_len, double epssq,
                                                        double* __restrict__ part, int64_t tpad) {
   __shared__ SphSrc tile[kSweTile64];
-  const int64_t i = blockIdx.x * int64_t(kSweNT) + threadIdx.x;
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   const int64_t c = blockIdx.y;
   const int64_t j0 = c * chunk_len, j1 = ns < j0 + chunk_len ? ns : j0 + chunk_len;
   const bool valid = i < nt;
@@ -452,7 +448,7 @@ __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
   for (int64_t t0 = j0; t0 < j1; t0 += kSweTile64) {
     const int m = int(j1 - t0 < kSweTile64 ? j1 - t0 : kSweTile64);
     __syncthreads();
-    for (int q = threadIdx.x; q < m * int(sizeof(SphSrc) / 16); q += kSweNT)
+    for (int q = threadIdx.x; q < m * int(sizeof(SphSrc) / 16); q += blockDim.x)
       reinterpret_cast<double2*>(tile)[q] = reinterpret_cast<const double2*>(src + t0)[q];
     __syncthreads();
     if (!valid) continue;
@@ -496,18 +492,13 @@ __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
   for (int k = 0; k < kSphNC; ++k) part[(c * kSphNC + k) * tpad + i] = r[k];
 }
 
-__global__ void k_swe_sphere_out(const double* __restrict__ part, int nchunks, int64_t tpad,
-                                 View tx, int64_t nt, double eps2, View u, double* __restrict__ ddot,
+__global__ void k_swe_sphere_out(const double* __restrict__ part, int64_t tpad, View tx, int64_t nt, double eps2, View u, double* __restrict__ ddot,
                                  double* __restrict__ grad, int do_velocity) {
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= nt) return;
   double s[kSphNC];
 #pragma unroll
-  for (int k = 0; k < kSphNC; ++k) s[k] = 0.0;
-#pragma unroll 2
-  for (int c = 0; c < nchunks; ++c)
-#pragma unroll
-    for (int k = 0; k < kSphNC; ++k) s[k] += part[(int64_t(c) * kSphNC + k) * tpad + i];
+  for (int k = 0; k < kSphNC; ++k) s[k] = part[k * tpad + i];
   const double x[3] = {tx(i, 0), tx(i, 1), tx(i, 2)};
   const double *A = s, *B = s + 3, *U1 = s + 6, *V1 = s + 9, *U2 = s + 12, *V2 = s + 18;
   const double Z = s[24], G = s[25], H = s[26];
@@ -729,18 +720,14 @@ __global__ void __launch_bounds__(kSweNT, 4) k_swe_sphere32(View tx, int64_t nt,
   for (int k = 0; k < kSph32NC; ++k) part[(c * kSph32NC + k) * tpad + i] = acc[k][tid];
 }
 
-__global__ void k_swe_sphere32_out(const double* __restrict__ part, int nchunks, int64_t tpad,
-                                   View tx, int64_t nt, double eps2, View u,
+__global__ void k_swe_sphere32_out(const double* __restrict__ part, int64_t tpad, View tx, int64_t nt, double eps2, View u,
                                    double* __restrict__ ddot, double* __restrict__ grad,
                                    int do_velocity) {
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= nt) return;
   double s[kSph32NC];
 #pragma unroll
-  for (int k = 0; k < kSph32NC; ++k) s[k] = 0.0;
-  for (int c = 0; c < nchunks; ++c)
-#pragma unroll
-    for (int k = 0; k < kSph32NC; ++k) s[k] += part[(int64_t(c) * kSph32NC + k) * tpad + i];
+  for (int k = 0; k < kSph32NC; ++k) s[k] = part[k * tpad + i];
   // the kernel's sz, ss were doubled (strengths stored as rot, pot / pi):
   // halve A, B, Z, G, H (exact)
   for (int k : {0, 1, 2, 3, 4, 5, 24, 25, 26}) s[k] *= 0.5;
@@ -798,13 +785,25 @@ __global__ void k_swe_sphere32_out(const double* __restrict__ part, int nchunks,
     for (int k = 0; k < 9; ++k) grad[9 * i + k] = M[k];
 }
 
+// The chunks' partials added in place (into the first chunk's), a thread per
+// component and target: a thread per target reads 11 to 28 of them one chunk after
+// the other, which on small grids took longer than the pair sums (and 0.25 of 2.9 ms
+// at quad level 5).
+__global__ void k_swe_sum(double* __restrict__ part, int nchunks, int64_t n) {
+  const int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (q >= n) return;
+  double s[1];
+  sum_chunks<1>(part + q, nchunks, n, s);
+  part[q] = s[0];
+}
+
 // Scratch and chunking shared by the four SWE paths: 128 targets per CTA,
 // sources compacted (masked slots dropped) and split into chunks of whole
 // tiles, about eight waves of CTAs; ncomp FP64 partials per (chunk, target),
 // added in fixed order by the epilogue.
 struct SwePlan {
   int64_t nb = 0, tpad = 0, ns = 0, chunk_len = 0;
-  int nchunks = 1;
+  int nchunks = 1, threads = kSweNT;
   int* src2slot = nullptr;
   void* src = nullptr;     // ns packed source records
   int* slot = nullptr;     // ns slot indices (when asked for)
@@ -816,8 +815,16 @@ SwePlan swe_plan(lpm_context& ctx, const uint8_t* mask, int64_t nt, int64_t nf, 
                  int ncomp, bool want_slot, int tile) {
   SwePlan p;
   ctx.arena.reset();
-  p.nb = (nt + kSweNT - 1) / kSweNT;
-  p.tpad = p.nb * kSweNT;
+  if (tile == kSweTile64) {
+    // FP64: one warp's pair takes the FP64 pipe of its sub-partition 2,000 to 3,000
+    // clocks, so few points are cut into chunks of down to 8 sources until every
+    // sub-partition has two warps (quad level 2, vertices and faces, with the chunks'
+    // sums by k_swe_sum: 306 -> 134 us); CTAs no larger than the targets.
+    p.threads = int(std::min<int64_t>(kSweNT, (nt + 31) / 32 * 32));
+    while (tile > 8 && (nt + 31) / 32 * ((nf + tile - 1) / tile) < int64_t(ctx.num_sms) * 8) tile /= 2;
+  }
+  p.nb = (nt + p.threads - 1) / p.threads;
+  p.tpad = p.nb * p.threads;
   const int64_t want = std::max<int64_t>(1, (int64_t(ctx.num_sms) * 4 * 8 + p.nb - 1) / p.nb);
   const int64_t nch_max =
       std::max<int64_t>(1, std::min<int64_t>(want, (nf + tile - 1) / tile));
@@ -838,6 +845,13 @@ SwePlan swe_plan(lpm_context& ctx, const uint8_t* mask, int64_t nt, int64_t nf, 
 }
 
 unsigned blocks256(int64_t n) { return unsigned((n + 255) / 256); }
+
+void swe_sum(lpm_context& ctx, const SwePlan& p, int ncomp) {
+  if (p.nchunks == 1) return;
+  const int64_t n = ncomp * p.tpad;
+  k_swe_sum<<<blocks256(n), 256, 0, ctx.stream>>>(p.part, p.nchunks, n);
+  ctx.launches++;
+}
 
 void swe_sphere_sums32(lpm_context& ctx, View tx, int64_t nt, View fx, const double* zeta,
                        const double* sigma, const double* area, const uint8_t* mask, int64_t nf,
@@ -860,7 +874,8 @@ void swe_sphere_sums32(lpm_context& ctx, View tx, int64_t nt, View fx, const dou
   else
     k_swe_sphere32<false><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, nt, src, pslot, p.ns,
                                                                p.chunk_len, c0, p.part, p.tpad);
-  k_swe_sphere32_out<<<blocks256(nt), 256, 0, ctx.stream>>>(p.part, p.nchunks, p.tpad, tx, nt,
+  swe_sum(ctx, p, kSph32NC);
+  k_swe_sphere32_out<<<blocks256(nt), 256, 0, ctx.stream>>>(p.part, p.tpad, tx, nt,
                                                             eps * eps, u, ddot, grad, do_velocity);
   ctx.launches += 2;
   LPM_CUDA(cudaGetLastError());
@@ -886,14 +901,15 @@ void swe_sphere_sums(lpm_context& ctx, View tx, int64_t nt, View fx, const doubl
     ctx.launches++;
   }
   if (collocated)
-    k_swe_sphere<true><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, nt, src, p.ns, p.chunk_len,
+    k_swe_sphere<true><<<p.grid(), p.threads, 0, ctx.stream>>>(tx, nt, src, p.ns, p.chunk_len,
                                                             eps * eps, p.part, p.tpad);
   else
-    k_swe_sphere<false><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, nt, src, p.ns, p.chunk_len,
+    k_swe_sphere<false><<<p.grid(), p.threads, 0, ctx.stream>>>(tx, nt, src, p.ns, p.chunk_len,
                                                              eps * eps, p.part, p.tpad);
+  swe_sum(ctx, p, kSphNC);
   const unsigned th = unsigned(sum_threads(nt));
   k_swe_sphere_out<<<unsigned((nt + th - 1) / th), th, 0, ctx.stream>>>(
-      p.part, p.nchunks, p.tpad, tx, nt, eps * eps, u, ddot, grad, do_velocity);
+      p.part, p.tpad, tx, nt, eps * eps, u, ddot, grad, do_velocity);
   ctx.launches += 2;
   LPM_CUDA(cudaGetLastError());
 }
@@ -924,7 +940,8 @@ void swe_plane_sums32(lpm_context& ctx, View tx, const double* ts, int64_t nt, V
   else
     k_swe_plane32<false><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, ts, nt, src, p.ns, p.chunk_len,
                                                               e2, ipse2, p.part, p.tpad);
-  k_swe_plane32_out<<<blocks256(nt), 256, 0, ctx.stream>>>(p.part, p.nchunks, p.tpad, nt, pse_eps,
+  swe_sum(ctx, p, kPl32NC);
+  k_swe_plane32_out<<<blocks256(nt), 256, 0, ctx.stream>>>(p.part, p.tpad, nt, pse_eps,
                                                            out);
   ctx.launches += 2;
   LPM_CUDA(cudaGetLastError());
@@ -949,13 +966,14 @@ void swe_plane_sums(lpm_context& ctx, View tx, const double* ts, int64_t nt, Vie
   }
   const double epssq = eps * eps, ipse2 = 1.0 / (pse_eps * pse_eps);
   if (collocated)
-    k_swe_plane<true><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, ts, nt, src, p.ns, p.chunk_len, epssq,
+    k_swe_plane<true><<<p.grid(), p.threads, 0, ctx.stream>>>(tx, ts, nt, src, p.ns, p.chunk_len, epssq,
                                                            ipse2, ctx.f64_tab, p.part, p.tpad);
   else
-    k_swe_plane<false><<<p.grid(), kSweNT, 0, ctx.stream>>>(tx, ts, nt, src, p.ns, p.chunk_len,
+    k_swe_plane<false><<<p.grid(), p.threads, 0, ctx.stream>>>(tx, ts, nt, src, p.ns, p.chunk_len,
                                                             epssq, ipse2, ctx.f64_tab, p.part, p.tpad);
+  swe_sum(ctx, p, kSweNC);
   const unsigned th = unsigned(sum_threads(nt));
-  k_swe_out<<<unsigned((nt + th - 1) / th), th, 0, ctx.stream>>>(p.part, p.nchunks, p.tpad, nt, epssq,
+  k_swe_out<<<unsigned((nt + th - 1) / th), th, 0, ctx.stream>>>(p.part, p.tpad, nt, epssq,
                                                                 pse_eps, out);
   ctx.launches += 2;
   LPM_CUDA(cudaGetLastError());

@@ -96,18 +96,26 @@ def sphere_tangency(ctx, udotx, x, u):
 _SWE_KEYS = ("ddot", "du1dx1", "du1dx2", "du2dx1", "du2dx2", "laps", "psi", "phi")
 
 
-def _swe_outputs(n, like):
+def _swe_velocity(n, nd, like, do_velocity):
+    """Written by the call if do_velocity (no fill launch then), zeros otherwise."""
     import torch
 
-    out = {k: torch.zeros(n, dtype=torch.float64, device=like.device) for k in _SWE_KEYS}
-    out["u"] = torch.zeros(n, 2, dtype=torch.float64, device=like.device)
+    make = torch.empty if do_velocity else torch.zeros
+    return make(n, nd, dtype=torch.float64, device=like.device)
+
+
+def _swe_outputs(n, like, do_velocity):
+    import torch
+
+    out = {k: torch.empty(n, dtype=torch.float64, device=like.device) for k in _SWE_KEYS}
+    out["u"] = _swe_velocity(n, 2, like, do_velocity)
     return out
 
 
 def swe_plane_vertex_sums(ctx, vx, vs, fx, fzeta, fsigma, farea, fmask, fs, eps, pse_eps,
                           do_velocity=True):
     """PlanarSWEVertexSums (src/lpm_swe_kernels.hpp:626-721): dict of outputs."""
-    o = _swe_outputs(_n(vx), vx)
+    o = _swe_outputs(_n(vx), vx, do_velocity)
     check(lib().lpm_swe_plane_vertex_sums(
         ctx.handle, view(o["u"]), *(ptr(o[k]) for k in _SWE_KEYS), view(vx), ptr(vs), _n(vx),
         view(fx), ptr(fzeta), ptr(fsigma), ptr(farea), ptr(fmask), ptr(fs), _n(fx), eps, pse_eps,
@@ -117,20 +125,20 @@ def swe_plane_vertex_sums(ctx, vx, vs, fx, fzeta, fsigma, farea, fmask, fs, eps,
 
 def swe_plane_face_sums(ctx, fx, fzeta, fsigma, farea, fmask, fs, eps, pse_eps, do_velocity=True):
     """PlanarSWEFaceSums (src/lpm_swe_kernels.hpp:787-876): dict of outputs."""
-    o = _swe_outputs(_n(fx), fx)
+    o = _swe_outputs(_n(fx), fx, do_velocity)
     check(lib().lpm_swe_plane_face_sums(
         ctx.handle, view(o["u"]), *(ptr(o[k]) for k in _SWE_KEYS), view(fx), ptr(fzeta),
         ptr(fsigma), ptr(farea), ptr(fmask), ptr(fs), _n(fx), eps, pse_eps, int(do_velocity)))
     return o
 
 
-def _sphere_swe_outputs(n, like, want_grad):
+def _sphere_swe_outputs(n, like, want_grad, do_velocity):
     import torch
 
-    out = {"u": torch.zeros(n, 3, dtype=torch.float64, device=like.device),
-           "ddot": torch.zeros(n, dtype=torch.float64, device=like.device)}
+    out = {"u": _swe_velocity(n, 3, like, do_velocity),
+           "ddot": torch.empty(n, dtype=torch.float64, device=like.device)}
     if want_grad:
-        out["grad"] = torch.zeros(n, 9, dtype=torch.float64, device=like.device)
+        out["grad"] = torch.empty(n, 9, dtype=torch.float64, device=like.device)
     return out
 
 
@@ -140,7 +148,7 @@ def swe_sphere_vertex_sums(ctx, vx, fx, fzeta, fsigma, farea, fmask, eps, do_vel
     ddot (n) and, if want_grad, the summed gradient tensor (n x 9, row-major).
     `out` reuses a dict from an earlier call (u keeps its values when
     do_velocity is false)."""
-    o = out if out is not None else _sphere_swe_outputs(_n(vx), vx, want_grad)
+    o = out if out is not None else _sphere_swe_outputs(_n(vx), vx, want_grad, do_velocity)
     check(lib().lpm_swe_sphere_vertex_sums(
         ctx.handle, view(o["u"]), ptr(o["ddot"]), ptr(o.get("grad")), view(vx), _n(vx), view(fx),
         ptr(fzeta), ptr(fsigma), ptr(farea), ptr(fmask), _n(fx), eps, int(do_velocity)))
@@ -151,7 +159,7 @@ def swe_sphere_face_sums(ctx, fx, fzeta, fsigma, farea, fmask, eps, do_velocity=
                          want_grad=False, out=None):
     """SphereFaceSums (src/lpm_swe_kernels.hpp:877-940): as swe_sphere_vertex_sums
     at every face slot (i == j skipped for |eps| < DBL_EPSILON)."""
-    o = out if out is not None else _sphere_swe_outputs(_n(fx), fx, want_grad)
+    o = out if out is not None else _sphere_swe_outputs(_n(fx), fx, want_grad, do_velocity)
     check(lib().lpm_swe_sphere_face_sums(
         ctx.handle, view(o["u"]), ptr(o["ddot"]), ptr(o.get("grad")), view(fx), ptr(fzeta),
         ptr(fsigma), ptr(farea), ptr(fmask), _n(fx), eps, int(do_velocity)))
