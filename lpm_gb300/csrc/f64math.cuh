@@ -10,10 +10,11 @@
 // 2^-12 (table), r = m f - 1 exactly (integers modulo 2^64), log x = (k ln 2 - log f)
 // + log1p(r), the series to r^5 / 5 in fixed point of 74 bits: 2 FP64 additions.
 // exp(-p): p = n ln 2 / 8192 + r in fixed point of 76 bits, 2^(-n/8192) from a table of
-// 63 bits, exp(-r) by its series to the cube: no FP64 operation.
+// 63 bits, exp(-r) by its series to r^4 / 24; the polynomial before it in 61 bits: no
+// FP64 operation.
 // The range reductions are those of Cody and Waite, and Tang's table-driven
-// methods.  Errors: 1/x and exp about half a unit in the last place, log two
-// roundings of its parts.  The tables (145 KB) are read through L1.
+// methods.  Errors: 1/x, its square and exp about half a unit in the last place, log
+// two roundings of its parts.  The tables (145 KB) are read through L1.
 #pragma once
 
 #include <cstdint>
@@ -68,8 +69,14 @@ __device__ __forceinline__ bool f64_plain(double x) {
 __device__ __forceinline__ uint64_t f64_mantissa(double x) {  // 2^52 m, m in [1, 2)
   return (uint64_t(__double_as_longlong(x)) & 0xfffffffffffffull) | 0x10000000000000ull;
 }
-// 1/d, |d| as f64_plain.
-__device__ __forceinline__ double f64_rcp(double d) {
+// a 2^(e - 1086) rounded to nearest, for the normalised a (bit 63 set) and the biased
+// exponent e of the result
+__device__ __forceinline__ uint64_t f64_pack(uint64_t a, int e) {
+  return (a >> 11) + (a >> 10 & 1) + (uint64_t(unsigned(e - 1)) << 52);
+}
+
+// 2^63 / m for the mantissa m of d.
+__device__ __forceinline__ uint64_t f64_rcp_mantissa(double d) {
   const unsigned h = unsigned(__double2hiint(d)), l = unsigned(__double2loint(d));
   const float mh = __int_as_float(int(__funnelshift_l(l, h & 0xfffff, 3)) | 0x3f800000);
   float y;
@@ -79,11 +86,25 @@ __device__ __forceinline__ double f64_rcp(double d) {
   const int64_t E = -int64_t(f64_mantissa(d) * Y);                         // 2^76 (1 - m y)
   const int e = int(E >> 32);                                              // 2^44 e
   const int64_t e2 = (int64_t(e) * e) >> 24;                               // 2^64 e^2
-  // 2^63 / m
-  const uint64_t W = (uint64_t(Y) << 39) + uint64_t((int64_t(Y) * (E >> 16)) >> 21) +
-                     ((uint64_t(unsigned(e2)) * Y) >> 25);
+  return (uint64_t(Y) << 39) + uint64_t((int64_t(Y) * (E >> 16)) >> 21) +
+         ((uint64_t(unsigned(e2)) * Y) >> 25);
+}
+// The reciprocal with that mantissa.
+__device__ __forceinline__ double f64_rcp_value(uint64_t W, double d) {
+  const unsigned h = unsigned(__double2hiint(d));
   const uint64_t b = ((W + 0x200) >> 10) + (uint64_t(2044 - ((h >> 20) & 0x7ff)) << 52);
   return __hiloint2double(int(unsigned(b >> 32) | (h & 0x80000000u)), int(unsigned(b)));
+}
+// 1/d, |d| as f64_plain.
+__device__ __forceinline__ double f64_rcp(double d) {
+  return f64_rcp_value(f64_rcp_mantissa(d), d);
+}
+// Its square, |d| in [2^-500, 2^500).
+__device__ __forceinline__ double f64_rcp_square(uint64_t W, double d) {
+  const uint64_t H = __umul64hi(W, W);  // 2^62 / m^2
+  const int z = __clzll(int64_t(H));
+  const int E = int(unsigned(__double2hiint(d)) >> 20 & 0x7ff);
+  return __longlong_as_double(int64_t(f64_pack(H << z, 3070 - z - 2 * E)));
 }
 
 // 1/d for any d.  The rare case is a call: inlined, its FP64 operations are issued
@@ -119,11 +140,13 @@ __device__ __forceinline__ double f64_ln(const F64Tables* __restrict__ T, double
   return f64_log_plain(x) ? f64_log(T, x) : f64_ln_any(x);
 }
 
-// q exp(-p) for 0 <= p < 746 (beyond, exp(-p) is 0 in FP64); q finite.
-__device__ __forceinline__ double f64_mul_exp_neg(const F64Tables* __restrict__ T, double q,
-                                                  double p) {
+// (40 (1 - p) + 10 p^2 - 2 p^3 / 3) exp(-p) for 0 <= p < 746 (beyond, exp(-p) is 0 in
+// FP64).  The cubic by Horner's rule in f = p / 2^K < 1, K >= 3, times 2^-3K, in 61
+// bits.
+__device__ __forceinline__ double f64_pse8(const F64Tables* __restrict__ T, double p) {
   const int ep = int((unsigned(__double2hiint(p)) >> 20) & 0x7ff) - 1023;  // <= 9
-  const uint64_t P = (f64_mantissa(p) << 11) >> min(unsigned(9 - ep), 63u);  // 2^54 p
+  const uint64_t m = f64_mantissa(p) << 11;
+  const uint64_t P = m >> min(9 - ep, 63);  // 2^54 p
   const unsigned n = unsigned((uint64_t(unsigned(P >> 32)) * 12102203u) >> 32);
   const int64_t r = int64_t((P << 22) - n * 0x58b90bfbe8e7bcd6ull);  // 2^76 r, r < 2^-13.4
   const int r1 = int((r + (int64_t(1) << 31)) >> 32);                // 2^44 r
@@ -132,11 +155,21 @@ __device__ __forceinline__ double f64_mul_exp_neg(const F64Tables* __restrict__ 
   const int64_t v = ((int64_t(r1) * r1) >> 13) - r - (int64_t(c) << 6);  // 2^76 (exp(-r) - 1)
   const uint64_t t = T->ex[n & ((1 << kExpBits) - 1)];
   const uint64_t E = t + uint64_t(__mul64hi(int64_t(t >> 1), v) >> 11);  // 2^63 2^(-j/8192 - r)
-  const int z = __clzll(int64_t(E));
-  const int e = 1023 - z - int(n >> kExpBits), e1 = max(e, 23);
-  const uint64_t a = E << z;
-  const uint64_t b = (a >> 11) + (a >> 10 & 1) + (uint64_t(unsigned(e1 - 1)) << 52);
-  double w = q * __longlong_as_double(int64_t(b));
+
+  const int K = max(ep + 1, 3);
+  const int64_t f = int64_t(m >> min(K - ep, 63));  // 2^63 p / 2^K
+  constexpr int64_t k5 = int64_t(5) << 60;          // 40 in 2^61, over 2^4
+  int64_t g = (k5 >> (K - 2)) - __mul64hi(0x2aaaaaaaaaaaaaabll, f);
+  g = 2 * __mul64hi(g, f) - (k5 >> (2 * K - 4));
+  g = 2 * __mul64hi(g, f) + (k5 >> (3 * K - 4));
+
+  // 2^61 |g| 2^(-j/8192 - r); E = 2^63 less one
+  const uint64_t h = __umul64hi(uint64_t(g < 0 ? -g : g), (E - (E >> 63)) << 1);
+  const int z = __clzll(int64_t(h | 1));
+  const int e = 1023 + 2 - z + 3 * K - int(n >> kExpBits), e1 = max(e, 23);
+  const uint64_t b = f64_pack(h << z, e1);
+  double w = __hiloint2double(int(unsigned(b >> 32) | (unsigned(g >> 32) & 0x80000000u)),
+                              int(unsigned(b)));
   if (e < e1) w *= __hiloint2double((1023 + e - e1) << 20, 0);
   return w;
 }

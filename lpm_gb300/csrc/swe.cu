@@ -115,18 +115,21 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
       if (COLL && y.slot == i) continue;
       const double d0 = x0 - y.x, d1 = x1 - y.y;
       const double rsq = fma(d1, d1, d0 * d0), R = rsq + epssq;
-      double w, lg;
-      if (f64_log_plain(R)) {
-        w = f64_rcp(R);
+      double w, w2, lg;
+      if (f64_log_plain(R) && unsigned(__double2hiint(R)) - (523u << 20) < (1000u << 20)) {
+        const uint64_t W = f64_rcp_mantissa(R);
+        w = f64_rcp_value(W, R);
+        w2 = f64_rcp_square(W, R);
         lg = f64_log(tab, R);
       } else {  // coincident points, out-of-range values, R beside 1
         w = 1.0 / R;
+        w2 = w * w;
         lg = log(R);
       }
       const double e0 = d0 * w, e1 = d1 * w;
       r[0] = fma(-y.rot, e1, fma(y.pot, e0, r[0]));
       r[1] = fma(y.rot, e0, fma(y.pot, e1, r[1]));
-      const double w2 = w * w, md = fma(e1, e1, -(e0 * e0)), xy = e0 * e1;
+      const double md = fma(e1, e1, -(e0 * e0)), xy = e0 * e1;
       r[2] = fma(y.rot, md, r[2]);
       r[3] = fma(y.rot, xy, r[3]);
       r[4] = fma(y.rot, w2, r[4]);
@@ -134,13 +137,12 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
       r[6] = fma(y.pot, xy, r[6]);
       r[7] = fma(y.pot, w2, r[7]);
       const double p = rsq * ipse2;
-      double pre = fma(p, -2.0 / 3, 10.0);
-      pre = fma(p, pre, -40.0);
-      pre = fma(p, pre, 40.0);
       // p < 746 or NaN, by the high word (p >= 0)
       const unsigned hp = unsigned(__double2hiint(p));
-      if (hp < 0x40875000u || hp > 0x7ff00000u)
-        r[8] = fma((y.s - si) * y.area, f64_mul_exp_neg(tab, pre, p), r[8]);
+      if (hp < 0x40875000u)
+        r[8] = fma((y.s - si) * y.area, f64_pse8(tab, p), r[8]);
+      else if (hp > 0x7ff00000u)
+        r[8] = p;
       r[9] = fma(y.rot, lg, r[9]);
       r[10] = fma(y.pot, lg, r[10]);
     }
