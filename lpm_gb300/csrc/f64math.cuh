@@ -13,7 +13,7 @@
 // 63 bits, exp(-r) by its series to r^4 / 24; the polynomial before it in 61 bits: no
 // FP64 operation.
 // The range reductions are those of Cody and Waite, and Tang's table-driven
-// methods.  Errors: 1/x, its square and exp about half a unit in the last place, log
+// methods.  Errors: 1/x and exp about half a unit in the last place, log
 // two roundings of its parts.  The tables (145 KB) are read through L1.
 #pragma once
 
@@ -75,6 +75,13 @@ __device__ __forceinline__ uint64_t f64_pack(uint64_t a, int e) {
   return (a >> 11) + (a >> 10 & 1) + (uint64_t(unsigned(e - 1)) << 52);
 }
 
+// -1^neg mag 2^k, within the normal range.
+__device__ __forceinline__ double f64_value(uint64_t mag, bool neg, int k) {
+  const int z = __clzll(int64_t(mag | 1));
+  const uint64_t b = mag != 0 ? f64_pack(mag << z, 1086 - z + k) : 0;
+  return __hiloint2double(int(unsigned(b >> 32) | (neg ? 0x80000000u : 0u)), int(unsigned(b)));
+}
+
 // 2^63 / m for the mantissa m of d.
 __device__ __forceinline__ uint64_t f64_rcp_mantissa(double d) {
   const unsigned h = unsigned(__double2hiint(d)), l = unsigned(__double2loint(d));
@@ -99,14 +106,6 @@ __device__ __forceinline__ double f64_rcp_value(uint64_t W, double d) {
 __device__ __forceinline__ double f64_rcp(double d) {
   return f64_rcp_value(f64_rcp_mantissa(d), d);
 }
-// Its square, |d| in [2^-500, 2^500).
-__device__ __forceinline__ double f64_rcp_square(uint64_t W, double d) {
-  const uint64_t H = __umul64hi(W, W);  // 2^62 / m^2
-  const int z = __clzll(int64_t(H));
-  const int E = int(unsigned(__double2hiint(d)) >> 20 & 0x7ff);
-  return __longlong_as_double(int64_t(f64_pack(H << z, 3070 - z - 2 * E)));
-}
-
 // 1/d for any d.  The rare case is a call: inlined, its FP64 operations are issued
 // for every pair and the result selected.
 static __device__ __noinline__ double f64_inv_any(double d) { return 1.0 / d; }
@@ -140,12 +139,10 @@ __device__ __forceinline__ double f64_ln(const F64Tables* __restrict__ T, double
   return f64_log_plain(x) ? f64_log(T, x) : f64_ln_any(x);
 }
 
-// (40 (1 - p) + 10 p^2 - 2 p^3 / 3) exp(-p) for 0 <= p < 746 (beyond, exp(-p) is 0 in
-// FP64).  The cubic by Horner's rule in f = p / 2^K < 1, K >= 3, times 2^-3K, in 61
-// bits.
-__device__ __forceinline__ double f64_pse8(const F64Tables* __restrict__ T, double p) {
-  const int ep = int((unsigned(__double2hiint(p)) >> 20) & 0x7ff) - 1023;  // <= 9
-  const uint64_t m = f64_mantissa(p) << 11;
+// (40 (1 - p) + 10 p^2 - 2 p^3 / 3) exp(-p) for p = m 2^(ep - 63), m in [2^63, 2^64),
+// p < 746 (beyond, exp(-p) is 0 in FP64).  The cubic by Horner's rule in f = p / 2^K
+// < 1, K >= 3, times 2^-3K, in 61 bits.
+__device__ __forceinline__ double f64_pse8(const F64Tables* __restrict__ T, uint64_t m, int ep) {
   const uint64_t P = m >> min(9 - ep, 63);  // 2^54 p
   const unsigned n = unsigned((uint64_t(unsigned(P >> 32)) * 12102203u) >> 32);
   const int64_t r = int64_t((P << 22) - n * 0x58b90bfbe8e7bcd6ull);  // 2^76 r, r < 2^-13.4

@@ -40,27 +40,28 @@ __device__ __forceinline__ double ds(double a, double b) { return __dsub_rn(a, b
 constexpr int kSweNT = 128;   // targets per CTA
 constexpr int kSweTile = 256;  // sources per shared-memory tile (FP32)
 // FP64: small tiles and chunks, so that a few thousand points spread evenly
-// (a warp's pair takes 2,000 to 3,000 clocks of its sub-partition's FP64 pipe)
+// (a warp's pair takes 1,200 to 3,000 clocks of its sub-partition's FP64 pipe)
 constexpr int kSweTile64 = 64;
 
 // ---- planar SWE sums, FP64 --------------------------------------------------
 // With e = d / R, the eleven sums
 //   U, V    = sum -rot e1 + pot e0, sum rot e0 + pot e1
-//   A1..A3  = sum rot (e1^2 - e0^2, e0 e1, 1 / R^2),   B1..B3 the same with pot
+//   A1..A3  = sum rot (e1^2 - e0^2, e0 e1, eps^2 / R^2),   B1..B3 the same with pot
 //   L       = sum (s_y - s_x) A (40 (1 - p) + 10 p^2 - 2 p^3 / 3) e^-p,
 //             p = |d|^2 / pse_eps^2
 //   P, Q    = sum rot log R, sum pot log R
 // give every output: 2 pi u = U, 2 pi v = V,
-//   2 pi du/dx = 2 A2 + B1 + eps^2 B3,   2 pi du/dy = A1 - eps^2 A3 - 2 B2,
-//   2 pi dv/dx = A1 + eps^2 A3 - 2 B2,   2 pi dv/dy = -2 A2 - B1 + eps^2 B3,
+//   2 pi du/dx = 2 A2 + B1 + B3,   2 pi du/dy = A1 - A3 - 2 B2,
+//   2 pi dv/dx = A1 + A3 - 2 B2,   2 pi dv/dy = -2 A2 - B1 + B3,
 //   lap = L / (pi pse_eps^2), psi, phi = -P / 4 pi, -Q / 4 pi
 // (R/2 taken from e1^2 and e0^2 pair by pair, so no large sums cancel).
 // The FP64 pipe bounds the kernel, 64 clocks of a sub-partition per operation of a
-// warp: 33 operations per pair, the reciprocal, logarithm and exponential in
-// integers (f64math.cuh), against about 260 for the reference's operation order
-// with its eight divisions, square root and library log and exp.  Quad level 5,
-// vertices and faces: 19.6 ms in that order, 4.73 ms with 55 operations (Newton
-// steps and series in FP64), 2.64 ms now (0.95 of the pipe's measured rate).
+// warp: 19 operations per pair (the differences, the sums and the two additions of
+// the logarithm), everything between formed in integers beside them (swe_pair), against
+// about 260 for the reference's operation order with its eight divisions, square root
+// and library log and exp.  Quad level 5, vertices and faces: 19.6 ms in that order,
+// 4.73 ms as moments in FP64 (55 operations), 1.81 ms now (0.83 of the pipe's rate, 42 %
+// of the issue slots).
 constexpr int kSweNC = 11;
 
 struct __align__(16) SweSrc {
@@ -85,6 +86,87 @@ __global__ void k_swe_pack(View fx, const double* __restrict__ zeta, const doubl
   r.pad[0] = r.pad[1] = r.pad[2] = 0;
   src[k] = r;
 }
+// A pair's factors: e = d / R, e1^2 - e0^2, e0 e1, eps^2 / R^2 (1 / R^2 itself overflows
+// where the sums do not), log R and the smoothing kernel.
+struct SwePair {
+  double e0, e1, md, xy, ew, lg, pse;
+};
+
+// In FP64, for any values.
+__device__ __noinline__ SwePair swe_pair_any(double d0, double d1, double epssq, double ipse2) {
+  SwePair v;
+  const double rsq = fma(d1, d1, d0 * d0), R = rsq + epssq, w = 1.0 / R, p = rsq * ipse2;
+  v.e0 = d0 * w;
+  v.e1 = d1 * w;
+  v.md = fma(v.e1, v.e1, -(v.e0 * v.e0));
+  v.xy = v.e0 * v.e1;
+  v.ew = epssq * w * w;
+  v.lg = log(R);
+  v.pse = p >= 746.0 ? 0.0 : fma(p, fma(p, fma(p, -2.0 / 3, 10.0), -40.0), 40.0) * exp(-p);
+  return v;
+}
+
+// eps^2 and 1 / pse_eps^2 for swe_pair: mantissas with bit 63 set (0 for eps = 0), and
+// biased exponents; eps < 2^(ee - 1022).
+struct SweScales {
+  uint64_t e2, ip;
+  int e2x, ipx, ee;
+};
+__device__ __forceinline__ SweScales swe_scales(double epssq, double ipse2) {
+  SweScales c;
+  c.e2x = int(unsigned(__double2hiint(epssq)) >> 20);
+  c.ipx = int(unsigned(__double2hiint(ipse2)) >> 20);
+  c.e2 = c.e2x > 0 ? f64_mantissa(epssq) << 11 : 0;
+  c.ip = f64_mantissa(ipse2) << 11;
+  c.ee = (c.e2x + 1023) / 2;
+  // out of range: no pair is plain
+  if (c.e2x > 1800 || c.ipx < 223 || c.ipx > 1823) c.ee = 4096;
+  return c;
+}
+
+// In 64-bit fixed point: d over 2^(eE - 1085) for the larger exponent eE of d0, d1 and
+// eps, so that |d|^2, R = |d|^2 + eps^2 and the products keep 58 bits and more.  False
+// for values it does not take: sizes outside 2^-240 .. 2^240, d below 2^-9 eps (whose
+// last bits it would drop) but not 0, R beside 1.
+__device__ __forceinline__ bool swe_pair(const F64Tables* __restrict__ tab, double d0, double d1,
+                                         const SweScales& c, SwePair& v) {
+  const unsigned h0 = unsigned(__double2hiint(d0)), h1 = unsigned(__double2hiint(d1));
+  const int x0 = int(h0 >> 20 & 0x7ff), x1 = int(h1 >> 20 & 0x7ff), eb = max(x0, x1);
+  const int eE = max(eb, c.ee);
+  const uint64_t D0 = (f64_mantissa(d0) << 10) >> min(eE - x0, 63);
+  const uint64_t D1 = (f64_mantissa(d1) << 10) >> min(eE - x1, 63);
+  const uint64_t S = __umul64hi(D0, D0) + __umul64hi(D1, D1);  // |d|^2
+  const uint64_t Q = S + (c.e2 >> min(2 * eE - 1020 - c.e2x, 63));  // R = Q 2^(2 eE - 2106)
+  const int zq = __clzll(int64_t(Q | 1));
+  const int xr = 2 * eE - 1020 - zq;
+  const double R = __longlong_as_double(int64_t(f64_pack(Q << zq, xr)));
+  if (unsigned(eE - 783) > 480u || (eE - eb > 9 && (d0 != 0.0 || d1 != 0.0)) || Q == 0 ||
+      !f64_log_plain(R))
+    return false;
+  const uint64_t W = f64_rcp_mantissa(R);
+  const int er = int(unsigned(__double2hiint(R)) >> 20);
+  const uint64_t E0 = __umul64hi(D0, W), E1 = __umul64hi(D1, W);  // |e| 2^(61 + er - eE)
+  const bool n0 = int(h0) < 0, n1 = int(h1) < 0;
+  const int ke = eE - 61 - er;
+  v.e0 = f64_value(E0, n0, ke);
+  v.e1 = f64_value(E1, n1, ke);
+  const int64_t md = int64_t(__umul64hi(2 * E1, 2 * E1)) - int64_t(__umul64hi(2 * E0, 2 * E0));
+  v.md = f64_value(uint64_t(md < 0 ? -md : md), md < 0, 2 * ke + 62);
+  v.xy = f64_value(__umul64hi(2 * E0, 2 * E1), n0 != n1, 2 * ke + 62);
+  const int kw = c.e2x - 1086 + 2 * (1023 - er);
+  v.ew = f64_value(kw < -1000 ? 0 : __umul64hi(__umul64hi(W, W) << 2, c.e2), false, kw);
+  v.lg = f64_log(tab, R);
+  // p = |d|^2 / pse_eps^2
+  const int zs = __clzll(int64_t(S | 1));
+  const uint64_t pm = __umul64hi(S << zs, c.ip);
+  const int zp = S == 0 ? 0 : __clzll(int64_t(pm));
+  const int ep = S == 0 ? -1000 : 2 * eE - 2043 - zs + c.ipx - 1023 + 1 - zp;
+  const uint64_t m = S == 0 ? uint64_t(1) << 63 : pm << zp;
+  v.pse = 0.0;
+  if (ep < 9 || (ep == 9 && m < 0xba80000000000000ull)) v.pse = f64_pse8(tab, m, ep);  // p < 746
+  return true;
+}
+
 // COLL: collocated targets, the source in the target's own slot is skipped.
 template <bool COLL>
 __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __restrict__ ts,
@@ -99,6 +181,7 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
   const bool valid = i < nt;
   const double x0 = valid ? tx(i, 0) : 0.0, x1 = valid ? tx(i, 1) : 0.0;
   const double si = valid ? ts[i] : 0.0;
+  const SweScales sc = swe_scales(epssq, ipse2);
   double r[kSweNC];
 #pragma unroll
   for (int k = 0; k < kSweNC; ++k) r[k] = 0.0;
@@ -114,37 +197,19 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
       const SweSrc& y = tile[q];
       if (COLL && y.slot == i) continue;
       const double d0 = x0 - y.x, d1 = x1 - y.y;
-      const double rsq = fma(d1, d1, d0 * d0), R = rsq + epssq;
-      double w, w2, lg;
-      if (f64_log_plain(R) && unsigned(__double2hiint(R)) - (523u << 20) < (1000u << 20)) {
-        const uint64_t W = f64_rcp_mantissa(R);
-        w = f64_rcp_value(W, R);
-        w2 = f64_rcp_square(W, R);
-        lg = f64_log(tab, R);
-      } else {  // coincident points, out-of-range values, R beside 1
-        w = 1.0 / R;
-        w2 = w * w;
-        lg = log(R);
-      }
-      const double e0 = d0 * w, e1 = d1 * w;
-      r[0] = fma(-y.rot, e1, fma(y.pot, e0, r[0]));
-      r[1] = fma(y.rot, e0, fma(y.pot, e1, r[1]));
-      const double md = fma(e1, e1, -(e0 * e0)), xy = e0 * e1;
-      r[2] = fma(y.rot, md, r[2]);
-      r[3] = fma(y.rot, xy, r[3]);
-      r[4] = fma(y.rot, w2, r[4]);
-      r[5] = fma(y.pot, md, r[5]);
-      r[6] = fma(y.pot, xy, r[6]);
-      r[7] = fma(y.pot, w2, r[7]);
-      const double p = rsq * ipse2;
-      // p < 746 or NaN, by the high word (p >= 0)
-      const unsigned hp = unsigned(__double2hiint(p));
-      if (hp < 0x40875000u)
-        r[8] = fma((y.s - si) * y.area, f64_pse8(tab, p), r[8]);
-      else if (hp > 0x7ff00000u)
-        r[8] = p;
-      r[9] = fma(y.rot, lg, r[9]);
-      r[10] = fma(y.pot, lg, r[10]);
+      SwePair v;
+      if (!swe_pair(tab, d0, d1, sc, v)) v = swe_pair_any(d0, d1, epssq, ipse2);
+      r[0] = fma(-y.rot, v.e1, fma(y.pot, v.e0, r[0]));
+      r[1] = fma(y.rot, v.e0, fma(y.pot, v.e1, r[1]));
+      r[2] = fma(y.rot, v.md, r[2]);
+      r[3] = fma(y.rot, v.xy, r[3]);
+      r[4] = fma(y.rot, v.ew, r[4]);
+      r[5] = fma(y.pot, v.md, r[5]);
+      r[6] = fma(y.pot, v.xy, r[6]);
+      r[7] = fma(y.pot, v.ew, r[7]);
+      if (v.pse != 0.0) r[8] = fma((y.s - si) * y.area, v.pse, r[8]);
+      r[9] = fma(y.rot, v.lg, r[9]);
+      r[10] = fma(y.pot, v.lg, r[10]);
     }
   }
   if (!valid) return;
@@ -178,14 +243,15 @@ __device__ __forceinline__ void swe_write(const SweOut& o, int64_t i, double u, 
   o.phi[i] = phi;
 }
 
-__global__ void k_swe_out(const double* __restrict__ part, int64_t tpad, int64_t nt, double epssq, double pse_eps, SweOut o) {
+__global__ void k_swe_out(const double* __restrict__ part, int64_t tpad, int64_t nt, double pse_eps,
+                          SweOut o) {
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= nt) return;
   double s[kSweNC];
 #pragma unroll
   for (int k = 0; k < kSweNC; ++k) s[k] = part[k * tpad + i];
   const double i2pi = 0.5 / kPI, i4pi = 0.25 / kPI;
-  const double ea = epssq * s[4], eb = epssq * s[7], a2 = 2.0 * s[3], b2 = 2.0 * s[6];
+  const double ea = s[4], eb = s[7], a2 = 2.0 * s[3], b2 = 2.0 * s[6];
   swe_write(o, i, s[0] * i2pi, s[1] * i2pi, (a2 + s[5] + eb) * i2pi, (s[2] - ea - b2) * i2pi,
             (s[2] + ea - b2) * i2pi, (eb - a2 - s[5]) * i2pi, s[8] / (kPI * pse_eps * pse_eps),
             -s[9] * i4pi, -s[10] * i4pi);
@@ -818,7 +884,7 @@ SwePlan swe_plan(lpm_context& ctx, const uint8_t* mask, int64_t nt, int64_t nf, 
   SwePlan p;
   ctx.arena.reset();
   if (tile == kSweTile64) {
-    // FP64: one warp's pair takes the FP64 pipe of its sub-partition 2,000 to 3,000
+    // FP64: one warp's pair takes the FP64 pipe of its sub-partition 1,200 to 3,000
     // clocks, so few points are cut into chunks of down to 8 sources until every
     // sub-partition has two warps (quad level 2, vertices and faces, with the chunks'
     // sums by k_swe_sum: 306 -> 134 us); CTAs no larger than the targets.
@@ -975,8 +1041,7 @@ void swe_plane_sums(lpm_context& ctx, View tx, const double* ts, int64_t nt, Vie
                                                             epssq, ipse2, ctx.f64_tab, p.part, p.tpad);
   swe_sum(ctx, p, kSweNC);
   const unsigned th = unsigned(sum_threads(nt));
-  k_swe_out<<<unsigned((nt + th - 1) / th), th, 0, ctx.stream>>>(p.part, p.tpad, nt, epssq,
-                                                                pse_eps, out);
+  k_swe_out<<<unsigned((nt + th - 1) / th), th, 0, ctx.stream>>>(p.part, p.tpad, nt, pse_eps, out);
   ctx.launches += 2;
   LPM_CUDA(cudaGetLastError());
 }

@@ -5,6 +5,8 @@ target exactly on a source with eps = 0 (the reference's non-finite values).
 
 Tolerance 1e-12 of the largest value of an output, as the other FP64 tests:
 targets and sources keep 0.02 apart where eps = 0."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -55,6 +57,36 @@ def test_plane(gpu_ctx, oracle, ns, nt, eps, pse, scale, coincident):
     assert _close(o["u"], r[:, :2])
     for k, c in COLS.items():
         assert _close(o[k], r[:, c]), k
+
+
+@pytest.mark.parametrize("scale", [1e-90, 1e-70, 1.0, 1e70, 1e75])
+@pytest.mark.parametrize("eps", [0.0, 1e-9, 0.05, 3.0, 1e4])
+def test_plane_scales(gpu_ctx, oracle, scale, eps):
+    """Positions around the ends of the fixed-point range, eps from far below to far
+    above the distances, pairs on an axis, close together and (eps > 0) coincident."""
+    from lpm_gb300 import core
+
+    rng = np.random.default_rng(7)
+    n = 200
+    x, y = rng.normal(size=(n, 2)), rng.normal(size=(n, 2))
+    x[:40, 1] = y[:40, 1] = 0.0
+    x[50] = y[60] + 1e-6
+    if eps > 0:
+        x[70] = y[80]
+    x, y, eps, pse = x * scale, y * scale, eps * scale, 0.5 * scale
+    z, sg, a = rng.normal(size=n), rng.normal(size=n), rng.uniform(0.5, 1.0, n)
+    sx, sy, m = rng.normal(size=n), rng.normal(size=n), np.zeros(n, np.uint8)
+    gpu_ctx.set_precision(core.FP64)
+    o = F.swe_plane_vertex_sums(gpu_ctx, _dev(x), _dev(sx), _dev(y), _dev(z), _dev(sg), _dev(a),
+                                _dev(m), _dev(sy), eps, pse)
+    gpu_ctx.synchronize()
+    r = oracle.swe_plane_sums(x, sx, y, z, sg, a, m, sy, eps, pse)
+    assert _close(o["u"], r[:, :2])
+    for k in ("psi", "phi"):
+        assert _close(o[k], r[:, COLS[k]]), k
+    if abs(math.log10(scale)) < 74:  # beyond, the oracle's pi R^2 leaves the normal range
+        for k in ("du1dx1", "du1dx2", "du2dx1", "du2dx2", "laps"):
+            assert _close(o[k], r[:, COLS[k]]), k
 
 
 @pytest.mark.parametrize("ns,nt", [(1, 1), (63, 129), (64, 127), (65, 128), (700, 260)])
