@@ -48,11 +48,12 @@ extern "C" {
 /* ---- arithmetic of the pairwise sum ------------------------------------ */
 /* LPM_FP64: the reference's pair kernels in FP64 (1 - x.y [+ eps^2] on the
  *            sphere, |x-y|^2 + eps^2 on the plane) with the cross product
- *            taken out of the sum (u = x cross sum_j (g_j / arg_j) y_j) and one
- *            Newton-Raphson quotient per pair; within 1e-12 of the reference.
+ *            taken out of the sum (u = x cross sum_j (g_j / arg_j) y_j); large
+ *            sphere sums run in error-free float pairs of no larger error;
+ *            within 1e-12 of the reference.
  * LPM_FP64_EXACT: every pair term in FP64 in the reference's evaluation
  *            order (correctly rounded divisions), each term equal to the
- *            reference's bit for bit; about 3x slower than LPM_FP64.
+ *            reference's bit for bit; about EXACT_HDR slower than LPM_FP64.
  * LPM_FP32C: FP32 pair kernel (denominator rebuilt as |x-y|^2/2 + eps^2),
  *            per-tile Kahan/TwoSum-compensated sums, FP64 epilogue. */
 #define LPM_FP64 64
@@ -91,8 +92,8 @@ int lpm_context_set_precision(lpm_context* ctx, int precision);
  * 128x8 with 4, 256x2 with 5, 128x8 with 3, 256x4 with 2; the same table as
  * lpm_ensemble_set_kernel) of later LPM_FP32C functor calls and of steppers
  * created afterwards (a stepper keeps the shape it was created with), or (-1,
- * the default) lets each problem size time the six shapes once and keep the
- * fastest.  A target's sums do not depend on the
+ * the default) lets each problem size of 2e9 pairs and more time the six shapes
+ * once and keep the fastest (smaller ones take a shape by their size).  A target's sums do not depend on the
  * shape. */
 int lpm_context_set_kernel_shape(lpm_context* ctx, int shape);
 /* Waits for the context's stream, then reports LPM_ERR_TIMEOUT if a bounded
@@ -233,7 +234,7 @@ int lpm_bve_rk4_advance_timestep(lpm_bve_rk4* st, lpm_view vx, double* vzeta,
 int lpm_bve_rk4_nbody_time(lpm_bve_rk4* st, double* ms, int64_t* launches);
 /* The N-body kernel shape the stepper runs: threads per CTA, targets per
  * thread and the CTAs per SM its register cap is set for (LPM_FP32C: the
- * autotuned one of the six shapes; FP64 forms: the fixed shape, 0 CTAs).
+ * chosen one of the six shapes; FP64 forms: the tiled kernels' shape, 0 CTAs).
  * Valid after the first step (LPM_ERR_STATE before). */
 int lpm_bve_rk4_kernel_shape(lpm_bve_rk4* st, int* threads, int* targets_per_thread,
                              int* min_ctas_per_sm);
@@ -403,8 +404,8 @@ int lpm_measure_fma_peak(lpm_context* ctx, int precision, double* tflops);
  * product du/dx^2 + 2 du/dy dv/dx + dv/dy^2, the four velocity gradients,
  * the PSE surface Laplacian (pse::BivariateOrder8 of width pse_eps), the
  * stream and potential functions; masked faces are skipped.  Context
- * precision LPM_FP64: the reference's pair arithmetic (planar_swe_sums_rhs_pse,
- * :394-480); LPM_FP32C: FP32 moment sums with compensation (velocity ~1e-7,
+ * precision LPM_FP64: the terms of planar_swe_sums_rhs_pse (:394-480) in FP64,
+ * regrouped into moments; LPM_FP32C: FP32 moment sums with compensation (velocity ~1e-7,
  * stream/potential ~1e-6, gradients and Laplacian ~1e-5 relative). */
 int lpm_swe_plane_vertex_sums(lpm_context* ctx, lpm_view u, double* ddot,
                               double* du1dx1, double* du1dx2, double* du2dx1,
@@ -434,7 +435,7 @@ int lpm_swe_plane_face_sums(lpm_context* ctx, lpm_view u, double* ddot,
  * pot = -sigma A; sphere_swe_velocity_sums, :335-373).  grad, if not NULL,
  * receives M itself (nv x 9, row-major, contiguous).  Masked faces are
  * skipped.  Context precision LPM_FP64 (or LPM_FP64_CHORD): FP64, the
- * reference's pair arithmetic; LPM_FP32C: FP32 chord-form moments with
+ * reference's terms regrouped into moments; LPM_FP32C: FP32 chord-form moments with
  * compensated sums (velocity ~1e-7, gradient ~1e-5 relative). */
 int lpm_swe_sphere_vertex_sums(lpm_context* ctx, lpm_view u, double* ddot,
                                double* grad, lpm_view vx, int64_t nv,
@@ -517,7 +518,7 @@ int lpm_farfield_create(lpm_context* ctx, lpm_farfield** out, double theta,
 int lpm_farfield_destroy(lpm_farfield* ff);
 /* Velocity at nx targets x (device, strided) from the face slots fx/zeta/
  * area/mask (nf slots, the BVEFaceVelocity source arguments).  Builds the
- * tree for these positions (host sort, synchronises) and evaluates. */
+ * tree for these positions (on the device; waits for two counts) and evaluates. */
 int lpm_farfield_velocity(lpm_farfield* ff, lpm_view u, lpm_view x,
                           int64_t nx, lpm_view fx, const double* zeta,
                           const double* area, const uint8_t* mask, int64_t nf,

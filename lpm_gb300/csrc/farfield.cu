@@ -3,16 +3,16 @@
 // Per evaluation (all on the context stream, capturable in a CUDA graph):
 //   k_ff_sort_src   packed double4_16a sources -> Morton-ordered float4
 //   k_ff_cells      per cell: centre, radius, frame, moments to order 4
-//                   (FP32 per 32-point batch, FP64 across batches and threads)
+//                   (FP32 per batch, FP64 across batches and threads)
 //   k_ff_tblocks    per block of 128 Morton-ordered targets: centre, radius
-//   k_ff_lists      per target block: tree walk with the opening criterion
+//   k_ff_lists      a warp per target block: tree walk with the opening criterion
 //                   h <= theta (D - r_b): far cells (of >= kExactMax points;
 //                   smaller accepted cells are leaves and join the near
 //                   list), near leaves, and the far cells close enough
 //                   (h / (D - r_b) >= rho_min) for the learned correction; a
 //                   block whose lists overflow is marked for the direct sum
-//   k_ff_eval       per target block: exact FP32 chord sum over the near
-//                   leaves (per-leaf partials merged by TwoSum) + order-4
+//   k_ff_eval       per target block and part: exact FP32 chord sum over the
+//                   near leaves (partials merged by TwoSum) + order-4
 //                   expansion of the far cells, or the full direct sum for
 //                   a marked block; writes FP64 w
 //   k_ff_mlp        (mlp.cu) learned correction on tensor cores, adds to w
