@@ -60,6 +60,16 @@ __device__ __forceinline__ void f64_table_entry(F64Tables* T, int i) {
   T->ex[i] = t;
 }
 
+// A float as a double by its bits: the conversion instruction holds the FP64 pipe as
+// long as an addition.
+static __device__ __noinline__ double f64_widen_any(float v) { return double(v); }
+__device__ __forceinline__ double f64_widen(float v) {
+  const unsigned b = __float_as_uint(v), m = b & 0x7fffffffu;
+  if (m - 0x00800000u < 0x7f000000u)  // normal
+    return __hiloint2double(int((b & 0x80000000u) | ((m >> 3) + (896u << 20))), int(b << 29));
+  return m == 0 ? 0.0 : f64_widen_any(v);
+}
+
 // Whether x is a positive normal number in [2^-1000, 2^1000).
 __device__ __forceinline__ bool f64_plain(double x) {
   const unsigned h = unsigned(__double2hiint(x));
