@@ -42,7 +42,7 @@ EPS = 0.01
 DT = 0.005
 OMEGA = 2 * math.pi
 FLOPS_PER_PAIR = 24  # credited flops of the sphere u pair (eps form)
-SPLIT_LANE_OPS = 125  # FP32 lane operations per pair of LPM_FP64's sphere sums
+SPLIT_LANE_OPS = 163  # FP32-pipe lane operations per pair of LPM_FP64's sphere sums (profile)
 L2_FLUSH_BYTES = 512 << 20
 
 

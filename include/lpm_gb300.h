@@ -53,7 +53,7 @@ extern "C" {
  *            within 1e-12 of the reference.
  * LPM_FP64_EXACT: every pair term in FP64 in the reference's evaluation
  *            order (correctly rounded divisions), each term equal to the
- *            reference's bit for bit; about EXACT_HDR slower than LPM_FP64.
+ *            reference's bit for bit; about 20x slower (sphere) than LPM_FP64.
  * LPM_FP32C: FP32 pair kernel (denominator rebuilt as |x-y|^2/2 + eps^2),
  *            per-tile Kahan/TwoSum-compensated sums, FP64 epilogue. */
 #define LPM_FP64 64

@@ -2,8 +2,8 @@
 // error-free transformations.
 //
 // Why: this part executes about 1.7 FP64 FMAs per clock per SM against 128
-// FP32 ones, so the 11 FP64 operations of a pair (nbody_f64h) cost as much
-// pipe time as 700 FP32 operations.  The form below takes about 115 FP32
+// FP32 ones, so the 8 FP64 operations of a pair (nbody_f64h) cost as much
+// pipe time as 500 FP32 operations.  The form below takes about 160 FP32
 // operations per sphere pair and keeps the accuracy of the FP64 kernels:
 //
 //  * Positions are scaled by a power of two into (-1, 1) and cut into three
@@ -42,10 +42,9 @@
 // path for all their pairs; all targets do when a sixteenth of the sources is
 // that far off the sphere or eps is far larger than the domain.
 // Measured on one GB300 (SM clock 2,070 MHz), pair kernel alone, velocity:
-// icosahedral level 4 (7,682 x 5,120 pairs) 169 us, 233 Gpairs/s, against
-// 0.92 ms for nbody_f64h; with the stream function 10 times nbody_f64h's rate.
-// Bound: FP32 issue, 125 lane operations per pair (128 lanes per clock per SM:
-// 76 % of that at level 4, whose 2,440 CTAs end in a ragged second wave).
+// icosahedral level 5 (10,242 x 20,480 pairs) 0.85 ms, 245 Gpairs/s, where 8 FP64
+// operations per pair take 2.7 ms.  Bound: the FP32 pipe: 163 instructions, mostly
+// f32x2 of two clocks each, per step of two sources fill 99 % of its clocks there.
 #pragma once
 
 #include <type_traits>
