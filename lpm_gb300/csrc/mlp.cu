@@ -1231,7 +1231,7 @@ void lpm_farfield::grad(const float* x_host, const float* y_host, int n, float* 
   Arena& ar = ctx->arena;
   ar.reset();
   ar.reserve(size_t(n) * (kIn * 6 + 7 * sizeof(float)) + sizeof(float) * size_t(slab) * (kNParam + 1) +
-             sizeof(double) * kNParam + 16 * 256);
+             (sizeof(double) + sizeof(float)) * kNParam + 16 * 256);
   float* dxf = static_cast<float*>(ar.take(sizeof(float) * size_t(n) * kIn));
   float* dyf = static_cast<float*>(ar.take(sizeof(float) * size_t(n) * 3));
   uint16_t* dX = static_cast<uint16_t*>(ar.take(sizeof(uint16_t) * size_t(n) * kIn));
@@ -1239,7 +1239,8 @@ void lpm_farfield::grad(const float* x_host, const float* y_host, int n, float* 
   float* gpart = static_cast<float*>(ar.take(sizeof(float) * kNParam * size_t(slab)));
   float* lpart = static_cast<float*>(ar.take(sizeof(float) * slab));
   double* gsum = static_cast<double*>(ar.take(sizeof(double) * kNParam));
-  float* gout = reinterpret_cast<float*>(dxf);  // the raw rows are spent by then
+  // (k_mlp_gsum's CTAs write it while others still read gpart)
+  float* gout = static_cast<float*>(ar.take(sizeof(float) * kNParam));
   LPM_CUDA(cudaMemcpyAsync(dxf, x_host, sizeof(float) * size_t(n) * kIn, cudaMemcpyHostToDevice, st));
   LPM_CUDA(cudaMemcpyAsync(dyf, y_host, sizeof(float) * size_t(n) * 3, cudaMemcpyHostToDevice, st));
   k_mlp_rows<<<unsigned((int64_t(n) * kIn / 2 + 255) / 256), 256, 0, st>>>(dxf, dyf, n, dX, dY);
