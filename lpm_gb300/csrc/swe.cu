@@ -452,35 +452,90 @@ __global__ void k_swe_plane32_out(const double* __restrict__ part, int64_t tpad,
 //     gkz = D [y]x + c v^T,          v = (1 + eps^2) x - y
 //     gks = -v w^T - D s P,          w = P y = y - s x
 //   (w - D x = -v because s + D = 1 + eps^2).
-// With d = x - y every term is a moment of d (c = d cross x, v = eps^2 x + d,
-// w = (1 - s) x - d, identically): writing sz, ss = rot, pot / (4 pi D) and
-// R, Q = rot, pot / (4 pi D^2), the 28 sums
-//   A, B = sum sz d, ss d;  U1, V1 = sum R d, Q d;  U2, V2 = sum R, Q d d^T;
-//   Z, G = sum sz, ss;  H = sum ss (1 - s);  K = sum Q
-// give, with O = sum Q (1 - s) = G - eps^2 K and N = B - eps^2 V1,
-//   u = A x x - B + H x
-//   M = eps^2 (U1 x x) x^T + [U2 columns] x x + V2 - N x^T + eps^2 x V1^T
-//       - eps^2 O x x^T + [Z x - A]x - (G - H) P.
+// Sums over sources are taken in the target's frame (t1, t2, n), x = rho n: with
+// p_a = t_a.(x - y), sz, ss = rot, pot / (4 pi D) and R, Q = rot, pot / (4 pi D^2),
+// c = rho (p2, -p1, 0), w = (-p1, -p2, k yn) and v = (p1, p2, rho D - k yn) for
+// k = 1 - |x|^2 and yn = s / rho, so the 17 sums
+//   sz p, ss p;  R, Q (p1 p1, p1 p2, p2 p2);  sz s, ss s;
+//   R s p, Q s p, Q s^2 (times k: targets off the unit sphere)
+// give u and M (sph_assemble).  A sum along x would be n / sqrt(n) times larger
+// than the tangential ones it is added to in fixed axes, whose roundings then
+// stay when x is projected out (same-sign strengths: errors 30 times larger), and
+// eps^2 enters no difference of sums.  t_a.x is not 0 but about 1e-16: p_a leaves it
+// out exactly (tau_a), as it would add up over the sources.
 // FP64: s and D = (1 - s) + eps^2 unfused in the reference's order (D is
 // the ill-conditioned quantity: a one-ulp change of s moves a near pair's D by
 // ~1e-16 / D relative), everything after it contracted, one reciprocal of D per
-// pair in integers (f64math.cuh).  The FP64 pipe bounds the kernel: 48 operations
-// per pair (66 in the form that added c v^T, v w^T, u term by term): icosahedral
-// level 5, vertices and faces, 96.5 -> 68.6 ms (81.8 ms with the reciprocal by the
-// hardware's FP64 approximation and three operations, which costs eight);
-// level 2, where chunks of 8 to 64 sources instead of 256 fill the SMs, 1.31 ->
-// 0.14 ms.
-constexpr int kSphNC = 28;  // A3 B3 U1[3] V1[3] U2[6] V2[6] Z G H K
+// pair in integers (f64math.cuh).  The FP64 pipe bounds the kernel: 44 operations
+// per pair (66 in the form that added c v^T, v w^T, u term by term in fixed axes, 48
+// as moments of x - y in fixed axes): icosahedral level 5, vertices and faces, 96.5 /
+// 68.5 / 61.4 ms, level 2, where chunks of 8 to 64 sources fill the SMs, 0.143 ms.
+constexpr int kSphNC = 17;
 
 struct __align__(16) SphSrc {
   double x, y, z, rot, pot;  // strengths over 4 pi
   int slot, pad;
 };
 
+// a.b exactly to about 1e-31, rounded to FP64.
+__device__ __forceinline__ double exact_dot(const double (&a)[3], const double (&b)[3], double s) {
+  double e = 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double p = dm(a[c], b[c]), pe = fma(a[c], b[c], -p);
+    const double t = da(s, p), bb = ds(t, s);
+    e += ds(s, ds(t, bb)) + ds(p, bb) + pe;
+    s = t;
+  }
+  return s + e;
+}
+
+// A target's frame, once per call (about 200 FP64 operations, as many as five pairs,
+// and a chunk may hold eight): t1, t2, tau1, tau2, tau1 / rho^2, tau2 / rho^2 for the
+// pair kernel; n, rho, 1 - rho^2 for the assembly.  At x = 0 any frame, rho = 0.
+enum : int { kT1 = 0, kT2 = 3, kTau = 6, kTauR = 8, kN = 10, kRho = 13, kDef = 14, kSphFrame = 15 };
+
+__device__ __forceinline__ void sph_frame(const double (&x)[3], double (&f)[kSphFrame]) {
+  const double mx[3] = {-x[0], -x[1], -x[2]};
+  f[kDef] = exact_dot(mx, x, 1.0);
+  double rho = sqrt(exact_dot(x, x, 0.0));
+  const bool zero = rho < 0x1p-300;
+  if (zero) rho = 0.0;
+  f[kRho] = rho;
+  const double ir = 1.0 / rho;
+  double n[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) f[kN + a] = n[a] = zero ? (a == 2 ? 1.0 : 0.0) : x[a] * ir;
+  const double sg = n[2] >= 0.0 ? 1.0 : -1.0, q = -1.0 / (sg + n[2]), b = n[0] * n[1] * q;
+  const double t1[3] = {1.0 + sg * n[0] * n[0] * q, sg * b, -sg * n[0]};
+  const double t2[3] = {b, sg + n[1] * n[1] * q, -n[1]};
+  const double tau[2] = {exact_dot(t1, x, 0.0), exact_dot(t2, x, 0.0)};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) f[kT1 + a] = t1[a], f[kT2 + a] = t2[a];
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
+    f[kTau + a] = zero ? 0.0 : tau[a];
+    f[kTauR + a] = zero ? 0.0 : tau[a] * (ir * ir);
+  }
+}
+
+// Source records, and in the blocks after them the targets' frames.
 __global__ void k_swe_sphere_pack(View fx, const double* __restrict__ zeta,
                                   const double* __restrict__ sigma, const double* __restrict__ area,
                                   const int* __restrict__ src2slot, int64_t ns,
-                                  SphSrc* __restrict__ src) {
+                                  SphSrc* __restrict__ src, View tx, int64_t nt, int64_t tpad,
+                                  double* __restrict__ fr) {
+  const int64_t src_blocks = (ns + blockDim.x - 1) / blockDim.x;
+  if (int64_t(blockIdx.x) >= src_blocks) {
+    const int64_t i = (blockIdx.x - src_blocks) * int64_t(blockDim.x) + threadIdx.x;
+    if (i >= nt) return;
+    const double x[3] = {tx(i, 0), tx(i, 1), tx(i, 2)};
+    double f[kSphFrame];
+    sph_frame(x, f);
+#pragma unroll
+    for (int k = 0; k < kSphFrame; ++k) fr[k * tpad + i] = f[k];
+    return;
+  }
   const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (k >= ns) return;
   const int64_t j = src2slot[k];
@@ -499,6 +554,7 @@ __global__ void k_swe_sphere_pack(View fx, const double* __restrict__ zeta,
 // COLL: collocated targets, the source in the target's own slot is skipped.
 template <bool COLL>
 __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
+                                                       const double* __restrict__ fr,
                                                        const SphSrc* __restrict__ src, int64_t ns,
                                                        int64_t chunk_len, double epssq,
                                                        double* __restrict__ part, int64_t tpad) {
@@ -510,6 +566,10 @@ __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
   double x[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) x[a] = valid ? tx(i, a) : 0.0;
+  double f[kN];
+#pragma unroll
+  for (int k = 0; k < kN; ++k) f[k] = valid ? fr[k * tpad + i] : 0.0;
+  const bool zero = valid && fr[kRho * tpad + i] == 0.0;
   double r[kSphNC];
 #pragma unroll
   for (int k = 0; k < kSphNC; ++k) r[k] = 0.0;
@@ -527,32 +587,34 @@ __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
       // x.y unfused in the reference's order: 1 - s cancels, and its rounding
       // is the reference's
       const double s = da(da(dm(x[0], y.x), dm(x[1], y.y)), dm(x[2], y.z));
-      const double om = ds(1.0, s), D = da(om, epssq);
+      const double D = da(ds(1.0, s), epssq);
       const double rd = f64_inv(D);
       const double d[3] = {x[0] - y.x, x[1] - y.y, x[2] - y.z};
+      // t_a.d less its part along x, tau_a (1 - s / rho^2)
+      const double p1 = fma(f[kTauR], s, fma(f[0], d[0], fma(f[1], d[1], fma(f[2], d[2], -f[kTau]))));
+      const double p2 = fma(f[kTauR + 1], s, fma(f[3], d[0], fma(f[4], d[1], fma(f[5], d[2], -f[kTau + 1]))));
       const double sz = y.rot * rd, ss = y.pot * rd;
       const double R = sz * rd, Q = ss * rd;
-      double rr[3], qq[3];
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        r[a] = fma(sz, d[a], r[a]);
-        r[3 + a] = fma(ss, d[a], r[3 + a]);
-        rr[a] = R * d[a];
-        qq[a] = Q * d[a];
-        r[6 + a] += rr[a];
-        r[9 + a] += qq[a];
-      }
-#pragma unroll
-      for (int a = 0, k = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = a; b < 3; ++b, ++k) {
-          r[12 + k] = fma(rr[a], d[b], r[12 + k]);
-          r[18 + k] = fma(qq[a], d[b], r[18 + k]);
-        }
-      r[24] += sz;
-      r[25] += ss;
-      r[26] = fma(ss, om, r[26]);
-      r[27] += Q;
+      const double r1 = R * p1, r2 = R * p2, q1 = Q * p1, q2 = Q * p2;
+      double sn = s;  // rho yn; yn at x = 0
+      if (zero) sn = y.z;
+      r[0] = fma(sz, p1, r[0]);
+      r[1] = fma(sz, p2, r[1]);
+      r[2] = fma(ss, p1, r[2]);
+      r[3] = fma(ss, p2, r[3]);
+      r[4] = fma(r1, p1, r[4]);
+      r[5] = fma(r1, p2, r[5]);
+      r[6] = fma(r2, p2, r[6]);
+      r[7] = fma(q1, p1, r[7]);
+      r[8] = fma(q1, p2, r[8]);
+      r[9] = fma(q2, p2, r[9]);
+      r[10] = fma(sz, sn, r[10]);
+      r[11] = fma(ss, sn, r[11]);
+      r[12] = fma(r1, sn, r[12]);
+      r[13] = fma(r2, sn, r[13]);
+      r[14] = fma(q1, sn, r[14]);
+      r[15] = fma(q2, sn, r[15]);
+      r[16] = fma(Q * sn, sn, r[16]);
     }
   }
   if (!valid) return;
@@ -560,50 +622,49 @@ __global__ void __launch_bounds__(kSweNT) k_swe_sphere(View tx, int64_t nt,
   for (int k = 0; k < kSphNC; ++k) part[(c * kSphNC + k) * tpad + i] = r[k];
 }
 
-__global__ void k_swe_sphere_out(const double* __restrict__ part, int64_t tpad, View tx, int64_t nt, double eps2, View u, double* __restrict__ ddot,
-                                 double* __restrict__ grad, int do_velocity) {
-  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i >= nt) return;
-  double s[kSphNC];
+// u and M of one target in its frame, then in the caller's axes.
+__device__ __forceinline__ void sph_assemble(const double (&f)[kSphFrame], const double (&s)[kSphNC],
+                                             double (&u)[3], double (&M)[9]) {
+  const double rho = f[kRho], k = f[kDef];
+  const bool zero = rho == 0.0;
+  const double ir = zero ? 1.0 : 1.0 / rho;  // yn = ir sn
+  const double kir = k * ir, rk = zero ? 0.0 : k;
+  const double Yn = s[10] * ir, G = zero ? 0.0 : s[11];  // sum sz yn, sum ss x.y
+  const double ul[3] = {rho * s[1] - s[2], -rho * s[0] - s[3], kir * s[11]};
+  // sum sz y = (-s0, -s1, Yn); P = diag(1, 1, k)
+  // (R c_a v_n = +-rho R (rho D - k yn) p; Q v_n = rho ss - k Q yn)
+  const double vn1 = rho * s[2] - kir * s[14], vn2 = rho * s[3] - kir * s[15];
+  const double L[9] = {
+      rho * s[5] + s[7] - G,  rho * s[6] + s[8] - Yn,  rho * rho * s[1] - rk * s[13] - kir * s[14] - s[1],
+      -rho * s[4] + s[8] + Yn, -rho * s[5] + s[9] - G, -rho * rho * s[0] + rk * s[12] - kir * s[15] + s[0],
+      vn1 + s[1],             vn2 - s[0],              -kir * (rho * s[11] - kir * s[16]) - G * k};
 #pragma unroll
-  for (int k = 0; k < kSphNC; ++k) s[k] = part[k * tpad + i];
-  const double x[3] = {tx(i, 0), tx(i, 1), tx(i, 2)};
-  const double *A = s, *B = s + 3, *U1 = s + 6, *V1 = s + 9, *U2 = s + 12, *V2 = s + 18;
-  const double Z = s[24], G = s[25], H = s[26];
-  const int sym[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};  // (a, b) -> packed symmetric index
-  auto cross = [](const double* p, const double* q, double* o) {
-    o[0] = p[1] * q[2] - p[2] * q[1];
-    o[1] = p[2] * q[0] - p[0] * q[2];
-    o[2] = p[0] * q[1] - p[1] * q[0];
-  };
-  if (do_velocity) {
-    double ax[3];
-    cross(A, x, ax);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) u(i, a) = ax[a] - B[a] + H * x[a];
-  }
-  const double O = G - eps2 * s[27];
-  double u1x[3], zy[3], N[3];
-  cross(U1, x, u1x);
+  for (int a = 0; a < 3; ++a) u[a] = ul[0] * f[kT1 + a] + ul[1] * f[kT2 + a] + ul[2] * f[kN + a];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    zy[a] = Z * x[a] - A[a];
-    N[a] = B[a] - eps2 * V1[a];
-  }
-  const double Yx[9] = {0.0, -zy[2], zy[1], zy[2], 0.0, -zy[0], -zy[1], zy[0], 0.0};
-  double M[9];
+    double h[3];  // row a of (F L)
 #pragma unroll
-  for (int b = 0; b < 3; ++b) {
-    const double col[3] = {U2[sym[b]], U2[sym[3 + b]], U2[sym[6 + b]]};
-    double t1[3];
-    cross(col, x, t1);
+    for (int q = 0; q < 3; ++q) h[q] = f[kT1 + a] * L[q] + f[kT2 + a] * L[3 + q] + f[kN + a] * L[6 + q];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double P = (a == b ? 1.0 : 0.0) - x[a] * x[b];
-      M[3 * a + b] = eps2 * (u1x[a] * x[b] + x[a] * V1[b] - O * x[a] * x[b]) + t1[a] +
-                     V2[sym[3 * a + b]] - N[a] * x[b] + Yx[3 * a + b] - (G - H) * P;
-    }
+    for (int b = 0; b < 3; ++b) M[3 * a + b] = h[0] * f[kT1 + b] + h[1] * f[kT2 + b] + h[2] * f[kN + b];
   }
+}
+
+__global__ void k_swe_sphere_out(const double* __restrict__ part, int64_t tpad,
+                                 const double* __restrict__ fr, int64_t nt, View u,
+                                 double* __restrict__ ddot, double* __restrict__ grad,
+                                 int do_velocity) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i >= nt) return;
+  double s[kSphNC], f[kSphFrame], v[3], M[9];
+#pragma unroll
+  for (int k = 0; k < kSphNC; ++k) s[k] = part[k * tpad + i];
+#pragma unroll
+  for (int k = 0; k < kSphFrame; ++k) f[k] = fr[k * tpad + i];
+  sph_assemble(f, s, v, M);
+  if (do_velocity)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) u(i, a) = v[a];
   // sum_ij M_ij M_ji in the functors' loop order
   double dsum = 0.0;
 #pragma unroll
@@ -875,12 +936,13 @@ struct SwePlan {
   int* src2slot = nullptr;
   void* src = nullptr;     // ns packed source records
   int* slot = nullptr;     // ns slot indices (when asked for)
+  double* tgt = nullptr;   // [tgt_doubles][tpad] (when asked for)
   double* part = nullptr;  // [chunk][ncomp][tpad]
   dim3 grid() const { return dim3{unsigned(nb), unsigned(nchunks), 1u}; }
 };
 
 SwePlan swe_plan(lpm_context& ctx, const uint8_t* mask, int64_t nt, int64_t nf, size_t rec_bytes,
-                 int ncomp, bool want_slot, int tile) {
+                 int ncomp, bool want_slot, int tile, int tgt_doubles = 0) {
   SwePlan p;
   ctx.arena.reset();
   if (tile == kSweTile64) {
@@ -897,7 +959,8 @@ SwePlan swe_plan(lpm_context& ctx, const uint8_t* mask, int64_t nt, int64_t nf, 
   const int64_t nch_max =
       std::max<int64_t>(1, std::min<int64_t>(want, (nf + tile - 1) / tile));
   ctx.arena.reserve(sizeof(int) * (3 * size_t(nf) + 2 * size_t(nf) / 1024 + 8) +
-                    rec_bytes * size_t(nf) + sizeof(double) * ncomp * size_t(nch_max) * p.tpad +
+                    rec_bytes * size_t(nf) +
+                    sizeof(double) * (ncomp * size_t(nch_max) + tgt_doubles) * p.tpad +
                     8 * 4096);
   int* slot2src = static_cast<int*>(ctx.arena.take(sizeof(int) * std::max<int64_t>(nf, 1)));
   p.src2slot = static_cast<int*>(ctx.arena.take(sizeof(int) * std::max<int64_t>(nf, 1)));
@@ -908,6 +971,7 @@ SwePlan swe_plan(lpm_context& ctx, const uint8_t* mask, int64_t nt, int64_t nf, 
   int64_t len = (p.ns + nch_max - 1) / nch_max;
   p.chunk_len = std::max<int64_t>(tile, (len + tile - 1) / tile * tile);
   p.nchunks = int(std::max<int64_t>(1, (p.ns + p.chunk_len - 1) / p.chunk_len));
+  if (tgt_doubles) p.tgt = static_cast<double*>(ctx.arena.take(sizeof(double) * tgt_doubles * p.tpad));
   p.part = static_cast<double*>(ctx.arena.take(sizeof(double) * ncomp * size_t(p.nchunks) * p.tpad));
   return p;
 }
@@ -961,23 +1025,22 @@ void swe_sphere_sums(lpm_context& ctx, View tx, int64_t nt, View fx, const doubl
                       do_velocity);
     return;
   }
-  const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(SphSrc), kSphNC, false, kSweTile64);
+  const SwePlan p = swe_plan(ctx, mask, nt, nf, sizeof(SphSrc), kSphNC, false, kSweTile64, kSphFrame);
   auto* src = static_cast<SphSrc*>(p.src);
-  if (p.ns > 0) {
-    k_swe_sphere_pack<<<blocks256(p.ns), 256, 0, ctx.stream>>>(fx, zeta, sigma, area, p.src2slot,
-                                                               p.ns, src);
-    ctx.launches++;
-  }
+  const unsigned nblk = unsigned((p.ns + 127) / 128 + (nt + 127) / 128);
+  k_swe_sphere_pack<<<nblk, 128, 0, ctx.stream>>>(fx, zeta, sigma, area, p.src2slot, p.ns, src, tx,
+                                                  nt, p.tpad, p.tgt);
+  ctx.launches++;
   if (collocated)
-    k_swe_sphere<true><<<p.grid(), p.threads, 0, ctx.stream>>>(tx, nt, src, p.ns, p.chunk_len,
-                                                            eps * eps, p.part, p.tpad);
+    k_swe_sphere<true><<<p.grid(), p.threads, 0, ctx.stream>>>(tx, nt, p.tgt, src, p.ns, p.chunk_len,
+                                                               eps * eps, p.part, p.tpad);
   else
-    k_swe_sphere<false><<<p.grid(), p.threads, 0, ctx.stream>>>(tx, nt, src, p.ns, p.chunk_len,
-                                                             eps * eps, p.part, p.tpad);
+    k_swe_sphere<false><<<p.grid(), p.threads, 0, ctx.stream>>>(tx, nt, p.tgt, src, p.ns, p.chunk_len,
+                                                                eps * eps, p.part, p.tpad);
   swe_sum(ctx, p, kSphNC);
   const unsigned th = unsigned(sum_threads(nt));
   k_swe_sphere_out<<<unsigned((nt + th - 1) / th), th, 0, ctx.stream>>>(
-      p.part, p.tpad, tx, nt, eps * eps, u, ddot, grad, do_velocity);
+      p.part, p.tpad, p.tgt, nt, u, ddot, grad, do_velocity);
   ctx.launches += 2;
   LPM_CUDA(cudaGetLastError());
 }
