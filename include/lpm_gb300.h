@@ -49,8 +49,10 @@ extern "C" {
 /* LPM_FP64: the reference's pair kernels in FP64 (1 - x.y [+ eps^2] on the
  *            sphere, |x-y|^2 + eps^2 on the plane) with the cross product
  *            taken out of the sum (u = x cross sum_j (g_j / arg_j) y_j); large
- *            sphere sums run in error-free float pairs of no larger error;
- *            within 1e-12 of the reference.
+ *            sphere sums run in float pairs (48 bits per term, exact x - y)
+ *            where the strengths have at least 256 effective sources,
+ *            (sum |g|)^2 / sum g^2, also counted with their signs if all lie
+ *            within about a hemisphere; within 1e-12 of the reference.
  * LPM_FP64_EXACT: every pair term in FP64 in the reference's evaluation
  *            order (correctly rounded divisions), each term equal to the
  *            reference's bit for bit; about 20x slower (sphere) than LPM_FP64.

@@ -480,11 +480,12 @@ namespace {
 // kernels for grids too small for them, or those.
 enum Fp64Kind : int { FP64_TILED = 0, FP64_FINE = 1, FP64_SPLIT = 2 };
 
-// Whether the split sums (nbody_split.cuh) replace nbody_f64h: the sphere
-// forms, from 1,024 sources on (their error falls as 1 / sqrt(nsrc); against
-// exact values, icosahedral and cubed meshes of 1,280 to 20,480 sources: split
-// 0.8e-15 to 1.8e-15, nbody_f64h 1.3e-15 to 5.1e-15) and half a million pairs
-// on (below, the fine grid of nbody_f64h takes less than the two extra launches).
+// Whether the split sums (nbody_split.cuh) may replace nbody_f64h (each evaluation
+// decides by its strengths): the sphere forms, from 1,024 sources on (their error
+// falls as 1 / sqrt(nsrc) for strengths of like size; against exact values,
+// icosahedral and cubed meshes of 1,280 to 20,480 sources: split 0.8e-15 to 1.8e-15,
+// nbody_f64h 1.3e-15 to 5.1e-15) and half a million pairs on (below, the fine grid of
+// nbody_f64h takes less than the two extra launches).
 bool split_wanted(int precision, int ndim, int64_t ntgt, int64_t nsrc) {
   return precision == LPM_FP64 && ndim == 3 && nsrc >= 1024 && double(ntgt) * double(nsrc) >= 5e5;
 }

@@ -10,6 +10,7 @@ namespace lpm {
 namespace {
 
 constexpr int kRangeThreads = 256;
+constexpr int kSplitSums = 7;  // of k_split_pack's sources
 
 // Magnitudes are compared by the high word of the double (exponent and 20
 // mantissa bits): integer operations, where FP64 ones would take longer than
@@ -29,7 +30,7 @@ __global__ void __launch_bounds__(kRangeThreads)
                   SplitScale* __restrict__ scale) {
   __shared__ int sh[3];
   if (threadIdx.x < 3) sh[threadIdx.x] = 0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) scale->off = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *scale = SplitScale{};
   __syncthreads();
   int ms = 0, mg = 0, mt = 0;
   const int64_t step = int64_t(gridDim.x) * kRangeThreads;
@@ -67,7 +68,7 @@ __device__ SplitScale split_scale(const int4* __restrict__ part, int nparts, dou
   ms = __reduce_max_sync(0xffffffffu, ms);
   mg = __reduce_max_sync(0xffffffffu, mg);
   mt = __reduce_max_sync(0xffffffffu, mt);
-  SplitScale s{0, 0, 0, 0};
+  SplitScale s{};
   // targets up to eight times as far out as the sources are in range; others
   // (divided faces that ran away, say) take the FP64 path one by one
   const int es = exponent_above(ms), ep = exponent_above(magnitude(eps));
@@ -83,7 +84,8 @@ __device__ SplitScale split_scale(const int4* __restrict__ part, int nparts, dou
 
 // The split records of the sources (pairs) and, in the blocks after them, of
 // the targets; once per evaluation, so the pair kernel's CTAs (one per target
-// block and chunk) start without FP64 work.
+// block and chunk) start without FP64 work.  The sources' blocks also sum what the
+// verdict goes by, in integers (in any order the same).
 __global__ void __launch_bounds__(128)
     k_split_pack(const double4_16a* __restrict__ src, int64_t nsrc, int64_t npairs,
                  const double4_16a* __restrict__ tgt, int64_t ntgt, int64_t ntgt_pad, double eps,
@@ -109,13 +111,14 @@ __global__ void __launch_bounds__(128)
     r.x = split3(x), r.y = split3(y), r.z = split3(z);
     const double off = unit_defect(t.x, t.y, t.z);
     split2((2.0 * eps * eps + off) * xs * xs, r.ch, r.cl);
-    r.exact = i < ntgt && (sc.big || fabs(off) > 1.0 || fabs(x) >= 1.0 || fabs(y) >= 1.0 ||
+    r.exact = i < ntgt && (fabs(off) > 1.0 || fabs(x) >= 1.0 || fabs(y) >= 1.0 ||
                            fabs(z) >= 1.0);
     st[i] = r;
     return;
   }
   const int64_t k = int64_t(blockIdx.x) * 128 + threadIdx.x;
-  if (k >= npairs) return;
+  // |g|, g^2, g, |g| y of the thread's sources in fixed point, and those off the sphere
+  int sum[kSplitSums] = {};
   // padding: zero strength, outside the domain, so no denominator is zero
   float3 p[2][3];
   float2 gh, gl, ch, cl;
@@ -132,8 +135,15 @@ __global__ void __launch_bounds__(128)
     float h, l;
     split2(-s.w * gs, h, l);
     put(gh, j, h), put(gl, j, l);
+    const int f = __float2int_rn(-h * 0x1p20f);
+    sum[0] += abs(f);
+    sum[1] += __float2int_rn(h * h * 0x1p24f);
+    sum[2] += f;
+    sum[3] += __float2int_rn(fabsf(h) * 0x1p20f * p[j][0].x);
+    sum[4] += __float2int_rn(fabsf(h) * 0x1p20f * p[j][1].x);
+    sum[5] += __float2int_rn(fabsf(h) * 0x1p20f * p[j][2].x);
     const double off = real ? unit_defect(s.x, s.y, s.z) : 0.0;
-    if (fabs(off) > 1.0) atomicAdd(&scale->off, 1);
+    if (fabs(off) > 1.0) sum[6]++;
     split2(off * xs * xs, h, l);
     put(ch, j, h), put(cl, j, l);
     (j == 0 ? slot.x : slot.y) = real ? int(i) : -2;
@@ -150,7 +160,21 @@ __global__ void __launch_bounds__(128)
   r.zl = make_float2(p[0][2].z, p[1][2].z);
   r.gh = gh, r.gl = gl, r.ch = ch, r.cl = cl;
   r.slot = slot;
-  sp[k] = r;
+  if (k < npairs) sp[k] = r;
+  __shared__ int part_sum[4][kSplitSums];
+#pragma unroll
+  for (int q = 0; q < kSplitSums; ++q) {
+    const int v = __reduce_add_sync(0xffffffffu, sum[q]);
+    if ((threadIdx.x & 31) == 0) part_sum[threadIdx.x >> 5][q] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < kSplitSums) {
+    const int q = threadIdx.x;
+    long long v = 0;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) v += part_sum[w][q];
+    atomicAdd(&scale->sum[q], (unsigned long long)(v));
+  }
 }
 
 struct SplitBufs {
@@ -166,11 +190,11 @@ void launch(lpm_context& ctx, const NbodyPlan& p, const SplitBufs& b, const doub
   dim3 grid(unsigned(p.ntgt_pad / split_nt(WP)), unsigned(p.nchunks));
   if (p.skipc)
     nbody_split<WU, WP, true><<<grid, split_nt(WP), 0, ctx.stream>>>(
-        tgt, tself, b.st, b.sp, src, b.scale, p.ntgt, p.ntgt_pad, p.nsrc, p.nsrc_pad, p.chunk_len,
+        tgt, tself, b.st, b.sp, src, b.scale, ctx.f64_tab, p.ntgt, p.ntgt_pad, p.nsrc, p.nsrc_pad, p.chunk_len,
         eps * eps, part, ctx.d_err);
   else
     nbody_split<WU, WP, false><<<grid, split_nt(WP), 0, ctx.stream>>>(
-        tgt, tself, b.st, b.sp, src, b.scale, p.ntgt, p.ntgt_pad, p.nsrc, p.nsrc_pad, p.chunk_len,
+        tgt, tself, b.st, b.sp, src, b.scale, ctx.f64_tab, p.ntgt, p.ntgt_pad, p.nsrc, p.nsrc_pad, p.chunk_len,
         eps * eps, part, ctx.d_err);
   ctx.launches++;
 }
@@ -197,6 +221,7 @@ void launch_split(lpm_context& ctx, const NbodyPlan& p, const void* tgt_, const 
   const auto* tgt = static_cast<const double4_16a*>(tgt_);
   const auto* src = static_cast<const double4_16a*>(src_);
   char* w = static_cast<char*>(p.split_buf);
+  static_assert(sizeof(SplitScale) <= 256, "the scratch's first 256 bytes");
   SplitBufs b;
   b.scale = reinterpret_cast<SplitScale*>(w);
   b.range = reinterpret_cast<int4*>(w + 256);

@@ -25,8 +25,15 @@
 // mean error, which a sum of n like terms averages to 5.2e-15 sqrt(sum t^2) /
 // |sum t|; the FP64 kernel's sum carries the rounding of the running sum and
 // the cancellation in 1 - x.y (1e-16 / (1 - x.y) per pair, so the nearer a
-// pair the more the split form is ahead).  split_wanted() in direct_sum.cu
-// holds the source count from which the split sum's error is the smaller.
+// pair the more the split form is ahead: a target among the strong sources has
+// errors of 1e-12 to 1e-14 in FP64, 1e-15 here).  For targets far from all strong
+// sources FP64 is the better one where those are few (one: 7e-16 against 3e-15 of a
+// velocity, 100: 3e-16 and 4e-16, 300 and 1,000: equal) or a compact cluster of
+// both signs, whose sum t cancels (1e-15 against 5e-15).  So all pairs of an evaluation are
+// in FP64 (split_verdict; the device decides, no launch depends on it) if the effective number of its sources, (sum |g|)^2 /
+// sum g^2, is below 256, or if their mean direction, weighted by |g|, is longer than 1/2
+// (strengths within about a hemisphere) and (sum g)^2 / sum g^2 is below 256.
+// split_wanted() in direct_sum.cu holds the least sizes.
 // Pairs closer than 2^-20 of the domain, where the float pairs would run out
 // of bits, are evaluated in FP64 with the arithmetic of nbody_f64h.
 //
@@ -39,8 +46,8 @@
 // with |C| above it and |arg'| < (|C| - 1/32) / 32 are evaluated in FP64 one by
 // one (a run without reprojection drifts, and has stray points late on).
 // Targets of |1 - |x|^2| > 1 or far outside the sources' range take the FP64
-// path for all their pairs; all targets do when a sixteenth of the sources is
-// that far off the sphere or eps is far larger than the domain.
+// path for all their pairs; all targets do when a sixteenth of the
+// sources is that far off the sphere or eps is far larger than the domain.
 // Measured on one GB300 (SM clock 2,070 MHz), pair kernel alone, velocity:
 // icosahedral level 5 (10,242 x 20,480 pairs) 0.85 ms, 245 Gpairs/s, where 8 FP64
 // operations per pair take 2.7 ms.  Bound: the FP32 pipe: 163 instructions, mostly
@@ -74,12 +81,27 @@ struct __align__(16) SplitTarget {
 };
 static_assert(sizeof(SplitTarget) == 48, "three 16-byte loads per target");
 
-// Scales of one evaluation: |position|, eps < 2^e, |strength| < 2^g.  big != 0:
-// out of range, or eps dwarfs the domain: FP64 path.
+// Scales of one evaluation, and what its verdict goes by: |position|, eps < 2^e,
+// |strength| < 2^g.
 struct SplitScale {
-  int e, g, big;
-  int off;  // sources of |1 - |y|^2| > 1 (counted by the record kernel)
+  int e, g;
+  int big;  // out of range, or eps dwarfs the domain
+  int pad;
+  // of the sources' scaled strengths g in units of 2^-20 (g^2: 2^-24), two's complement
+  unsigned long long sum[7];  // |g|, g^2, g, |g| y (3); sources of |1 - |y|^2| > 1
 };
+
+// Whether every pair is evaluated in FP64.
+__device__ __forceinline__ bool split_verdict(const SplitScale& s, int64_t nsrc) {
+  constexpr float kLeast = 256.f;  // effective sources
+  auto v = [&](int q) { return float((long long)(s.sum[q])); };
+  const float A = v(0), Q = 65536.f * v(1), G = v(2);  // Q in the others' units squared
+  const float k = s.big ? 0.f : exp2f(float(s.e));
+  const float m0 = k * v(3), m1 = k * v(4), m2 = k * v(5);
+  const bool compact = m0 * m0 + m1 * m1 + m2 * m2 > 0.25f * A * A;
+  return s.big || s.sum[6] * 16 > (unsigned long long)(nsrc) || A * A < kLeast * Q ||
+         (compact && G * G < kLeast * Q);
+}
 
 // 2^k for |k| <= 1022
 __device__ __forceinline__ double pow2d(int k) {
@@ -246,6 +268,42 @@ __device__ __noinline__ void split_near64(const double4_16a* t, const double4_16
   split_pair64<WU, WP>(*t, *s, eps2, a);
 }
 
+// All pairs of one target and chunk with the operations of nbody_f64h, whose rate it
+// has (the FP64 pipe bounds it; the sources are uniform loads).  Out of line, called
+// before the split sums hold registers.
+template <bool WU, bool WP, bool SKIP>
+__device__ __noinline__ void split_fp64(const double4_16a* __restrict__ tgt,
+                                        const int* __restrict__ tself,
+                                        const double4_16a* __restrict__ src, int64_t ti, int64_t j0,
+                                        int64_t j1, double eps2, const F64Tables* __restrict__ tab,
+                                        double* __restrict__ out, int64_t ntgt_pad) {
+  constexpr int NC = (WU ? 3 : 0) + (WP ? 1 : 0);
+  const double4_16a t = tgt[ti];
+  const int self = SKIP ? tself[ti] : -1;
+  double a[NC];
+#pragma unroll
+  for (int k = 0; k < NC; ++k) a[k] = 0.0;
+#pragma unroll 2
+  for (int64_t j = j0; j < j1; ++j) {
+    const double4_16a s = src[j];
+    const double arg = eps2 - fma(t.z, s.z, fma(t.y, s.y, fma(t.x, s.x, -1.0)));
+    const bool skip = SKIP && j == self;
+    if (WU) {
+      const double q = f64_plain(fabs(arg)) ? s.w * f64_rcp(arg) : div_nr_any(s.w, arg);
+      const double g = skip ? 0.0 : q;
+      a[0] = fma(g, s.x, a[0]);
+      a[1] = fma(g, s.y, a[1]);
+      a[2] = fma(g, s.z, a[2]);
+    }
+    if (WP) {
+      const double l = fma(f64_ln(tab, arg), s.w, a[NC - 1]);
+      a[NC - 1] = skip ? a[NC - 1] : l;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NC; ++k) out[k * ntgt_pad + ti] = a[k];
+}
+
 //   tgt, tself, src, part: as nbody_f64h (sphere forms)
 //   st: SplitTarget per target (ntgt_pad entries)
 //   sp: SplitPair per two sources (nsrc_pad / 2 entries)
@@ -254,7 +312,8 @@ template <bool WU, bool WP, bool SKIP>
 __global__ void __launch_bounds__(split_nt(WP), 512 / split_nt(WP))
     nbody_split(const double4_16a* __restrict__ tgt, const int* __restrict__ tself,
                 const SplitTarget* __restrict__ st, const SplitPair* __restrict__ sp,
-                const double4_16a* __restrict__ src, const SplitScale* __restrict__ scale, int64_t ntgt, int64_t ntgt_pad,
+                const double4_16a* __restrict__ src, const SplitScale* __restrict__ scale,
+                const F64Tables* __restrict__ tab, int64_t ntgt, int64_t ntgt_pad,
                 int64_t nsrc, int64_t nsrc_pad, int chunk_len, double eps2,
                 double* __restrict__ part, int* err) {
   constexpr int NC = (WU ? 3 : 0) + (WP ? 1 : 0);
@@ -262,18 +321,23 @@ __global__ void __launch_bounds__(split_nt(WP), 512 / split_nt(WP))
   __shared__ __align__(8) uint64_t sbar[2];
   using Log = typename std::conditional<WP, SplitLog, float4>::type;
   __shared__ __align__(16) Log slog;
+  const SplitScale sc = *scale;
 
   const int64_t ti = (int64_t)blockIdx.x * split_nt(WP) + threadIdx.x;
   const int64_t s0 = (int64_t)blockIdx.y * chunk_len;
   int64_t slen = nsrc_pad - s0;
   if (slen > chunk_len) slen = chunk_len;
+  if (split_verdict(sc, nsrc)) {
+    split_fp64<WU, WP, SKIP>(tgt, tself, src, ti, s0, s0 + slen < nsrc ? s0 + slen : nsrc, eps2, tab,
+                             part + (int64_t)blockIdx.y * NC * ntgt_pad, ntgt_pad);
+    return;
+  }
   TilePipe<SplitPair, kSplitTile> pipe{sbuf, sbar, sp + s0 / 2, int(slen / (2 * kSplitTile))};
   pipe.start();
 
-  const SplitScale sc = *scale;
   const SplitTarget t = st[ti];
   const int self = SKIP ? tself[ti] : -1;
-  const bool exact = t.exact != 0 || (int64_t(sc.off) * 16 > nsrc && ti < ntgt);
+  const bool exact = t.exact != 0;
   // log(arg) = log(arg' 2^(2e)) - ln 2
   if constexpr (WP) split_log_tables(slog, 2 * sc.e - 1);
   const u64 XH = dup2(t.x.x), XM = dup2(t.x.y), XL = dup2(t.x.z);
