@@ -19,16 +19,21 @@ __device__ __forceinline__ int magnitude(double v) {
   const int h = __double2hiint(v) & 0x7fffffff;
   return h < 0x7ff00000 ? h : 0;
 }
+__device__ __forceinline__ bool not_finite(double v) {
+  return (__double2hiint(v) & 0x7fffffff) >= 0x7ff00000;
+}
 __device__ __forceinline__ int exponent_above(int h) {  // values of magnitude h: < 2^result
   return (h >> 20) - 1022;
 }
 
-// Per-CTA largest magnitudes: source coordinates, strengths, target coordinates.
+// Per-CTA largest magnitudes: source coordinates, strengths, target coordinates; and
+// whether a source is not finite (an infinity has no float pair).
 __global__ void __launch_bounds__(kRangeThreads)
     k_split_range(const double4_16a* __restrict__ tgt, int64_t nt,
                   const double4_16a* __restrict__ src, int64_t ns, int4* __restrict__ out,
                   SplitScale* __restrict__ scale) {
   __shared__ int sh[3];
+  bool bad = false;
   if (threadIdx.x < 3) sh[threadIdx.x] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) *scale = SplitScale{};
   __syncthreads();
@@ -40,6 +45,7 @@ __global__ void __launch_bounds__(kRangeThreads)
     const double4_16a p = src[i];
     ms = max(ms, max(magnitude(p.x), max(magnitude(p.y), magnitude(p.z))));
     mg = max(mg, magnitude(p.w));
+    bad |= not_finite(p.x) || not_finite(p.y) || not_finite(p.z) || not_finite(p.w);
   }
 #pragma unroll 4
   for (int64_t i = first; i < nt; i += step) {
@@ -54,17 +60,20 @@ __global__ void __launch_bounds__(kRangeThreads)
     atomicMax(&sh[1], mg);
     atomicMax(&sh[2], mt);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) out[blockIdx.x] = make_int4(sh[0], sh[1], sh[2], 0);
+  const int any_bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) out[blockIdx.x] = make_int4(sh[0], sh[1], sh[2], any_bad);
 }
 
 // Scales of the evaluation from the range kernel's partials (one warp).
 __device__ SplitScale split_scale(const int4* __restrict__ part, int nparts, double eps) {
   int ms = 0, mg = 0, mt = 0;
+  bool bad = false;
   for (int b = threadIdx.x; b < nparts; b += 32) {
     const int4 v = part[b];
     ms = max(ms, v.x), mg = max(mg, v.y), mt = max(mt, v.z);
+    bad |= v.w != 0;
   }
+  bad = __any_sync(0xffffffffu, bad);
   ms = __reduce_max_sync(0xffffffffu, ms);
   mg = __reduce_max_sync(0xffffffffu, mg);
   mt = __reduce_max_sync(0xffffffffu, mt);
@@ -73,9 +82,9 @@ __device__ SplitScale split_scale(const int4* __restrict__ part, int nparts, dou
   // (divided faces that ran away, say) take the FP64 path one by one
   const int es = exponent_above(ms), ep = exponent_above(magnitude(eps));
   const int ee = max(es, min(exponent_above(mt), es + 3));
-  s.e = ms > 0 ? max(ee, ep) : 0;  // no finite source position: every sum is NaN
+  s.e = ms > 0 ? max(ee, ep) : 0;
   s.g = mg > 0 ? exponent_above(mg) : 0;
-  if (s.e < -400 || s.e > 400 || abs(s.g) > 400 || ep > (ms > 0 ? ee : 0) + 8) {
+  if (bad || s.e < -400 || s.e > 400 || abs(s.g) > 400 || ep > (ms > 0 ? ee : 0) + 8) {
     s.big = 1;
     s.e = s.g = 0;
   }

@@ -85,7 +85,7 @@ static_assert(sizeof(SplitTarget) == 48, "three 16-byte loads per target");
 // |strength| < 2^g.
 struct SplitScale {
   int e, g;
-  int big;  // out of range, or eps dwarfs the domain
+  int big;  // out of range, not finite, or eps dwarfs the domain
   int pad;
   // of the sources' scaled strengths g in units of 2^-20 (g^2: 2^-24), two's complement
   unsigned long long sum[7];  // |g|, g^2, g, |g| y (3); sources of |1 - |y|^2| > 1

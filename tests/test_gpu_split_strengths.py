@@ -1,5 +1,6 @@
 """LPM_FP64 sphere sums over at least 1,024 sources whose strengths are not of like
-size and sign: a few strong ones seen from afar, a compact cluster of random signs.
+size and sign: a few strong ones seen from afar, a compact cluster of random signs,
+infinite and NaN strengths.
 
 A pair 90 degrees and more apart has 1 - x.y in [1, 2], formed by three roundings of
 at most 1.1e-16, its reciprocal and quotient two more: 5.5e-16 of the term.  The cross
@@ -80,3 +81,19 @@ def test_compact_cluster_of_random_signs(gpu_ctx, n):
     ur = _reference(x, y, g)[0]
     t2 = ((g / (1 - x @ y.T)) ** 2).sum(1)
     assert (np.abs(u - ur).max(1) <= 12 * 4e-16 * np.sqrt(t2) / (4 * np.pi)).all()
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("eps", [0.0, 0.1])
+def test_strength_not_finite(gpu_ctx, value, eps):
+    """As the same call with a few sources: infinite values stay infinite."""
+    y = _spread(1500)
+    g = np.full(1500, 0.01)
+    g[700] = value
+    x = _spread(1100)[:, [1, 2, 0]]
+    u, p = _sums(gpu_ctx, x, y, g, eps)
+    uf, pf = _sums(gpu_ctx, x, y[690:710], g[690:710], eps)
+    assert np.array_equal(np.isnan(p), np.isnan(pf))
+    assert np.array_equal(p[~np.isfinite(p)], pf[~np.isfinite(pf)], equal_nan=True)
+    assert np.array_equal(np.isnan(u), np.isnan(uf))
+    assert np.array_equal(u[np.isinf(u)], uf[np.isinf(uf)])
