@@ -66,8 +66,14 @@ constexpr int kSweNC = 11;
 
 struct __align__(16) SweSrc {
   double x, y, rot, pot, s, area;
-  int slot, pad[3];
+  int slot;
+  int wild;  // (s_y - s_x) A may not be finite
+  int pad[2];
 };
+// Not finite, or so large that a product of two such may not be.
+__device__ __forceinline__ bool swe_wild(double v) {
+  return (__double2hiint(v) & 0x7fffffff) >= (1023 + 500) << 20;
+}
 
 __global__ void k_swe_pack(View fx, const double* __restrict__ zeta, const double* __restrict__ sigma,
                            const double* __restrict__ area, const double* __restrict__ sfc,
@@ -83,7 +89,8 @@ __global__ void k_swe_pack(View fx, const double* __restrict__ zeta, const doubl
   r.s = sfc[j];
   r.area = area[j];
   r.slot = int(j);
-  r.pad[0] = r.pad[1] = r.pad[2] = 0;
+  r.wild = swe_wild(r.s) || swe_wild(r.area);
+  r.pad[0] = r.pad[1] = 0;
   src[k] = r;
 }
 // A pair's factors: e = d / R, e1^2 - e0^2, e0 e1, eps^2 / R^2 (1 / R^2 itself overflows
@@ -102,7 +109,7 @@ __device__ __noinline__ SwePair swe_pair_any(double d0, double d1, double epssq,
   v.xy = v.e0 * v.e1;
   v.ew = epssq * w * w;
   v.lg = log(R);
-  v.pse = p >= 746.0 ? 0.0 : fma(p, fma(p, fma(p, -2.0 / 3, 10.0), -40.0), 40.0) * exp(-p);
+  v.pse = p >= 746.0 && p < INFINITY ? 0.0 : fma(p, fma(p, fma(p, -2.0 / 3, 10.0), -40.0), 40.0) * exp(-p);
   return v;
 }
 
@@ -181,6 +188,7 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
   const bool valid = i < nt;
   const double x0 = valid ? tx(i, 0) : 0.0, x1 = valid ? tx(i, 1) : 0.0;
   const double si = valid ? ts[i] : 0.0;
+  const bool wild = swe_wild(si);
   const SweScales sc = swe_scales(epssq, ipse2);
   double r[kSweNC];
 #pragma unroll
@@ -207,7 +215,8 @@ __global__ void __launch_bounds__(kSweNT) k_swe_plane(View tx, const double* __r
       r[5] = fma(y.pot, v.md, r[5]);
       r[6] = fma(y.pot, v.xy, r[6]);
       r[7] = fma(y.pot, v.ew, r[7]);
-      if (v.pse != 0.0) r[8] = fma((y.s - si) * y.area, v.pse, r[8]);
+      // (0 times a value that is not finite is NaN)
+      if (v.pse != 0.0 || wild || y.wild) r[8] = fma((y.s - si) * y.area, v.pse, r[8]);
       r[9] = fma(y.rot, v.lg, r[9]);
       r[10] = fma(y.pot, v.lg, r[10]);
     }
