@@ -60,8 +60,7 @@ constexpr int kSweTile64 = 64;
 // the logarithm), everything between formed in integers beside them (swe_pair), against
 // about 260 for the reference's operation order with its eight divisions, square root
 // and library log and exp.  Quad level 5, vertices and faces: 19.6 ms in that order,
-// 4.73 ms as moments in FP64 (55 operations), 1.81 ms now (0.83 of the pipe's rate, 42 %
-// of the issue slots).
+// 4.73 ms as moments in FP64 (55 operations), 1.64 ms now (0.92 of the pipe's rate).
 constexpr int kSweNC = 11;
 
 struct __align__(16) SweSrc {
@@ -132,34 +131,40 @@ __device__ __forceinline__ SweScales swe_scales(double epssq, double ipse2) {
 }
 
 // In 64-bit fixed point: d over 2^(eE - 1085) for the larger exponent eE of d0, d1 and
-// eps, so that |d|^2, R = |d|^2 + eps^2 and the products keep 58 bits and more.  False
-// for values it does not take: sizes outside 2^-240 .. 2^240, d below 2^-9 eps (whose
-// last bits it would drop) but not 0, R beside 1.
+// eps, so that |d|^2, R = |d|^2 + eps^2 and e1^2 - e0^2 keep 58 bits and more; e0, e1
+// and their product from each component's own exponent, so that the smaller one loses
+// nothing.  False for values it does not take: sizes outside 2^-240 .. 2^240, d below
+// 2^-9 eps (whose last bits it would drop) but not 0, a component below 2^-200 of that
+// but not 0, R beside 1.
 __device__ __forceinline__ bool swe_pair(const F64Tables* __restrict__ tab, double d0, double d1,
                                          const SweScales& c, SwePair& v) {
   const unsigned h0 = unsigned(__double2hiint(d0)), h1 = unsigned(__double2hiint(d1));
   const int x0 = int(h0 >> 20 & 0x7ff), x1 = int(h1 >> 20 & 0x7ff), eb = max(x0, x1);
   const int eE = max(eb, c.ee);
-  const uint64_t D0 = (f64_mantissa(d0) << 10) >> min(eE - x0, 63);
-  const uint64_t D1 = (f64_mantissa(d1) << 10) >> min(eE - x1, 63);
+  const uint64_t F0 = x0 > 0 ? f64_mantissa(d0) << 10 : 0, F1 = x1 > 0 ? f64_mantissa(d1) << 10 : 0;
+  const int s0 = min(eE - x0, 63), s1 = min(eE - x1, 63);
+  const uint64_t D0 = F0 >> s0, D1 = F1 >> s1;
   const uint64_t S = __umul64hi(D0, D0) + __umul64hi(D1, D1);  // |d|^2
   const uint64_t Q = S + (c.e2 >> min(2 * eE - 1020 - c.e2x, 63));  // R = Q 2^(2 eE - 2106)
   const int zq = __clzll(int64_t(Q | 1));
   const int xr = 2 * eE - 1020 - zq;
   const double R = __longlong_as_double(int64_t(f64_pack(Q << zq, xr)));
-  if (unsigned(eE - 783) > 480u || (eE - eb > 9 && (d0 != 0.0 || d1 != 0.0)) || Q == 0 ||
-      !f64_log_plain(R))
+  const bool z0 = ((h0 << 1) | unsigned(__double2loint(d0))) == 0;
+  const bool z1 = ((h1 << 1) | unsigned(__double2loint(d1))) == 0;
+  if (unsigned(eE - 783) > 480u || (eE - eb > 9 && !(z0 && z1)) || (eE - x0 > 200 && !z0) ||
+      (eE - x1 > 200 && !z1) || Q == 0 || !f64_log_plain(R))
     return false;
   const uint64_t W = f64_rcp_mantissa(R);
   const int er = int(unsigned(__double2hiint(R)) >> 20);
-  const uint64_t E0 = __umul64hi(D0, W), E1 = __umul64hi(D1, W);  // |e| 2^(61 + er - eE)
+  const uint64_t E0 = __umul64hi(F0, W), E1 = __umul64hi(F1, W);  // |e| 2^(61 + er - x)
   const bool n0 = int(h0) < 0, n1 = int(h1) < 0;
-  const int ke = eE - 61 - er;
-  v.e0 = f64_value(E0, n0, ke);
-  v.e1 = f64_value(E1, n1, ke);
-  const int64_t md = int64_t(__umul64hi(2 * E1, 2 * E1)) - int64_t(__umul64hi(2 * E0, 2 * E0));
-  v.md = f64_value(uint64_t(md < 0 ? -md : md), md < 0, 2 * ke + 62);
-  v.xy = f64_value(__umul64hi(2 * E0, 2 * E1), n0 != n1, 2 * ke + 62);
+  const int k0 = x0 - 61 - er, k1 = x1 - 61 - er;
+  v.e0 = f64_value(E0, n0, k0);
+  v.e1 = f64_value(E1, n1, k1);
+  const uint64_t G0 = (2 * E0) >> s0, G1 = (2 * E1) >> s1;  // over the common exponent
+  const int64_t md = int64_t(__umul64hi(G1, G1)) - int64_t(__umul64hi(G0, G0));
+  v.md = f64_value(uint64_t(md < 0 ? -md : md), md < 0, 2 * (eE - 61 - er) + 62);
+  v.xy = f64_value(__umul64hi(2 * E0, 2 * E1), n0 != n1, k0 + k1 + 62);
   const int kw = c.e2x - 1086 + 2 * (1023 - er);
   v.ew = f64_value(kw < -1000 ? 0 : __umul64hi(__umul64hi(W, W) << 2, c.e2), false, kw);
   v.lg = f64_log(tab, R);
