@@ -141,6 +141,7 @@ int lpm_farfield_set_weights(lpm_farfield* ff, const float* w, const float* norm
   if (!ff || !w || !norm) return fail(LPM_ERR_ARG, "null argument");
   try {
     lpm::DeviceGuard device_guard(ff->ctx->device);
+    ff->image_current = false;
     ff->w.assign(w, w + lpm::kNParam);
     ff->norm.assign(norm, norm + LPM_FF_NNORM);
     ff->upload_net();

@@ -948,6 +948,7 @@ void ensure_net(lpm_farfield& ff) {
 
 void lpm_farfield::init_net(uint64_t seed) {
   using namespace lpm;
+  image_current = false;
   w.assign(kNParam, 0.f);
   std::mt19937_64 rng(seed);
   auto fill = [&](int off, int rows, int cols, int fan, int nrows_live, int bias_col) {
@@ -973,6 +974,7 @@ void lpm_farfield::init_net(uint64_t seed) {
 void lpm_farfield::upload_net() {
   using namespace lpm;
   ensure_net(*this);
+  image_current = false;
   float* dw = nullptr;
   LPM_CUDA(cudaMalloc(&dw, sizeof(float) * kNParam));
   cudaError_t e = cudaMemcpyAsync(dw, w.data(), sizeof(float) * kNParam, cudaMemcpyHostToDevice, ctx->stream);
@@ -985,6 +987,7 @@ void lpm_farfield::upload_net() {
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   cudaFree(dw);
   LPM_CUDA(e);
+  image_current = true;
 }
 
 namespace {
@@ -1155,6 +1158,7 @@ std::vector<float> lpm_farfield::train(const lpm::TrainCfg& cfg) {
   ctx->launches += 2;
   // ---- Adam ----------------------------------------------------------------
   upload_net();  // BF16 image of the initial weights, this normalisation
+  image_current = false;  // the steps advance it; w follows at the end
   float* wm = static_cast<float*>(tb.alloc(sizeof(float) * kNParam));
   float* mm = static_cast<float*>(tb.alloc(sizeof(float) * kNParam));
   float* vv = static_cast<float*>(tb.alloc(sizeof(float) * kNParam));
@@ -1213,6 +1217,7 @@ std::vector<float> lpm_farfield::train(const lpm::TrainCfg& cfg) {
   LPM_CUDA(cudaMemcpyAsync(net->norm, norm.data(), sizeof(float) * norm.size(), cudaMemcpyHostToDevice, st));
   LPM_CUDA(cudaStreamSynchronize(st));
   check_device_error(*ctx);
+  image_current = true;
   trained = true;
   return hist;
 }
@@ -1223,6 +1228,7 @@ void lpm_farfield::grad(const float* x_host, const float* y_host, int n, float* 
   set_train_attr();
   if (n < 128 || n % 128) throw Error(LPM_ERR_ARG, "grad check: n must be a positive multiple of 128");
   if (w.size() != size_t(kNParam)) throw Error(LPM_ERR_STATE, "grad check: no weights");
+  if (!image_current) upload_net();  // (a training run that failed half-way, say)
   cudaStream_t st = ctx->stream;
   // Workspace kept in the context's arena (no allocation per call): the rows as
   // they arrive and as the kernel reads them, the partial gradients of at most
@@ -1255,7 +1261,7 @@ void lpm_farfield::grad(const float* x_host, const float* y_host, int n, float* 
     a.pb = 0;
     a.row0 = int64_t(t0) * 128;
     a.inv_batch = 1.f / float(n);
-    a.wbf = net->wbf;  // the image of w: set_weights and training keep it current
+    a.wbf = net->wbf;
     a.gpart = gpart;
     a.lpart = lpart;
     a.err = ctx->d_err;
