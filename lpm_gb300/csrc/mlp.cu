@@ -1270,6 +1270,7 @@ void lpm_farfield::grad(const float* x_host, const float* y_host, int n, float* 
     ctx->launches += 2;
   }
   LPM_CUDA(cudaGetLastError());
+  check_device_error(*ctx);  // before the caller's array is written
   LPM_CUDA(cudaMemcpyAsync(g_host, gout, sizeof(float) * kNParam, cudaMemcpyDeviceToHost, st));
-  check_device_error(*ctx);  // synchronises the stream
+  LPM_CUDA(cudaStreamSynchronize(st));
 }
