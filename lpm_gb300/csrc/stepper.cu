@@ -544,6 +544,14 @@ int lpm_bve_rk4_kernel_shape(lpm_bve_rk4* st, int* threads, int* targets_per_thr
     *threads = k.nt;
     *targets_per_thread = k.r;
     *min_ctas_per_sm = k.minb;
+  } else if (st->plan.split) {
+    *threads = lpm::split_nt(st->plan.wp);
+    *targets_per_thread = 1;
+    *min_ctas_per_sm = 512 / *threads;
+  } else if (st->plan.fine) {
+    *threads = lpm::FINE_NT;
+    *targets_per_thread = 1;
+    *min_ctas_per_sm = 0;
   } else {
     *threads = lpm::F64_NT;
     *targets_per_thread = lpm::F64_R;
