@@ -236,9 +236,8 @@ int lpm_bve_rk4_advance_timestep(lpm_bve_rk4* st, lpm_view vx, double* vzeta,
 int lpm_bve_rk4_nbody_time(lpm_bve_rk4* st, double* ms, int64_t* launches);
 /* The N-body kernel shape the stepper runs: threads per CTA, targets per
  * thread and the CTAs per SM its register cap is set for (LPM_FP32C: the
- * chosen one of the six shapes; large LPM_FP64 sphere sums: 64 x 1, or 128 x 1
- * with a stream function, capped for 8 or 4 CTAs; other FP64 forms: 64 x 1 on
- * small grids, 128 x 2 on larger ones, 0 CTAs).
+ * chosen one of the six shapes; large LPM_FP64 sphere sums: 64 x 1, 8 CTAs;
+ * other FP64 forms: 64 x 1 on small grids, 128 x 2 on larger ones, 0 CTAs).
  * Valid after the first step (LPM_ERR_STATE before). */
 int lpm_bve_rk4_kernel_shape(lpm_bve_rk4* st, int* threads, int* targets_per_thread,
                              int* min_ctas_per_sm);

@@ -506,7 +506,7 @@ NbodyPlan plan_kind(lpm_context& ctx, int precision, int ndim, int form, bool wu
   const bool f32 = precision == LPM_FP32C;
   Fp64Shape s{F64_NT * F64_R, F64_TILE, f32 ? 4 : 0};
   if (f32) s = Fp64Shape{F32_TB, F32_TILE, 4};
-  else if (kind == FP64_SPLIT) s = Fp64Shape{split_nt(wp), SPLIT_TILE, 512 / split_nt(wp)};
+  else if (kind == FP64_SPLIT) s = Fp64Shape{SPLIT_NT, SPLIT_TILE, 512 / SPLIT_NT};
   else if (kind == FP64_FINE) s = Fp64Shape{FINE_NT, FINE_TILE, 4};
   else s.ctas = occupancy(precision);
   p.split = kind == FP64_SPLIT;

@@ -896,11 +896,10 @@ constexpr int F64_NT = 128, F64_R = 2, F64_TILE = 256;
 // thousand targets and sources still give every SM work (a warp's FP64
 // instruction takes 64 clocks of its SM sub-partition).
 constexpr int FINE_NT = 64, FINE_TILE = 8;
-// nbody_split: targets per CTA, sources per tile.  128 targets with the stream
-// function (a CTA copies the log tables), 64 without: icosahedral level 4's 7,682
-// targets leave 4,840 CTAs, four waves, where 128 leave 2,440, four waves and eight
-// CTAs (RK4 step 776 -> 740 us; with stream function 64 cost 1.4 %).
-__host__ __device__ constexpr int split_nt(bool wp) { return wp ? 128 : 64; }
+// nbody_split: targets per CTA, sources per tile.  64 targets: icosahedral level 4's
+// 7,682 leave 4,840 CTAs, four waves, where 128 leave 2,440, four waves and eight CTAs
+// (RK4 step 776 -> 740 us).
+constexpr int SPLIT_NT = 64;
 constexpr int SPLIT_TILE = 128;
 
 // FP32 kernel shapes: threads, targets per thread, minimum resident CTAs per

@@ -99,7 +99,8 @@ __global__ void __launch_bounds__(128)
     k_split_pack(const double4_16a* __restrict__ src, int64_t nsrc, int64_t npairs,
                  const double4_16a* __restrict__ tgt, int64_t ntgt, int64_t ntgt_pad, double eps,
                  const int4* __restrict__ part, int nparts, SplitPair* __restrict__ sp,
-                 SplitTarget* __restrict__ st, SplitScale* __restrict__ scale) {
+                 SplitTarget* __restrict__ st, SplitFixed* __restrict__ ps,
+                 SplitFixed* __restrict__ pt, SplitScale* __restrict__ scale) {
   __shared__ SplitScale sc;
   if (threadIdx.x < 32) {
     const SplitScale s = split_scale(part, nparts, eps);
@@ -123,6 +124,8 @@ __global__ void __launch_bounds__(128)
     r.exact = i < ntgt && (fabs(off) > 1.0 || fabs(x) >= 1.0 || fabs(y) >= 1.0 ||
                            fabs(z) >= 1.0);
     st[i] = r;
+    // (padding at the origin would be next to arg = 1, the logarithm's rare case)
+    if (pt) pt[i] = split_fixed(t, sc.e, i < ntgt ? off + 2.0 * eps * eps : 7.0, 0.0, r.exact != 0);
     return;
   }
   const int64_t k = int64_t(blockIdx.x) * 128 + threadIdx.x;
@@ -153,6 +156,8 @@ __global__ void __launch_bounds__(128)
     sum[5] += __float2int_rn(fabsf(h) * 0x1p20f * p[j][2].x);
     const double off = real ? unit_defect(s.x, s.y, s.z) : 0.0;
     if (fabs(off) > 1.0) sum[6]++;
+    // padding: a positive arg of no strength
+    if (ps && k < npairs) ps[i] = real ? split_fixed(s, sc.e, off, s.w, false) : SplitFixed{0, 0, 0, 1ll << 61};
     split2(off * xs * xs, h, l);
     put(ch, j, h), put(cl, j, l);
     (j == 0 ? slot.x : slot.y) = real ? int(i) : -2;
@@ -191,21 +196,25 @@ struct SplitBufs {
   SplitScale* scale;
   SplitTarget* st;
   SplitPair* sp;
+  SplitFixed *ps, *pt;  // nullptr: no stream function
 };
 
-template <bool WU, bool WP>
+template <bool SKIP>
 void launch(lpm_context& ctx, const NbodyPlan& p, const SplitBufs& b, const double4_16a* tgt,
             const int* tself, const double4_16a* src, double* part, double eps) {
-  dim3 grid(unsigned(p.ntgt_pad / split_nt(WP)), unsigned(p.nchunks));
-  if (p.skipc)
-    nbody_split<WU, WP, true><<<grid, split_nt(WP), 0, ctx.stream>>>(
-        tgt, tself, b.st, b.sp, src, b.scale, ctx.f64_tab, p.ntgt, p.ntgt_pad, p.nsrc, p.nsrc_pad, p.chunk_len,
-        eps * eps, part, ctx.d_err);
-  else
-    nbody_split<WU, WP, false><<<grid, split_nt(WP), 0, ctx.stream>>>(
-        tgt, tself, b.st, b.sp, src, b.scale, ctx.f64_tab, p.ntgt, p.ntgt_pad, p.nsrc, p.nsrc_pad, p.chunk_len,
-        eps * eps, part, ctx.d_err);
-  ctx.launches++;
+  const dim3 grid(unsigned(p.ntgt_pad / SPLIT_NT), unsigned(p.nchunks));
+  if (p.wu) {
+    nbody_split<SKIP><<<grid, SPLIT_NT, 0, ctx.stream>>>(
+        tgt, tself, b.st, b.sp, src, b.scale, p.ntgt, p.ntgt_pad, p.nsrc, p.nsrc_pad, p.chunk_len,
+        eps * eps, part, p.ncomp, ctx.d_err);
+    ctx.launches++;
+  }
+  if (p.wp) {
+    nbody_psi<SKIP><<<grid, SPLIT_NT, 0, ctx.stream>>>(tgt, tself, b.pt, b.ps, src, b.scale,
+                                                       ctx.f64_tab, p.ntgt_pad, p.nsrc_pad,
+                                                       p.chunk_len, eps * eps, part, p.ncomp);
+    ctx.launches++;
+  }
 }
 
 int range_blocks(const lpm_context& ctx, const NbodyPlan& p) {
@@ -221,8 +230,8 @@ size_t range_bytes(const lpm_context& ctx) {
 }  // namespace
 
 size_t split_bytes(const lpm_context& ctx, int64_t ntgt_pad, int64_t nsrc_pad) {
-  return 256 + range_bytes(ctx) + sizeof(SplitTarget) * size_t(ntgt_pad) +
-         sizeof(SplitPair) * size_t(nsrc_pad / 2);
+  return 256 + range_bytes(ctx) + (sizeof(SplitTarget) + sizeof(SplitFixed)) * size_t(ntgt_pad) +
+         (sizeof(SplitPair) / 2 + sizeof(SplitFixed)) * size_t(nsrc_pad);
 }
 
 void launch_split(lpm_context& ctx, const NbodyPlan& p, const void* tgt_, const int* tself,
@@ -236,18 +245,18 @@ void launch_split(lpm_context& ctx, const NbodyPlan& p, const void* tgt_, const 
   b.range = reinterpret_cast<int4*>(w + 256);
   b.st = reinterpret_cast<SplitTarget*>(w + 256 + range_bytes(ctx));
   b.sp = reinterpret_cast<SplitPair*>(b.st + p.ntgt_pad);  // ntgt_pad is a multiple of 64
+  b.ps = p.wp ? reinterpret_cast<SplitFixed*>(b.sp + p.nsrc_pad / 2) : nullptr;
+  b.pt = p.wp ? b.ps + p.nsrc_pad : nullptr;
   const int nb = range_blocks(ctx, p);
   k_split_range<<<nb, kRangeThreads, 0, ctx.stream>>>(tgt, p.ntgt, src, p.nsrc, b.range, b.scale);
   const int64_t npairs = p.nsrc_pad / 2;
   k_split_pack<<<unsigned((npairs + 127) / 128 + (p.ntgt_pad + 127) / 128), 128, 0, ctx.stream>>>(
-      src, p.nsrc, npairs, tgt, p.ntgt, p.ntgt_pad, eps, b.range, nb, b.sp, b.st, b.scale);
+      src, p.nsrc, npairs, tgt, p.ntgt, p.ntgt_pad, eps, b.range, nb, b.sp, b.st, b.ps, b.pt, b.scale);
   ctx.launches += 2;
-  if (p.wu && p.wp)
-    launch<true, true>(ctx, p, b, tgt, tself, src, part, eps);
-  else if (p.wu)
-    launch<true, false>(ctx, p, b, tgt, tself, src, part, eps);
+  if (p.skipc)
+    launch<true>(ctx, p, b, tgt, tself, src, part, eps);
   else
-    launch<false, true>(ctx, p, b, tgt, tself, src, part, eps);
+    launch<false>(ctx, p, b, tgt, tself, src, part, eps);
 }
 
 }  // namespace lpm

@@ -18,8 +18,7 @@
 //  * q = g / arg' as a float pair: MUFU reciprocal, one Newton step in FP32,
 //    one residual; then q d as float pairs.
 //  * Sums: float pairs over 4 steps, then three-float sums, then FP64 per chunk.
-//  * log(arg') (stream function): m 2^k = arg', 1/m from a 128-entry table,
-//    log1p by its series, all in float pairs.
+//  * The stream function in 64-bit fixed point (nbody_psi).
 //
 // A pair's term carries 5.2e-15 of random relative error (rms) and 1.3e-16 of
 // mean error, which a sum of n like terms averages to 5.2e-15 sqrt(sum t^2) /
@@ -54,8 +53,6 @@
 // f32x2 of two clocks each, per step of two sources fill 99 % of its clocks there.
 #pragma once
 
-#include <type_traits>
-
 #include "f32x2.cuh"
 #include "nbody.cuh"
 
@@ -71,6 +68,16 @@ static_assert(sizeof(SplitPair) == 112, "seven 16-byte loads per pair of sources
 
 constexpr int kSplitTile = SPLIT_TILE / 2;  // pairs of sources per tile
 constexpr float kSplitTiny = 9.094947e-13f;  // 2^-40: a pair's least scaled arg'
+
+// One point of the stream function: scaled position in units of 2^-61; its defect
+// (targets: plus 2 eps^2) in units of 2^-58, with 32 bits after the point; strength
+// (sources); whether a target lies outside the scaled range.
+struct __align__(16) SplitFixed {
+  long long x, y, z, c;
+  double g;
+  unsigned lo;
+  int exact;
+};
 
 // One target: its three-float position, the constant part of arg' (its defect
 // and 2 eps^2) and whether it lies outside the scaled range (the FP64 path).
@@ -137,6 +144,13 @@ __device__ __forceinline__ double unit_defect(double x, double y, double z) {
   return s + e;
 }
 
+__device__ __forceinline__ SplitFixed split_fixed(const double4_16a& p, int e, double off, double g,
+                                                  bool exact) {
+  const double k = pow2d(61 - e), c = off * pow2d(58 - 2 * e), f = floor(c);
+  return SplitFixed{__double2ll_rn(p.x * k), __double2ll_rn(p.y * k), __double2ll_rn(p.z * k),
+                    (long long)(f), g, unsigned((c - f) * 0x1p32), exact};
+}
+
 __device__ __forceinline__ void two_sum2(u64 a, u64 b, u64& s, u64& e) {
   s = add2(a, b);
   const u64 bb = sub2(s, a);
@@ -180,156 +194,182 @@ struct SplitAcc {
   __device__ __forceinline__ double value() const { return double(t0) + (double(t1) + double(t2)); }
 };
 
-// log tables: reciprocal f of the interval centre, -log f as a float pair
-// (less ln 2 from sqrt 2 on, where the exponent is one higher); k ln 2 pairs.
-struct SplitLog {
-  float4 m[128];   // f, hi, lo, -
-  float4 k[64];    // (k + offset) ln 2 in three parts for k = -41 .. 22
-};
-constexpr int kSplitLogK0 = -41;
-constexpr int kSplitLogUp = 53;  // intervals from here on lie above sqrt 2
-
-__device__ __forceinline__ void split_log_tables(SplitLog& T, int offset) {
-  for (int i = threadIdx.x; i < 128; i += blockDim.x) {
-    const float f = __frcp_rn(1.f + (float(i) + 0.5f) * (1.f / 128));
-    const double ln2 = 0.69314718055994530942;
-    float h, l;
-    split2(-log(double(f)) - (i >= kSplitLogUp ? ln2 : 0.0), h, l);
-    T.m[i] = make_float4(f, h, l, 0.f);
-  }
-  for (int i = threadIdx.x; i < 64; i += blockDim.x) {
-    const double v = double(i + kSplitLogK0 + offset) * 0.69314718055994530942;
-    float h, l;
-    split2(v, h, l);
-    T.k[i] = make_float4(h, l, float((v - double(h)) - double(l)), 0.f);
-  }
-}
-
-// log(a + al) + offset ln 2 of two values in [2^-40, 2^21] as float pairs.
-__device__ __forceinline__ void split_log2v(const SplitLog& T, u64 a, u64 al, u64& lh, u64& ll) {
-  float a0, a1;
-  upk2(a, a0, a1);
-  const unsigned b0 = __float_as_uint(a0), b1 = __float_as_uint(a1);
-  const int i0 = (b0 >> 16) & 127, i1 = (b1 >> 16) & 127;
-  const float4 e0 = T.m[i0], e1 = T.m[i1];
-  // indexes are kept in range for values outside [2^-40, 2^21] (marked targets)
-  const int x0 = min(max(int(b0 >> 23) - 127 + (i0 >= kSplitLogUp ? 1 : 0) - kSplitLogK0, 0), 63);
-  const int x1 = min(max(int(b1 >> 23) - 127 + (i1 >= kSplitLogUp ? 1 : 0) - kSplitLogK0, 0), 63);
-  const float4 k0 = T.k[x0], k1 = T.k[x1];
-  const u64 m = pk2(__uint_as_float((b0 & 0x7fffffu) | 0x3f800000u),
-                    __uint_as_float((b1 & 0x7fffffu) | 0x3f800000u));
-  const u64 sc = pk2(__uint_as_float(0x7f000000u - (b0 & 0x7f800000u)),
-                     __uint_as_float(0x7f000000u - (b1 & 0x7f800000u)));
-  const u64 f = pk2(e0.x, e1.x);
-  const u64 ml = mul2(al, sc);
-  // t = (m + ml) f - 1, |t| < 2^-7.9
-  const u64 p = mul2(m, f);
-  u64 tl = fma2(ml, f, fma2(m, f, neg2(p)));
-  const u64 t1 = sub2(p, dup2(1.f));
-  const u64 th = add2(t1, tl);
-  tl = sub2(tl, sub2(th, t1));
-  // log1p: th + tl - th^2/2 - th tl + t^3 (1/3 - t/4 + t^2/5 - t^3/6)
-  const u64 nhalf = dup2(-0.5f);
-  const u64 sq = mul2(th, th);
-  const u64 se = fma2(th, th, neg2(sq));
-  u64 P = fma2(th, dup2(-1.f / 6), dup2(0.2f));
-  P = fma2(th, P, dup2(-0.25f));
-  P = fma2(th, P, dup2(1.f / 3));
-  const u64 hs = mul2(sq, nhalf);
-  const u64 r = add2(th, hs);           // |hs| < |th|
-  u64 lo = sub2(hs, sub2(r, th));
-  lo = fma2(se, nhalf, lo);
-  lo = fma2(mul2(sq, th), P, lo);
-  lo = add2(lo, fma2(neg2(th), tl, tl));
-  u64 s, e;
-  two_sum2(pk2(k0.x, k1.x), pk2(e0.y, e1.y), s, e);
-  lo = add2(add2(lo, pk2(k0.z, k1.z)), add2(e, add2(pk2(k0.y, k1.y), pk2(e0.z, e1.z))));
-  two_sum2(s, r, lh, e);
-  ll = add2(lo, e);
-}
-
 // One pair in FP64, the arithmetic of nbody_f64h, added to its partials.
-template <bool WU, bool WP>
 __device__ __forceinline__ void split_pair64(const double4_16a& t, const double4_16a& s,
                                              double eps2, double* a) {
   const double arg = eps2 - fma(t.z, s.z, fma(t.y, s.y, fma(t.x, s.x, -1.0)));
-  if (WU) {
-    const double q = div_nr(s.w, arg);
-    a[0] = fma(q, s.x, a[0]);
-    a[1] = fma(q, s.y, a[1]);
-    a[2] = fma(q, s.z, a[2]);
-  }
-  if (WP) a[WU ? 3 : 0] = fma(log(arg), s.w, a[WU ? 3 : 0]);
+  const double q = div_nr(s.w, arg);
+  a[0] = fma(q, s.x, a[0]);
+  a[1] = fma(q, s.y, a[1]);
+  a[2] = fma(q, s.z, a[2]);
 }
-// The rare pair of the split loop, out of line.
-template <bool WU, bool WP>
-__device__ __noinline__ void split_near64(const double4_16a* t, const double4_16a* s, double eps2,
-                                          double* a) {
-  split_pair64<WU, WP>(*t, *s, eps2, a);
+// The rare pair, out of line.
+static __device__ __noinline__ void split_near64(const double4_16a* t, const double4_16a* s,
+                                                 double eps2, double* a) {
+  split_pair64(*t, *s, eps2, a);
 }
 
 // All pairs of one target and chunk with the operations of nbody_f64h, whose rate it
 // has (the FP64 pipe bounds it; the sources are uniform loads).  Out of line, called
 // before the split sums hold registers.
-template <bool WU, bool WP, bool SKIP>
+template <bool SKIP>
 __device__ __noinline__ void split_fp64(const double4_16a* __restrict__ tgt,
                                         const int* __restrict__ tself,
                                         const double4_16a* __restrict__ src, int64_t ti, int64_t j0,
-                                        int64_t j1, double eps2, const F64Tables* __restrict__ tab,
-                                        double* __restrict__ out, int64_t ntgt_pad) {
-  constexpr int NC = (WU ? 3 : 0) + (WP ? 1 : 0);
+                                        int64_t j1, double eps2, double* __restrict__ out,
+                                        int64_t ntgt_pad) {
   const double4_16a t = tgt[ti];
   const int self = SKIP ? tself[ti] : -1;
-  double a[NC];
-#pragma unroll
-  for (int k = 0; k < NC; ++k) a[k] = 0.0;
+  double a[3] = {0.0, 0.0, 0.0};
 #pragma unroll 2
   for (int64_t j = j0; j < j1; ++j) {
     const double4_16a s = src[j];
     const double arg = eps2 - fma(t.z, s.z, fma(t.y, s.y, fma(t.x, s.x, -1.0)));
     const bool skip = SKIP && j == self;
-    if (WU) {
-      const double q = f64_plain(fabs(arg)) ? s.w * f64_rcp(arg) : div_nr_any(s.w, arg);
-      const double g = skip ? 0.0 : q;
-      a[0] = fma(g, s.x, a[0]);
-      a[1] = fma(g, s.y, a[1]);
-      a[2] = fma(g, s.z, a[2]);
-    }
-    if (WP) {
-      const double l = fma(f64_ln(tab, arg), s.w, a[NC - 1]);
-      a[NC - 1] = skip ? a[NC - 1] : l;
-    }
+    const double q = f64_plain(fabs(arg)) ? s.w * f64_rcp(arg) : div_nr_any(s.w, arg);
+    const double g = skip ? 0.0 : q;
+    a[0] = fma(g, s.x, a[0]);
+    a[1] = fma(g, s.y, a[1]);
+    a[2] = fma(g, s.z, a[2]);
   }
 #pragma unroll
-  for (int k = 0; k < NC; ++k) out[k * ntgt_pad + ti] = a[k];
+  for (int k = 0; k < 3; ++k) out[k * ntgt_pad + ti] = a[k];
 }
 
+// ---- the stream function --------------------------------------------------------
+// |d|^2 in units of 2^-58 (to about one).  The squares from 32-bit halves, D = h 2^32 + l
+// with signed h and l: h^2 + 2 h l / 2^32, without l^2.
+__device__ __forceinline__ long long split_square(const long long (&d)[3]) {
+  long long T = 0, c = 0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int l = int(unsigned(d[k])), h = int(d[k] >> 32) + (l < 0);
+    T += (long long)(h) * h;
+    c += (long long)(h) * l;
+  }
+  return T + (c >> 31);
+}
+// arg = T 2^(e2 - 59) as a double, T > 0.
+__device__ __forceinline__ double split_arg_value(long long T, int e2) {
+  const int z = __clzll(T);
+  return __longlong_as_double(int64_t(f64_pack(uint64_t(T) << z, 1023 + 63 - z + e2 - 59)));
+}
+// Sums below this (arg < 1e-6 on the unit sphere) keep too few bits; above, arg' is good
+// to about 1.4e-17, where 1 - x.y in FP64 has 1e-16.
+constexpr long long kPsiClose = 1ll << 37;
+// arg in FP64: with ref (what the fixed point does not hold) as nbody_f64h, else from
+// |d|^2, for pairs within about 1e-6.
+static __device__ __noinline__ double split_arg64(const double4_16a* t, const double4_16a* s,
+                                                  double eps2, bool ref) {
+  if (ref) return eps2 - fma(t->z, s->z, fma(t->y, s->y, fma(t->x, s->x, -1.0)));
+  const double d0 = t->x - s->x, d1 = t->y - s->y, d2 = t->z - s->z;
+  const double c = unit_defect(t->x, t->y, t->z) + unit_defect(s->x, s->y, s->z) + 2.0 * eps2;
+  return 0.5 * (fma(d0, d0, fma(d1, d1, d2 * d2)) + c);
+}
+// Any pair's arg.  A close one's d is taken k bits up, C from its bits after the point.
+static __device__ __noinline__ double split_arg_any(long long d0, long long d1, long long d2,
+                                                    long long C, unsigned lo, int e,
+                                                    const double4_16a* t, const double4_16a* s,
+                                                    double eps2, bool ref) {
+  if (!ref) {
+    long long d[3] = {d0, d1, d2};
+    const long long m = llabs(d0) | llabs(d1) | llabs(d2);
+    const int k = max(0, min(min(__clzll(m) - 2, (__clzll(llabs(C) | 1) - 3) / 2), 16));
+#pragma unroll
+    for (int q = 0; q < 3; ++q) d[q] *= 1ll << k;
+    const long long T = split_square(d) + C * (1ll << (2 * k)) + (long long)(((unsigned long long)(lo) << (2 * k)) >> 32);
+    if (T >= kPsiClose) return split_arg_value(T, 2 * (e - k));
+  }
+  return split_arg64(t, s, eps2, ref);
+}
+
+// Partials of the stream function, sum g log(arg): a logarithm carries arg's relative
+// error as an absolute one, and far pairs weigh as much as near ones, so float pairs
+// (5e-15 a pair) were 1.5 to 4 times further off than nbody_f64h on meshes of 1,280 to
+// 6,144 sources.  Here arg is exact to 53 bits (no cancellation of 1 - x.y), formed in
+// integers as its logarithm is (f64math.cuh): 3 FP64 operations per pair.  A kernel of
+// its own: beside the float-pair velocity its registers left 16 warps per SM, which do
+// not hide its chains of operations (velocity and stream function, 14,336 targets by
+// 6,144 sources: 1.35 ms in one kernel, 1.08 ms in two, 2.46 ms as nbody_f64h, 0.75 ms
+// in float pairs).  Bound: the FP64 pipe, 0.80 of its rate.
+//   pt, ps: SplitFixed per target and source, ntgt_pad and nsrc_pad of them
+//   part: [chunk][nc][ntgt_pad], the last component
+template <bool SKIP>
+__global__ void __launch_bounds__(SPLIT_NT, 16)
+    nbody_psi(const double4_16a* __restrict__ tgt, const int* __restrict__ tself,
+              const SplitFixed* __restrict__ pt, const SplitFixed* __restrict__ ps,
+              const double4_16a* __restrict__ src, const SplitScale* __restrict__ scale,
+              const F64Tables* __restrict__ tab, int64_t ntgt_pad, int64_t nsrc_pad, int chunk_len,
+              double eps2, double* __restrict__ part, int nc) {
+  const int64_t ti = (int64_t)blockIdx.x * SPLIT_NT + threadIdx.x;
+  const int64_t s0 = (int64_t)blockIdx.y * chunk_len;
+  const int64_t s1 = s0 + chunk_len < nsrc_pad ? s0 + chunk_len : nsrc_pad;
+  const int e = scale->e;
+  const SplitFixed x = pt[ti];
+  const bool ref = scale->big != 0 || x.exact != 0;
+  const int self = SKIP ? tself[ti] : -1;
+  double sum = 0.0;
+  for (int64_t i0 = s0; i0 < s1; i0 += SPLIT_TILE) {
+    double run = 0.0;
+#pragma unroll 1
+    for (int64_t i = i0; i < i0 + SPLIT_TILE; i += 2) {
+      // (two sources' chains side by side)
+      const SplitFixed y0 = ps[i], y1 = ps[i + 1];
+      const long long d0[3] = {x.x - y0.x, x.y - y0.y, x.z - y0.z};
+      const long long d1[3] = {x.x - y1.x, x.y - y1.y, x.z - y1.z};
+      // (a target's own source: any argument of the common path, left out below)
+      const bool own0 = SKIP && i == self, own1 = SKIP && i + 1 == self;
+      const long long T0 = own0 ? 1ll << 58 : split_square(d0) + (x.c + y0.c);
+      const long long T1 = own1 ? 1ll << 58 : split_square(d1) + (x.c + y1.c);
+      double a0 = split_arg_value(T0, 2 * e), a1 = split_arg_value(T1, 2 * e);
+      if (ref || T0 < kPsiClose || T1 < kPsiClose) {
+        const unsigned l0 = x.lo + y0.lo, l1 = x.lo + y1.lo;
+        if (!own0)
+          a0 = split_arg_any(d0[0], d0[1], d0[2], x.c + y0.c + (l0 < x.lo), l0, e, tgt + ti, src + i,
+                             eps2, ref);
+        if (!own1)
+          a1 = split_arg_any(d1[0], d1[1], d1[2], x.c + y1.c + (l1 < x.lo), l1, e, tgt + ti,
+                             src + i + 1, eps2, ref);
+      }
+      double v0, v1;
+      if (f64_log_plain(a0) && f64_log_plain(a1)) {
+        v0 = f64_log(tab, a0), v1 = f64_log(tab, a1);
+      } else {
+        v0 = f64_ln_any(a0), v1 = f64_ln_any(a1);
+      }
+      if (!own0) run = fma(v0, y0.g, run);
+      if (!own1) run = fma(v1, y1.g, run);
+    }
+    sum += run;
+  }
+  part[((int64_t)blockIdx.y * nc + nc - 1) * ntgt_pad + ti] = sum;
+}
+
+// ---- the velocity ---------------------------------------------------------------
 //   tgt, tself, src, part: as nbody_f64h (sphere forms)
 //   st: SplitTarget per target (ntgt_pad entries)
 //   sp: SplitPair per two sources (nsrc_pad / 2 entries)
 //   SKIP: the pair of tself is left out
-template <bool WU, bool WP, bool SKIP>
-__global__ void __launch_bounds__(split_nt(WP), 512 / split_nt(WP))
+//   nc: components of the partials, the velocity's first
+template <bool SKIP>
+__global__ void __launch_bounds__(SPLIT_NT, 512 / SPLIT_NT)
     nbody_split(const double4_16a* __restrict__ tgt, const int* __restrict__ tself,
                 const SplitTarget* __restrict__ st, const SplitPair* __restrict__ sp,
                 const double4_16a* __restrict__ src, const SplitScale* __restrict__ scale,
-                const F64Tables* __restrict__ tab, int64_t ntgt, int64_t ntgt_pad,
-                int64_t nsrc, int64_t nsrc_pad, int chunk_len, double eps2,
-                double* __restrict__ part, int* err) {
-  constexpr int NC = (WU ? 3 : 0) + (WP ? 1 : 0);
+                int64_t ntgt, int64_t ntgt_pad, int64_t nsrc, int64_t nsrc_pad, int chunk_len,
+                double eps2, double* __restrict__ part, int nc, int* err) {
+  constexpr int NC = 3;
   __shared__ __align__(128) SplitPair sbuf[2 * kSplitTile];
   __shared__ __align__(8) uint64_t sbar[2];
-  using Log = typename std::conditional<WP, SplitLog, float4>::type;
-  __shared__ __align__(16) Log slog;
   const SplitScale sc = *scale;
 
-  const int64_t ti = (int64_t)blockIdx.x * split_nt(WP) + threadIdx.x;
+  const int64_t ti = (int64_t)blockIdx.x * SPLIT_NT + threadIdx.x;
   const int64_t s0 = (int64_t)blockIdx.y * chunk_len;
   int64_t slen = nsrc_pad - s0;
   if (slen > chunk_len) slen = chunk_len;
   if (split_verdict(sc, nsrc)) {
-    split_fp64<WU, WP, SKIP>(tgt, tself, src, ti, s0, s0 + slen < nsrc ? s0 + slen : nsrc, eps2, tab,
-                             part + (int64_t)blockIdx.y * NC * ntgt_pad, ntgt_pad);
+    split_fp64<SKIP>(tgt, tself, src, ti, s0, s0 + slen < nsrc ? s0 + slen : nsrc, eps2,
+                     part + (int64_t)blockIdx.y * nc * ntgt_pad, ntgt_pad);
     return;
   }
   TilePipe<SplitPair, kSplitTile> pipe{sbuf, sbar, sp + s0 / 2, int(slen / (2 * kSplitTile))};
@@ -338,14 +378,12 @@ __global__ void __launch_bounds__(split_nt(WP), 512 / split_nt(WP))
   const SplitTarget t = st[ti];
   const int self = SKIP ? tself[ti] : -1;
   const bool exact = t.exact != 0;
-  // log(arg) = log(arg' 2^(2e)) - ln 2
-  if constexpr (WP) split_log_tables(slog, 2 * sc.e - 1);
   const u64 XH = dup2(t.x.x), XM = dup2(t.x.y), XL = dup2(t.x.z);
   const u64 YH = dup2(t.y.x), YM = dup2(t.y.y), YL = dup2(t.y.z);
   const u64 ZH = dup2(t.z.x), ZM = dup2(t.z.y), ZL = dup2(t.z.z);
   const u64 CH = dup2(t.ch), CL = dup2(t.cl);
-  SplitAcc acc[NC];
-  double near[NC];  // the pairs evaluated in FP64, in the partials' units
+  SplitAcc acc[3];
+  double near[NC];  // what is evaluated in FP64, in the partials' units
 #pragma unroll
   for (int k = 0; k < NC; ++k) near[k] = 0.0;
   // -1/1024 in the scale of arg'; padding targets take out nothing
@@ -356,7 +394,6 @@ __global__ void __launch_bounds__(split_nt(WP), 512 / split_nt(WP))
   // (a warp whose targets all do, or are padding, still passes its tiles, without
   // the sums)
   const bool idle = __all_sync(0xffffffffu, exact || ti >= ntgt);
-  __syncthreads();  // the tables
   for (int tl = 0; tl < pipe.ntiles; ++tl) {
     if (!pipe.acquire(tl)) {
       pipe.drain(tl, err);
@@ -405,22 +442,19 @@ __global__ void __launch_bounds__(split_nt(WP), 512 / split_nt(WP))
         float a0, a1;
         upk2(A, a0, a1);
         // pairs taken out (rare): the closest and those off the sphere,
-        // evaluated in FP64 (with a logarithm also those of a negative arg',
-        // which has none), and the target's own source
+        // evaluated in FP64, and the target's own source
         float c0, c1;
         upk2(c, c0, c1);
-        bool n0 = (WP ? a0 : fabsf(a0)) < fmaxf(tiny, fmaf(fabsf(c0), 1.f / 32, off));
-        bool n1 = (WP ? a1 : fabsf(a1)) < fmaxf(tiny, fmaf(fabsf(c1), 1.f / 32, off));
-        if (SKIP) {
-          n0 |= s.slot.x == self;
-          n1 |= s.slot.y == self;
-        }
+        const bool n0 = fabsf(a0) < fmaxf(tiny, fmaf(fabsf(c0), 1.f / 32, off)) ||
+                        (SKIP && s.slot.x == self);
+        const bool n1 = fabsf(a1) < fmaxf(tiny, fmaf(fabsf(c1), 1.f / 32, off)) ||
+                        (SKIP && s.slot.y == self);
         u64 gh = pkf2(s.gh), gl = pkf2(s.gl);
         if (n0 || n1) {
           if (n0 && s.slot.x >= 0 && !(SKIP && s.slot.x == self))
-            split_near64<WU, WP>(tgt + ti, src + s.slot.x, eps2, near);
+            split_near64(tgt + ti, src + s.slot.x, eps2, near);
           if (n1 && s.slot.y >= 0 && !(SKIP && s.slot.y == self))
-            split_near64<WU, WP>(tgt + ti, src + s.slot.y, eps2, near);
+            split_near64(tgt + ti, src + s.slot.y, eps2, near);
           // strength 0 and denominator 1 in the split sum
           float b0, b1;
           upk2(Al, b0, b1);
@@ -431,43 +465,32 @@ __global__ void __launch_bounds__(split_nt(WP), 512 / split_nt(WP))
           gh = pk2(n0 ? 0.f : s.gh.x, n1 ? 0.f : s.gh.y);
           gl = pk2(n0 ? 0.f : s.gl.x, n1 ? 0.f : s.gl.y);
         }
-        if (WU) {
-          // r = -1 / arg': the MUFU's value, one Newton step, its residual
-          u64 r = pk2(rcp_approx(-a0), rcp_approx(-a1));
-          r = fma2(r, fma2(A, r, one), r);
-          e = fma2(Al, r, fma2(A, r, one));
-          const u64 rl = mul2(r, fma2(e, e, e));
-          // the record holds -g: q = g / arg'
-          const u64 qh = mul2(gh, r);
-          u64 ql = fma2(gh, r, neg2(qh));
-          ql = fma2(gh, rl, ql);
-          ql = fma2(gl, r, ql);
+        // r = -1 / arg': the MUFU's value, one Newton step, its residual
+        u64 r = pk2(rcp_approx(-a0), rcp_approx(-a1));
+        r = fma2(r, fma2(A, r, one), r);
+        e = fma2(Al, r, fma2(A, r, one));
+        const u64 rl = mul2(r, fma2(e, e, e));
+        // the record holds -g: q = g / arg'
+        const u64 qh = mul2(gh, r);
+        u64 ql = fma2(gh, r, neg2(qh));
+        ql = fma2(gh, rl, ql);
+        ql = fma2(gl, r, ql);
 #pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const u64 ph = mul2(qh, dh[k]);
-            u64 pl = fma2(qh, dh[k], neg2(ph));
-            pl = fma2(ql, dl[k], fma2(qh, dl[k], pl));
-            pl = fma2(ql, dh[k], pl);
-            acc[k].add(ph, pl);
-          }
-        }
-        if constexpr (WP) {
-          u64 lh, ll;
-          split_log2v(slog, A, Al, lh, ll);
-          const u64 ph = mul2(gh, lh);
-          u64 pl = fma2(gh, lh, neg2(ph));
-          pl = fma2(gh, ll, pl);
-          pl = fma2(gl, lh, pl);
-          acc[NC - 1].add(ph, pl);
+        for (int k = 0; k < 3; ++k) {
+          const u64 ph = mul2(qh, dh[k]);
+          u64 pl = fma2(qh, dh[k], neg2(ph));
+          pl = fma2(ql, dl[k], fma2(qh, dl[k], pl));
+          pl = fma2(ql, dh[k], pl);
+          acc[k].add(ph, pl);
         }
       }
 #pragma unroll
-      for (int c = 0; c < NC; ++c) acc[c].merge();
+      for (int c = 0; c < 3; ++c) acc[c].merge();
     }
     pipe.release(tl);
   }
 
-  double* out = part + (int64_t)blockIdx.y * NC * ntgt_pad;
+  double* out = part + (int64_t)blockIdx.y * nc * ntgt_pad;
   const unsigned lanes = __ballot_sync(0xffffffffu, exact);
   if (lanes != 0) {
     // FP64 targets: each by its own thread where they fill half the warp, one
@@ -487,7 +510,7 @@ __global__ void __launch_bounds__(split_nt(WP), 512 / split_nt(WP))
 #pragma unroll 2
         for (int64_t j = s0 + (own ? 0 : lane); j < j1; j += own ? 1 : 32) {
           const double4_16a y = src[j];
-          if (!(SKIP && j == sb)) split_pair64<WU, WP>(x, y, eps2, a);
+          if (!(SKIP && j == sb)) split_pair64(x, y, eps2, a);
         }
       }
       if (!own) {
@@ -504,12 +527,9 @@ __global__ void __launch_bounds__(split_nt(WP), 512 / split_nt(WP))
   if (!exact) {
     // the sum of g d / arg' in the caller's units; -2 times it equals the sum
     // of (g / arg) y in the cross product with x
-    if (WU) {
-      const double f = -2.0 * pow2d(sc.g - sc.e);
+    const double f = -2.0 * pow2d(sc.g - sc.e);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) near[k] += acc[k].value() * f;
-    }
-    if (WP) near[NC - 1] -= acc[NC - 1].value() * pow2d(sc.g);  // the records hold -g
+    for (int k = 0; k < 3; ++k) near[k] += acc[k].value() * f;
 #pragma unroll
     for (int k = 0; k < NC; ++k) out[k * ntgt_pad + ti] = near[k];
   }

@@ -545,7 +545,7 @@ int lpm_bve_rk4_kernel_shape(lpm_bve_rk4* st, int* threads, int* targets_per_thr
     *targets_per_thread = k.r;
     *min_ctas_per_sm = k.minb;
   } else if (st->plan.split) {
-    *threads = lpm::split_nt(st->plan.wp);
+    *threads = lpm::SPLIT_NT;
     *targets_per_thread = 1;
     *min_ctas_per_sm = 512 / *threads;
   } else if (st->plan.fine) {
