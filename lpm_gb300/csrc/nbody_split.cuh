@@ -29,9 +29,14 @@
 // sources FP64 is the better one where those are few (one: 7e-16 against 3e-15 of a
 // velocity, 100: 3e-16 and 4e-16, 300 and 1,000: equal) or a compact cluster of
 // both signs, whose sum t cancels (1e-15 against 5e-15).  So all pairs of an evaluation are
-// in FP64 (split_verdict; the device decides, no launch depends on it) if the effective number of its sources, (sum |g|)^2 /
-// sum g^2, is below 256, or if their mean direction, weighted by |g|, is longer than 1/2
-// (strengths within about a hemisphere) and (sum g)^2 / sum g^2 is below 256.
+// in FP64 (split_verdict; the device decides, no launch depends on it) if the effective
+// number of its sources, (sum |g|)^2 / sum g^2, is below a least one, or if their mean
+// direction, weighted by |g|, is longer than 1/2 (strengths within about a hemisphere)
+// and (sum g)^2 / sum g^2 is.  The least number: 256; and, as the velocity's error is
+// 2e-14 (like signs) to 6e-14 (a Rossby-Haurwitz wave) over its root and the FP64 form's
+// is 2e-16 / max(mesh spacing, 2.7 eps), 500,000 / sources and 500,000 eps^2 (measured
+// rms, split and FP64: wave, 1,280 sources, eps = 0.05 2.0e-15, 1.7e-15; 5,120 1.1e-15,
+// 1.5e-15; eps = 0.2 1.2e-15, 0.6e-15; 81,920 0.74e-15, 0.76e-15).
 // split_wanted() in direct_sum.cu holds the least sizes.
 // Pairs closer than 2^-20 of the domain, where the float pairs would run out
 // of bits, are evaluated in FP64 with the arithmetic of nbody_f64h.
@@ -99,15 +104,16 @@ struct SplitScale {
 };
 
 // Whether every pair is evaluated in FP64.
-__device__ __forceinline__ bool split_verdict(const SplitScale& s, int64_t nsrc) {
-  constexpr float kLeast = 256.f;  // effective sources
+__device__ __forceinline__ bool split_verdict(const SplitScale& s, int64_t nsrc, double eps2) {
+  // effective sources
+  const float least = fmaxf(256.f, fmaxf(5e5f / float(nsrc), 5e5f * float(eps2)));
   auto v = [&](int q) { return float((long long)(s.sum[q])); };
   const float A = v(0), Q = 65536.f * v(1), G = v(2);  // Q in the others' units squared
   const float k = s.big ? 0.f : exp2f(float(s.e));
   const float m0 = k * v(3), m1 = k * v(4), m2 = k * v(5);
   const bool compact = m0 * m0 + m1 * m1 + m2 * m2 > 0.25f * A * A;
-  return s.big || s.sum[6] * 16 > (unsigned long long)(nsrc) || A * A < kLeast * Q ||
-         (compact && G * G < kLeast * Q);
+  return s.big || s.sum[6] * 16 > (unsigned long long)(nsrc) || A * A < least * Q ||
+         (compact && G * G < least * Q);
 }
 
 // 2^k for |k| <= 1022
@@ -367,7 +373,7 @@ __global__ void __launch_bounds__(SPLIT_NT, 512 / SPLIT_NT)
   const int64_t s0 = (int64_t)blockIdx.y * chunk_len;
   int64_t slen = nsrc_pad - s0;
   if (slen > chunk_len) slen = chunk_len;
-  if (split_verdict(sc, nsrc)) {
+  if (split_verdict(sc, nsrc, eps2)) {
     split_fp64<SKIP>(tgt, tself, src, ti, s0, s0 + slen < nsrc ? s0 + slen : nsrc, eps2,
                      part + (int64_t)blockIdx.y * nc * ntgt_pad, ntgt_pad);
     return;
