@@ -216,7 +216,8 @@ static __device__ __noinline__ void split_near64(const double4_16a* t, const dou
 }
 
 // All pairs of one target and chunk with the operations of nbody_f64h, whose rate it
-// has (the FP64 pipe bounds it; the sources are uniform loads).  Out of line, called
+// has (the FP64 pipe bounds it; the sources are uniform loads), summed in runs of a tile:
+// a split chunk may be several times as long as one of nbody_f64h.  Out of line, called
 // before the split sums hold registers.
 template <bool SKIP>
 __device__ __noinline__ void split_fp64(const double4_16a* __restrict__ tgt,
@@ -226,20 +227,25 @@ __device__ __noinline__ void split_fp64(const double4_16a* __restrict__ tgt,
                                         int64_t ntgt_pad) {
   const double4_16a t = tgt[ti];
   const int self = SKIP ? tself[ti] : -1;
-  double a[3] = {0.0, 0.0, 0.0};
+  double sum[3] = {0.0, 0.0, 0.0};
+  for (int64_t i = j0; i < j1; i += SPLIT_TILE) {
+    const int64_t end = i + SPLIT_TILE < j1 ? i + SPLIT_TILE : j1;
+    double a[3] = {0.0, 0.0, 0.0};
 #pragma unroll 2
-  for (int64_t j = j0; j < j1; ++j) {
-    const double4_16a s = src[j];
-    const double arg = eps2 - fma(t.z, s.z, fma(t.y, s.y, fma(t.x, s.x, -1.0)));
-    const bool skip = SKIP && j == self;
-    const double q = f64_plain(fabs(arg)) ? s.w * f64_rcp(arg) : div_nr_any(s.w, arg);
-    const double g = skip ? 0.0 : q;
-    a[0] = fma(g, s.x, a[0]);
-    a[1] = fma(g, s.y, a[1]);
-    a[2] = fma(g, s.z, a[2]);
+    for (int64_t j = i; j < end; ++j) {
+      const double4_16a s = src[j];
+      const double arg = eps2 - fma(t.z, s.z, fma(t.y, s.y, fma(t.x, s.x, -1.0)));
+      const double q = f64_plain(fabs(arg)) ? s.w * f64_rcp(arg) : div_nr_any(s.w, arg);
+      const double g = SKIP && j == self ? 0.0 : q;
+      a[0] = fma(g, s.x, a[0]);
+      a[1] = fma(g, s.y, a[1]);
+      a[2] = fma(g, s.z, a[2]);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) sum[k] += a[k];
   }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) out[k * ntgt_pad + ti] = a[k];
+  for (int k = 0; k < 3; ++k) out[k * ntgt_pad + ti] = sum[k];
 }
 
 // ---- the stream function --------------------------------------------------------

@@ -69,3 +69,11 @@ def _errors(ctx, level, field, eps, targets):
 def test_wide_smoothing(gpu_ctx, level, field, eps):
     got, f64 = _errors(gpu_ctx, level, field, eps, 200)
     assert got <= 1.5 * f64
+
+
+@pytest.mark.parametrize("eps", [0.0, 0.05])
+def test_cancelling_vortices(gpu_ctx, eps):
+    """81,920 sources, 40,962 targets: chunks of thousands of sources, of one sign and
+    then the other."""
+    got, f64 = _errors(gpu_ctx, 6, "dipole", eps, 40)
+    assert got <= 1.5 * f64
