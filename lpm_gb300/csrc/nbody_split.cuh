@@ -33,10 +33,11 @@
 // number of its sources, (sum |g|)^2 / sum g^2, is below a least one, or if their mean
 // direction, weighted by |g|, is longer than 1/2 (strengths within about a hemisphere)
 // and (sum g)^2 / sum g^2 is.  The least number: 256; and, as the velocity's error is
-// 2e-14 (like signs) to 6e-14 (a Rossby-Haurwitz wave) over its root and the FP64 form's
-// is 2e-16 / max(mesh spacing, 2.7 eps), 500,000 / sources and 500,000 eps^2 (measured
-// rms, split and FP64: wave, 1,280 sources, eps = 0.05 2.0e-15, 1.7e-15; 5,120 1.1e-15,
-// 1.5e-15; eps = 0.2 1.2e-15, 0.6e-15; 81,920 0.74e-15, 0.76e-15).
+// 2e-14 (like signs: |sum g| of half sum |g| and more) to 6e-14 (a Rossby-Haurwitz wave)
+// over its root and the FP64 form's is 2e-16 / max(mesh spacing, 2.7 eps), 100,000 eps^2
+// for like signs, 500,000 eps^2 and 500,000 / sources for others (measured rms, split and
+// FP64: wave, 1,280 sources, eps = 0.05 2.0e-15, 1.7e-15; 5,120 1.1e-15, 1.5e-15; eps =
+// 0.2 1.2e-15, 0.6e-15; 81,920 0.74e-15, 0.76e-15).
 // split_wanted() in direct_sum.cu holds the least sizes.
 // Pairs closer than 2^-20 of the domain, where the float pairs would run out
 // of bits, are evaluated in FP64 with the arithmetic of nbody_f64h.
@@ -105,10 +106,11 @@ struct SplitScale {
 
 // Whether every pair is evaluated in FP64.
 __device__ __forceinline__ bool split_verdict(const SplitScale& s, int64_t nsrc, double eps2) {
-  // effective sources
-  const float least = fmaxf(256.f, fmaxf(5e5f / float(nsrc), 5e5f * float(eps2)));
   auto v = [&](int q) { return float((long long)(s.sum[q])); };
   const float A = v(0), Q = 65536.f * v(1), G = v(2);  // Q in the others' units squared
+  const float e2 = float(eps2);
+  const float least =  // effective sources
+      fmaxf(256.f, 4.f * G * G >= A * A ? 1e5f * e2 : 5e5f * fmaxf(1.f / float(nsrc), e2));
   const float k = s.big ? 0.f : exp2f(float(s.e));
   const float m0 = k * v(3), m1 = k * v(4), m2 = k * v(5);
   const bool compact = m0 * m0 + m1 * m1 + m2 * m2 > 0.25f * A * A;

@@ -65,7 +65,8 @@ def _errors(ctx, level, field, eps, targets):
 
 
 @pytest.mark.parametrize("level,field,eps", [(3, "wave", 0.05), (3, "wave", 0.1), (3, "wave", 0.2),
-                                             (4, "wave", 0.2), (4, "vortex", 0.2), (5, "wave", 0.3)])
+                                             (4, "wave", 0.2), (4, "vortex", 0.2), (5, "wave", 0.3),
+                                             (4, "vortex", 0.05), (5, "vortex", 0.1)])
 def test_wide_smoothing(gpu_ctx, level, field, eps):
     got, f64 = _errors(gpu_ctx, level, field, eps, 200)
     assert got <= 1.5 * f64
