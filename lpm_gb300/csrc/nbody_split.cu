@@ -124,8 +124,14 @@ __global__ void __launch_bounds__(128)
     r.exact = i < ntgt && (fabs(off) > 1.0 || fabs(x) >= 1.0 || fabs(y) >= 1.0 ||
                            fabs(z) >= 1.0);
     st[i] = r;
-    // (padding at the origin would be next to arg = 1, the logarithm's rare case)
-    if (pt) pt[i] = split_fixed(t, sc.e, i < ntgt ? off + 2.0 * eps * eps : 7.0, 0.0, r.exact != 0);
+    if (pt) {
+      // padding and positions that are NaN: any argument of the common path (the origin's
+      // is next to 1, the logarithm's rare case); NaN is added to the sum
+      const bool nan = isnan(t.x + t.y + t.z);
+      pt[i] = i < ntgt && !nan
+                  ? split_fixed(t, sc.e, off + 2.0 * eps * eps, 0.0, r.exact != 0)
+                  : SplitFixed{0, 0, 0, 1ll << 61, nan ? t.x + t.y + t.z : 0.0, 0, 0};
+    }
     return;
   }
   const int64_t k = int64_t(blockIdx.x) * 128 + threadIdx.x;

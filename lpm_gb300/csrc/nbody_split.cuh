@@ -76,8 +76,9 @@ constexpr int kSplitTile = SPLIT_TILE / 2;  // pairs of sources per tile
 constexpr float kSplitTiny = 9.094947e-13f;  // 2^-40: a pair's least scaled arg'
 
 // One point of the stream function: scaled position in units of 2^-61; its defect
-// (targets: plus 2 eps^2) in units of 2^-58, with 32 bits after the point; strength
-// (sources); whether a target lies outside the scaled range.
+// (targets: plus 2 eps^2) in units of 2^-58, with 32 bits after the point; a source's
+// strength, or what is added to a target's sum (0 or NaN); whether a target lies
+// outside the scaled range.
 struct __align__(16) SplitFixed {
   long long x, y, z, c;
   double g;
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(SPLIT_NT, 16)
     }
     sum += run;
   }
-  part[((int64_t)blockIdx.y * nc + nc - 1) * ntgt_pad + ti] = sum;
+  part[((int64_t)blockIdx.y * nc + nc - 1) * ntgt_pad + ti] = sum + x.g;
 }
 
 // ---- the velocity ---------------------------------------------------------------

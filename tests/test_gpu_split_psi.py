@@ -48,3 +48,28 @@ def test_rossby_haurwitz_stream_function(gpu_ctx, level, n, eps):
         arg = ((d * d).sum(1) + hy + (1 - (t * t).sum())) / 2 + ld(eps * eps)
         ref[k] = -(g * np.log(arg)).sum() / (4 * ld(math.pi))
     assert np.abs(p[idx] - ref).max() <= 1e-15 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("eps", [0.0, 0.05])
+def test_target_not_finite(gpu_ctx, value, eps):
+    """A target that is not finite: its sums are those of a call of the same sources over
+    that target and three others (few pairs: FP64 throughout), the others' are finite."""
+    vx, fx, fa, fm = core.build_mesh(core.MESH_ICOS_TRI, 3, 1.0)
+    y, a = fx[fm == 0], fa[fm == 0]
+    x = vx[:600].copy()
+    x[77, 1] = value
+
+    def sums(x):
+        dev = lambda v: torch.from_numpy(np.ascontiguousarray(v)).cuda()
+        u = torch.empty(len(x), 3, dtype=torch.float64, device="cuda")
+        p = torch.empty(len(x), dtype=torch.float64, device="cuda")
+        gpu_ctx.set_precision(core.FP64)
+        F.ic2d_passive_sums(gpu_ctx, u, p, dev(x), dev(y), dev(y[:, 0].copy()), dev(a),
+                            dev(np.zeros(len(y), np.uint8)), eps)
+        gpu_ctx.synchronize()
+        return np.c_[u.cpu().numpy(), p.cpu().numpy()]
+
+    s = sums(x)
+    assert np.isfinite(np.delete(s, 77, 0)).all()
+    assert np.array_equal(s[77], sums(x[75:79])[2], equal_nan=True)
