@@ -48,11 +48,12 @@ extern "C" {
 /* ---- arithmetic of the pairwise sum ------------------------------------ */
 /* LPM_FP64: the reference's pair kernels in FP64 (1 - x.y [+ eps^2] on the
  *            sphere, |x-y|^2 + eps^2 on the plane) with the cross product
- *            taken out of the sum (u = x cross sum_j (g_j / arg_j) y_j); large
- *            sphere sums run in float pairs (48 bits per term, exact x - y)
- *            where the strengths have at least 256 effective sources,
- *            (sum |g|)^2 / sum g^2, also counted with their signs if all lie
- *            within about a hemisphere; within 1e-12 of the reference.
+ *            taken out of the sum (u = x cross sum_j (g_j / arg_j) y_j).  Large
+ *            sphere sums take the velocity in float pairs (48 bits per term,
+ *            exact x - y) where the sources are many enough, by the effective
+ *            number (sum |g|)^2 / sum g^2 (256 and more, more with a wide eps),
+ *            to average that out, and the stream function in 64-bit fixed
+ *            point.  Within 1e-12 of the reference.
  * LPM_FP64_EXACT: every pair term in FP64 in the reference's evaluation
  *            order (correctly rounded divisions), each term equal to the
  *            reference's bit for bit; about 20x slower (sphere) than LPM_FP64.

@@ -306,7 +306,7 @@ static __device__ __noinline__ double split_arg_any(long long d0, long long d1, 
 // its own: beside the float-pair velocity its registers left 16 warps per SM, which do
 // not hide its chains of operations (velocity and stream function, 14,336 targets by
 // 6,144 sources: 1.35 ms in one kernel, 1.08 ms in two, 2.46 ms as nbody_f64h, 0.75 ms
-// in float pairs).  Bound: the FP64 pipe, 0.80 of its rate.
+// in float pairs).  Bound: the FP64 pipe, 0.82 of its rate.
 //   pt, ps: SplitFixed per target and source, ntgt_pad and nsrc_pad of them
 //   part: [chunk][nc][ntgt_pad], the last component
 template <bool SKIP>

@@ -60,7 +60,7 @@ constexpr int kSweTile64 = 64;
 // the logarithm), everything between formed in integers beside them (swe_pair), against
 // about 260 for the reference's operation order with its eight divisions, square root
 // and library log and exp.  Quad level 5, vertices and faces: 19.6 ms in that order,
-// 4.73 ms as moments in FP64 (55 operations), 1.64 ms now (0.92 of the pipe's rate).
+// 4.73 ms as moments in FP64 (55 operations), 1.64 ms now (0.88 of the pipe's rate).
 constexpr int kSweNC = 11;
 
 struct __align__(16) SweSrc {
