@@ -73,3 +73,23 @@ def test_target_not_finite(gpu_ctx, value, eps):
     s = sums(x)
     assert np.isfinite(np.delete(s, 77, 0)).all()
     assert np.array_equal(s[77], sums(x[75:79])[2], equal_nan=True)
+
+
+@pytest.mark.parametrize("collocated", [False, True])
+def test_stream_function_alone(gpu_ctx, collocated):
+    """Without the velocity: the same kernel over the same chunks, the same bits."""
+    vx, fx, fa, fm = core.build_mesh(core.MESH_CUBED_SPHERE, 4, 1.0)
+    y, a = fx[fm == 0], fa[fm == 0]
+    x = y if collocated else vx
+    dev = lambda v: torch.from_numpy(np.ascontiguousarray(v)).cuda()
+    X, Y, Z, A, M = dev(x), dev(y), dev(y[:, 1].copy()), dev(a), dev(np.zeros(len(y), np.uint8))
+    u = torch.empty(len(x), 3, dtype=torch.float64, device="cuda")
+    p, q = (torch.empty(len(x), dtype=torch.float64, device="cuda") for _ in range(2))
+    gpu_ctx.set_precision(core.FP64)
+    for vel, psi in ((u, p), (None, q)):
+        if collocated:
+            F.ic2d_active_sums(gpu_ctx, vel, psi, Y, Z, A, M, 0.0, self_rule=1)
+        else:
+            F.ic2d_passive_sums(gpu_ctx, vel, psi, X, Y, Z, A, M, 0.0)
+    gpu_ctx.synchronize()
+    assert torch.isfinite(p).all() and torch.equal(p, q)
