@@ -557,9 +557,9 @@ void ff_cells(lpm_context& ctx, const float4* ys, const int4* cells, int ncells,
   LPM_CUDA(cudaGetLastError());
 }
 
-// Parts of an evaluation: at least kPartWaves waves of CTAs (seven resident per
-// SM).  Icosahedral level 6, theta 0.4 (1,600 blocks: 1.5 waves in one part):
-// 470 us in one part, 407 in four; level 8 (25,557 blocks) runs one part.
+// Parts of an evaluation: at least kPartWaves waves of seven CTAs per SM (six are
+// resident, at 79 registers).  Icosahedral level 6, theta 0.4 (1,628 blocks: 1.8 waves in
+// one part): 470 us in one part, 407 in three; level 8 (25,557 blocks) runs one part.
 int ff_parts(const lpm_context& ctx, int64_t nblocks) {
   constexpr int64_t kPartWaves = 6;
   const int64_t slots = int64_t(std::max(ctx.num_sms, 1)) * 7;
